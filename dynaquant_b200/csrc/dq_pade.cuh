@@ -236,6 +236,179 @@ __device__ inline PadeOut pade_exp_tbar(int m, const cd* alpha, const cd* beta, 
     return out;
 }
 
+// ---------------------------------------------------------------------------
+// The columns of exp(tau Tbar) that a step uses, by one warp.
+//
+// A step needs E e_0 (the combine weights) and E(m-1, m), E(m-1, m+1) (the
+// error estimate) only.  With A = tau T (m x m, tridiagonal) the augmented
+// columns are E e_{m+q-1} = tau^q sum_k A^k e_0 / (k+q)!, q >= 1, so one
+// sequence t_k = A^k e_0 / k! gives all of them, and lane i of a warp holds
+// row i: two neighbour shuffles and ten FP64 operations per term, no shared
+// memory and no barrier.  The matrix is scaled by the dense form's own rule
+// (row-sum norm <= 1/2 after s halvings), where the series reaches 1e-19 in
+// about 16 terms; with s > 0 the scaled exponential is applied 2^s times.
+// The dense Padé(6,6) above (LU of a (m+2)^2 matrix by one CTA, a serial chain
+// of about 6 L barriers) stays for what the series does not cover: more than
+// kSeriesMaxS halvings, and the |Re|-only norm on a matrix of complex norm
+// above 1/2, whose quotient the reference takes unscaled.
+// Measured on a B200 (kernel time): one trajectory, m = 16, 41 us dense and
+// 4.4 us this way; 256 trajectories, m = 20, 61 and 6.6 us.
+// ---------------------------------------------------------------------------
+constexpr int kSeriesMaxS = 4;
+constexpr int kSeriesTerms = 24;   // never reached at a norm <= 1/2 (16 terms); bounds the loops
+
+// 1/k
+__device__ __constant__ static const double kInvK[kSeriesTerms + 3] = {
+    0.0,      1.0,      1.0 / 2,  1.0 / 3,  1.0 / 4,  1.0 / 5,  1.0 / 6,  1.0 / 7,  1.0 / 8,
+    1.0 / 9,  1.0 / 10, 1.0 / 11, 1.0 / 12, 1.0 / 13, 1.0 / 14, 1.0 / 15, 1.0 / 16, 1.0 / 17,
+    1.0 / 18, 1.0 / 19, 1.0 / 20, 1.0 / 21, 1.0 / 22, 1.0 / 23, 1.0 / 24, 1.0 / 25, 1.0 / 26};
+
+// The dense form's halvings of one norm.
+__device__ __forceinline__ int halvings(double nrm) {
+    int s = 0;
+    while (nrm > 0.5 && s < 60) { nrm *= 0.5; s++; }
+    return s;
+}
+
+// A warp's tridiagonal matrix: lane i holds row i of A = tau T, its diagonal
+// and the imaginary parts of its (purely imaginary) couplings to rows i - 1
+// and i + 1; lanes >= m hold zeros.
+struct WarpTri {
+    cd a;
+    double bl, br;
+    // A v
+    __device__ __forceinline__ cd mul(cd v) const {
+        const double px = __shfl_down_sync(0xffffffffu, v.x, 1), py = __shfl_down_sync(0xffffffffu, v.y, 1);
+        const double mx = __shfl_up_sync(0xffffffffu, v.x, 1), my = __shfl_up_sync(0xffffffffu, v.y, 1);
+        return cmk(a.x * v.x - a.y * v.y - (br * py + bl * my), a.x * v.y + a.y * v.x + (br * px + bl * mx));
+    }
+};
+
+// alpha, beta of rows 0..m-1 as the warp's lanes hold them (lane i: alpha_{i+1}
+// and beta_{i+1}); lanes >= m pass anything.
+__device__ __forceinline__ WarpTri warp_tri(int m, cd alpha, double beta, double tau_im) {
+    const int lane = threadIdx.x & 31;
+    WarpTri t;
+    t.a = lane < m ? cmk(-tau_im * alpha.y, tau_im * alpha.x) : cmk(0.0, 0.0);
+    t.br = lane < m - 1 ? tau_im * beta : 0.0;
+    const double up = __shfl_up_sync(0xffffffffu, t.br, 1);
+    t.bl = lane > 0 && lane < m ? up : 0.0;
+    return t;
+}
+
+// Row-sum infinity norms of the augmented matrix (the ones of its extra
+// columns scaled by tau, too): |Re|-only and complex.
+__device__ __forceinline__ void warp_tri_norms(const WarpTri& t, double tau_im, double& re, double& cn) {
+    const int lane = threadIdx.x & 31;
+    const double one = fabs(tau_im);
+    re = fabs(t.a.x);
+    cn = fmax(sqrt(cabs2(t.a)) + fabs(t.bl) + fabs(t.br) + (lane == 0 ? one : 0.0), one);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        re = fmax(re, __shfl_xor_sync(0xffffffffu, re, o));
+        cn = fmax(cn, __shfl_xor_sync(0xffffffffu, cn, o));
+    }
+}
+
+// Rows of E e_0 (y), E e_m (f1) and E e_{m+1} (f2) in their lanes.  Returns
+// false where the dense form has to be used; s is its number of halvings, -1
+// when that would reach 50 (then nothing is computed).  Called by all 32
+// lanes; every lane returns the same.
+__device__ __forceinline__ bool series_exp_tbar(int m, cd alpha, double beta, double tau_im, int norm_mode, cd& y,
+                                                cd& f1, cd& f2, int& s) {
+    const int lane = threadIdx.x & 31;
+    WarpTri t = warp_tri(m, alpha, beta, tau_im);
+    double re, cn;
+    warp_tri_norms(t, tau_im, re, cn);
+    s = halvings(norm_mode == 0 ? re : cn);
+    y = f1 = f2 = cmk(0.0, 0.0);
+    if (s >= 50) {
+        s = -1;
+        return true;
+    }
+    if (s > kSeriesMaxS || (norm_mode == 0 && cn > 0.5)) return false;
+    const double h = ldexp(1.0, -s);
+    t.a = cscale(t.a, h);
+    t.bl *= h;
+    t.br *= h;
+    cn *= h;
+    // t_k = A^k e_0 / k!: the sums of t_k, t_k / (k+1) and t_k / ((k+1)(k+2))
+    cd v = cmk(lane == 0 ? 1.0 : 0.0, 0.0);
+    y = v;
+    f1 = v;
+    f2 = cscale(v, 0.5);
+    double bound = 1.0;
+    for (int k = 1; k <= kSeriesTerms && bound > 1e-19; ++k) {
+        v = cscale(t.mul(v), kInvK[k]);
+        bound *= cn * kInvK[k];
+        y = cadd(y, v);
+        const cd u = cscale(v, kInvK[k + 1]);
+        f1 = cadd(f1, u);
+        f2 = cadd(f2, cscale(u, kInvK[k + 2]));
+    }
+    // times tau h and (tau h)^2 = -(tau_im h)^2
+    const double th = tau_im * h;
+    f1 = cmk(-th * f1.y, th * f1.x);
+    f2 = cscale(f2, -th * th);
+    if (s == 0) return true;
+    // the other 2^s - 1 steps of length h: (x; c; 1) -> (exp(hA) x + c g1 + g2; c + tau h; 1)
+    const cd g1 = f1, g2 = f2;
+    double c = th;   // the (m, m+1) entry so far, times -i
+    for (int r = 1; r < (1 << s); ++r) {
+        cd vy = y, v1 = f1, v2 = f2;
+        double bd = 1.0;
+        for (int k = 1; k <= kSeriesTerms && bd > 1e-19; ++k) {
+            vy = cscale(t.mul(vy), kInvK[k]);
+            v1 = cscale(t.mul(v1), kInvK[k]);
+            v2 = cscale(t.mul(v2), kInvK[k]);
+            bd *= cn * kInvK[k];
+            y = cadd(y, vy);
+            f1 = cadd(f1, v1);
+            f2 = cadd(f2, v2);
+        }
+        f1 = cadd(f1, g1);
+        f2 = cadd(f2, cadd(cmk(-c * g1.y, c * g1.x), g2));
+        c += th;
+    }
+    return true;
+}
+
+// Taylor-Krylov's augmented matrix (ones at (0, mb) and (mb+k, mb+k+1), k < p
+// - 1): rows of its last column (fp), of column mb (f1) and of column mb + 1
+// (f2).  Returns false where the dense form has to be used (any halving).
+__device__ __forceinline__ bool series_exp_tk(int mb, int p, cd alpha, double beta, double tau_im, int norm_mode,
+                                              cd& fp, cd& f1, cd& f2) {
+    const int lane = threadIdx.x & 31;
+    const WarpTri t = warp_tri(mb, alpha, beta, tau_im);
+    double re, cn;
+    warp_tri_norms(t, tau_im, re, cn);
+    fp = f1 = f2 = cmk(0.0, 0.0);
+    if (!(cn <= 0.5) || !(re <= 0.5)) return false;
+    // c_k = k! / (k + p)!; fp's terms are t_k c_k
+    double c = 1.0;
+    for (int q = 2; q <= p; ++q) c /= q;
+    cd v = cmk(lane == 0 ? 1.0 : 0.0, 0.0);
+    fp = cscale(v, c);
+    f1 = v;
+    f2 = cscale(v, 0.5);
+    double bound = 1.0;
+    for (int k = 1; k <= kSeriesTerms && bound > 1e-19; ++k) {
+        v = cscale(t.mul(v), kInvK[k]);
+        bound *= cn * kInvK[k];
+        c *= (double)k / (double)(k + p);
+        fp = cadd(fp, cscale(v, c));
+        const cd u = cscale(v, kInvK[k + 1]);
+        f1 = cadd(f1, u);
+        f2 = cadd(f2, cscale(u, kInvK[k + 2]));
+    }
+    cd tp = cmk(1.0, 0.0);
+    for (int q = 0; q < p; ++q) tp = cmk(-tau_im * tp.y, tau_im * tp.x);
+    fp = cmul(fp, tp);
+    f1 = cmk(-tau_im * f1.y, tau_im * f1.x);
+    f2 = cscale(f2, -tau_im * tau_im);
+    return true;
+}
+
 // EXPOKIT Algorithm 3.2 as padeClass.cu:750-782 with the floor of
 // systemClass.cu:2075-2077.
 __device__ __forceinline__ double expokit_error(double beta_m, double norm_av, cd e_m1_m, cd e_m1_mp1) {

@@ -223,6 +223,28 @@ __global__ void __launch_bounds__(kPlainThreads) k_spmv_norm(int n, int j, const
 __global__ void k_pade_plain(int m, double tau_im, int norm_mode, PlainScalars* ps, double* erracc, int traj) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ cd y[kMaxM];
+    __shared__ bool dense;
+    // the series on one warp; the other warps wait in case the dense form is needed
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, k = min(lane, m - 1) + 1;
+        cd yl, f1, f2;
+        int s;
+        const bool ok = series_exp_tbar(m, ps->alpha[k], ps->beta[k].x, tau_im, norm_mode, yl, f1, f2, s);
+        if (lane == 0) dense = !ok;
+        if (ok && s < 0) {
+            if (lane == 0) atomicCAS(&ps->status, 0, DQ_ERR_SCALING);
+        } else if (ok) {
+            if (lane < m) ps->yt[lane + 1] = cscale(yl, ps->sc[lane + 1]);
+            if (lane == m - 1) {
+                ps->s = s;
+                const double est = expokit_error(ps->beta[m].x, ps->nav, f1, f2);
+                ps->err = est;
+                if (erracc) erracc[traj] += est;
+            }
+        }
+    }
+    __syncthreads();
+    if (!dense) return;
     PadeOut o = pade_exp_tbar(m, ps->alpha, ps->beta, cmk(0.0, tau_im), norm_mode, y, smem);
     if (o.s < 0) {
         if (threadIdx.x == 0) atomicCAS(&ps->status, 0, (o.s == -1) ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
@@ -339,6 +361,22 @@ __global__ void __launch_bounds__(kPlainThreads) k_tk_power(int n, int k, int p,
 // column scaled by ||A^p psi||; the EXPOKIT estimate of the B part.
 __global__ void k_pade_tk(int mb, int p, double tau_im, int norm_mode, PlainScalars* ps) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ bool dense;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, k = min(lane, mb - 1) + 1;
+        cd fp, f1, f2;
+        const bool ok = series_exp_tk(mb, p, ps->alpha[k], ps->beta[k].x, tau_im, norm_mode, fp, f1, f2);
+        if (lane == 0) dense = !ok;
+        if (ok) {
+            if (lane < mb) ps->yt[lane + 1] = cscale(fp, ps->tk_beta0 * ps->sc[lane + 1]);
+            if (lane == mb - 1) {
+                ps->s = 0;
+                ps->tk_kerr = expokit_error(ps->beta[mb].x, ps->nav, f1, f2);
+            }
+        }
+    }
+    __syncthreads();
+    if (!dense) return;
     const int L = mb + p;
     cd* A = reinterpret_cast<cd*>(smem);
     const cd tau = cmk(0.0, tau_im);

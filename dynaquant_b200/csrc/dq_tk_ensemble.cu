@@ -223,7 +223,21 @@ __global__ void __launch_bounds__(kTkThreads) k_tke_nav(int n, int B, int j, con
 // part's EXPOKIT estimate, as k_pade_tk of the per-trajectory path.
 __global__ void k_tke_pade(int mb, int p, int B, double tau_im, int norm_mode, TkScal S) {
     extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ bool dense;
     const int b = blockIdx.x;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const size_t k = (size_t)(min(lane, mb - 1) + 1) * B + b;
+        cd fp, f1, f2;
+        const bool ok = series_exp_tk(mb, p, S.alpha[k], S.beta[k].x, tau_im, norm_mode, fp, f1, f2);
+        if (lane == 0) dense = !ok;
+        if (ok) {
+            if (lane < mb) S.yt[k] = cscale(fp, S.beta0[b] * S.sc[k]);
+            if (lane == mb - 1) S.kerr[b] = expokit_error(S.beta[k].x, S.nav[b], f1, f2);
+        }
+    }
+    __syncthreads();
+    if (!dense) return;
     const int L = mb + p;
     cd* A = reinterpret_cast<cd*>(smem);
     const cd tau = cmk(0.0, tau_im);
