@@ -47,9 +47,10 @@ dq_status upload_couplings(dq_ctx* c) {
         if (!c->cls.empty()) s = c->scales[c->cls[k]];
         c->val[k] = s * c->val_base[k];
     }
-    dq_status st = batched_invalidate_blocks(c);
+    // the values first: the packed coupling blocks are rebuilt from the device CSR
+    dq_status st = upload(c, &c->d_val, c->val.data(), c->val.size());
     if (st) return st;
-    return upload(c, &c->d_val, c->val.data(), c->val.size());
+    return batched_invalidate_blocks(c);
 }
 
 }  // namespace

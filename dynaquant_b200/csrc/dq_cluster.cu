@@ -1,0 +1,939 @@
+// dq_cluster.cu — one launch per step for ensembles that fit on the chip.
+//
+// Trajectories do not exchange anything, so a thread-block cluster can carry a
+// few of them through a whole step by itself: noise, the m Lanczos iterations,
+// the exponential, the combination, the norms.  The grid-wide form of
+// dq_batched.cu runs 2 m + 4 launches for the same step, and on a small system
+// each is bound by its launch, its dependent scalar loads and its grid-wide
+// reduction (ticket, partials through L2), not by the data: 12 us per
+// iteration for a 1 MB slab, 20 us for 2 to 4 MB.
+//
+// A cluster owns TC trajectories, each of its CTAs a contiguous range of rows.
+// Shared memory holds, for the whole step, the CTA's window of r_j (its own
+// rows and the bandwidth on either side), r_{j-1} (then w in its place), the
+// diagonal and, where they fit, the coupling records: the gathers of an
+// iteration touch nothing else.  r_{j+1} also goes to its global slab, for the
+// combination.  alpha_j and beta_j are sums over the cluster: every CTA stores
+// its part into every CTA's shared memory (DSMEM), and after one hardware
+// cluster barrier (0.2 to 0.3 us) every CTA adds the parts in rank order, so
+// all hold the same bits and no scalar takes a trip through global memory.
+// After the second barrier the window's margins are read from the
+// neighbours' shared memory.  A one-CTA cluster needs none of this.
+//
+// What bounds it: at 2 couplings per row the latency of an iteration's two
+// reductions; at 28 per row the gathers' shared-memory wavefronts.
+#include <algorithm>
+#include <cmath>
+
+#include "dq_batched.cuh"
+#include "dq_rng.cuh"
+
+namespace dq {
+
+constexpr int kClThreads = 512;
+constexpr int kClWarps = kClThreads / 32;
+constexpr int kClMaxCtas = 16;            // CTAs per cluster (above 8: not portable, sm_100 allows 16)
+// dynamic shared memory of one CTA (one CTA per SM: 128 registers a thread)
+constexpr size_t kClSmemMax = 224 * 1024;
+
+enum { kClNoise = 1, kClFinish = 2 };
+
+struct ClusterArgs {
+    int n, B, TC, rpc, bw, m, flags, bil, chunks;
+    int rec_smem;             // bytes of coupling records kept in shared memory (0: read through L1)
+    const int* bptr;
+    const int* bcol;
+    const void* bcoef;
+    void* slabs;
+    size_t slab;              // complex values per slab
+    void* diag;
+    BatchedScalars S;
+    int noise, ns, traj0;
+    double subdt, sqrt_subdt;
+    uint64_t seed;
+    const double* sigma;
+    const double* invtau;
+    const double* coeff;
+    const double* eps;
+    double* deps;
+    const double* zzD;
+    const int* zz_start;
+    int norm_mode, m_min;
+    double tau_im, tol;
+    double* erracc;
+    const cd* bra;
+    unsigned char* scratch;   // per chunk, for the dense exponential
+    size_t scratch_stride;
+};
+
+// Shared memory of a CTA: reductions, the chunk's scalars, the vectors, the records.
+struct ClLayout {
+    size_t ex, red, al, y, par, be, sc, win, prev, d, rec, total;
+};
+
+static __host__ __device__ inline ClLayout cl_layout(int CS, int TC, int m, int rpc, int bw, size_t rsz, size_t rec) {
+    ClLayout L;
+    size_t p = 0;
+    L.ex = p; p += sizeof(double2) * 2 * CS * TC;
+    L.red = p; p += sizeof(double2) * 2 * kClWarps * TC;
+    L.al = p; p += sizeof(double2) * (m + 2) * TC;
+    L.y = p; p += sizeof(double2) * m * TC;
+    L.par = p; p += sizeof(double2) * 2 * TC;
+    L.be = p; p += sizeof(double) * (m + 2) * TC;
+    L.sc = p; p += sizeof(double) * (m + 2) * TC;
+    p = (p + 127) & ~(size_t)127;
+    const size_t row = (size_t)TC * 2 * rsz;
+    L.win = p; p += (rpc + (CS > 1 ? 2 * (size_t)bw : 0)) * row;
+    L.prev = p; p += rpc * row;
+    L.d = p; p += rpc * row / 2;
+    p = (p + 15) & ~(size_t)15;
+    L.rec = p; p += rec;
+    L.total = (p + 15) & ~(size_t)15;
+    return L;
+}
+
+__device__ __forceinline__ unsigned cl_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cl_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cl_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// p in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ void cl_store(double2* p, unsigned rank, double2 v) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(ra), "d"(v.x), "d"(v.y) : "memory");
+}
+
+// 16 or 8 bytes of `p` in the shared memory of CTA `rank`
+template <typename T>
+__device__ __forceinline__ T cl_load(const T* p, unsigned rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
+    T v;
+    if constexpr (sizeof(T) == 16) {
+        unsigned* u = reinterpret_cast<unsigned*>(&v);
+        asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]) : "r"(ra) : "memory");
+    } else {
+        unsigned* u = reinterpret_cast<unsigned*>(&v);
+        asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(u[0]), "=r"(u[1]) : "r"(ra) : "memory");
+    }
+    return v;
+}
+
+// the dense exponential out of line: its registers stay out of the step's
+__device__ __noinline__ PadeOut cl_dense(int m, const cd* al, const cd* be, double tau_im, int norm_mode, cd* y,
+                                         unsigned char* scratch) {
+    return pade_exp_tbar(m, al, be, cmk(0.0, tau_im), norm_mode, y, scratch);
+}
+
+// One CTA's view of its cluster's sums.
+template <int TPT, bool kLocal>
+struct ClSum {
+    double2* ex;    // [2][CS][TC]
+    double2* red;   // [2][warps][TC]
+    int TC, CS;
+    unsigned rank;
+
+    __device__ __forceinline__ void sync() const {
+        if constexpr (kLocal) __syncthreads();
+        else cl_sync();
+    }
+    // this CTA's part of sum `buf` into every CTA's ex[buf]; the caller syncs.
+    // kPair: y is summed too.
+    template <bool kPair>
+    __device__ __forceinline__ void part(int buf, const double (&x)[TPT], const double (&y)[TPT]) const {
+        const int TL = TC / TPT, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        double a[TPT], b[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+            a[t] = x[t];
+            b[t] = kPair ? y[t] : 0.0;
+        }
+        for (int o = TL; o < 32; o <<= 1) {
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) {
+                a[t] += __shfl_xor_sync(0xffffffffu, a[t], o);
+                if (kPair) b[t] += __shfl_xor_sync(0xffffffffu, b[t], o);
+            }
+        }
+        if (lane < TL) {
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) red[(buf * kClWarps + warp) * TC + lane * TPT + t] = make_double2(a[t], b[t]);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < TC * CS; e += kClThreads) {
+            const int t = e % TC, dst = e / TC;
+            double2 v[kClWarps];
+#pragma unroll
+            for (int w = 0; w < kClWarps; ++w) v[w] = red[(buf * kClWarps + w) * TC + t];
+#pragma unroll
+            for (int h = kClWarps / 2; h > 0; h >>= 1)
+#pragma unroll
+                for (int w = 0; w < h; ++w) {
+                    v[w].x += v[w + h].x;
+                    if (kPair) v[w].y += v[w + h].y;
+                }
+            double2* p = ex + ((size_t)buf * CS + rank) * TC + t;
+            if constexpr (kLocal) *p = v[0];
+            else cl_store(p, dst, v[0]);
+        }
+    }
+    // the whole sum of trajectory t (after the sync), in rank order
+    __device__ __forceinline__ double2 get(int buf, int t) const {
+        double2 s = ex[(size_t)buf * CS * TC + t];
+        if constexpr (!kLocal) {
+#pragma unroll 4
+            for (int r = 1; r < CS; ++r) {
+                const double2 v = ex[((size_t)buf * CS + r) * TC + t];
+                s.x += v.x;
+                s.y += v.y;
+            }
+        }
+        return s;
+    }
+};
+
+// Four coupling entries of one row block: window row and R coefficients each.
+template <typename Real, int R>
+struct ClRec {
+    int c[4];
+    Real cf[4][R];
+    // entries [e, e + 4) of a block that ends at pe; col/rec in shared memory or global
+    __device__ __forceinline__ void load(int e, int pe, const int* col, const void* rec) {
+        if constexpr (sizeof(Real) == 4) {
+            // packed records {col, c0, c1, c2}, a multiple of 4 per block
+            const float4* r4 = reinterpret_cast<const float4*>(rec) + e;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 r = r4[u];
+                c[u] = __float_as_int(r.x);
+                cf[u][0] = r.y;
+                if constexpr (R > 1) cf[u][R > 1 ? 1 : 0] = r.z;
+                if constexpr (R > 2) cf[u][R > 2 ? 2 : 0] = r.w;
+            }
+        } else {
+            const Real* cb = reinterpret_cast<const Real*>(rec);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int p = min(e + u, pe - 1);
+                c[u] = col[p];
+#pragma unroll
+                for (int i = 0; i < R; ++i) cf[u][i] = e + u < pe ? cb[(size_t)p * R + i] : Real(0);
+            }
+        }
+    }
+};
+
+// acc += the couplings of one row block, entries [pb, pe), times the window's
+// rows (`win` points at this thread's trajectories of global row 0); the next
+// four entries load while the current four gather.
+template <typename Real, int TPT, int R>
+__device__ __forceinline__ void cl_gather(int pb, int pe, const int* col, const void* rec, const Real* win, int row,
+                                          CV<Real, TPT> (&acc)[R]) {
+    if (pb >= pe) return;
+    ClRec<Real, R> A;
+    A.load(pb, pe, col, rec);
+    for (int e = pb;; e += 4) {
+        const bool more = e + 4 < pe;
+        ClRec<Real, R> N;
+        if (more) N.load(e + 4, pe, col, rec);
+        CV<Real, TPT> y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = ldv<Real, TPT, false>(win + (ptrdiff_t)A.c[u] * row, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int i = 0; i < R; ++i) cfma<Real, TPT>(acc[i], A.cf[u][i], y[u]);
+        if (!more) break;
+        A = N;
+    }
+}
+
+template <typename Real, int TPT, int R, bool kLocal>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArgs A) {
+    using T = typename VL<Real, TPT>::T;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int mtr[kMaxTC];
+    __shared__ int flag;   // some trajectory's exponential needs the dense form
+    const int TC = A.TC, TL = TC / TPT, B = A.B, n = A.n;
+    const int CS = kLocal ? 1 : (int)cl_size();
+    const unsigned rank = kLocal ? 0u : cl_rank();
+    const int bw = kLocal ? 0 : A.bw;
+    const ClLayout Y = cl_layout(CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem);
+    double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
+    double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
+    double2* par = reinterpret_cast<double2*>(smem + Y.par);   // [0][t] alpha_j sc_j, [1][t] (sc_j, the factor of r_{j-1})
+    double* be = reinterpret_cast<double*>(smem + Y.be);
+    double* scs = reinterpret_cast<double*>(smem + Y.sc);
+    const int rowr = TC * 2;                                   // Reals of one row
+    Real* win = reinterpret_cast<Real*>(smem + Y.win);
+    Real* cur = win + (size_t)bw * rowr;                       // the own rows of the window
+    Real* prev = reinterpret_cast<Real*>(smem + Y.prev);
+    Real* dsm = reinterpret_cast<Real*>(smem + Y.d);
+    const ClSum<TPT, kLocal> sum{reinterpret_cast<double2*>(smem + Y.ex), reinterpret_cast<double2*>(smem + Y.red),
+                                 TC, CS, rank};
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tl = threadIdx.x % TL, rl = threadIdx.x / TL, RL = kClThreads / TL;
+    const int chunk = blockIdx.x / CS, c0 = chunk * TC;
+    const int b0 = c0 + tl * TPT;
+    const bool act = b0 < B;                 // lanes past the last trajectory only keep the barriers
+    const int bb = act ? b0 : 0;
+    const int r0 = min((int)rank * A.rpc, n), nrow = min(n - r0, A.rpc);
+    const int nbk = act ? (nrow + R - 1) / R : 0;
+    const int hlo = kLocal ? 0 : min(bw, r0), hhi = kLocal ? 0 : min(bw, n - (r0 + nrow));
+    Real* slabs = reinterpret_cast<Real*>(A.slabs);
+    auto slab = [&](int j) { return slabs + 2 * A.slab * j; };
+    // own row `row` (within the CTA) of this thread's trajectories
+    auto loc = [&](int row) { return (size_t)row * TC + tl * TPT; };
+    auto glo = [&](int row) { return (size_t)(r0 + row) * B + bb; };
+
+    // ---- the coupling records of the own row blocks --------------------------
+    const int kb0 = r0 / R, nbo = (nrow + R - 1) / R;
+    const int* bptr = A.bptr + kb0;
+    const int* col = A.bcol;
+    const void* rec = A.bcoef;
+    int ebase = 0;
+    if (A.rec_smem) {
+        // block starts, columns (FP64), coefficients
+        ebase = __ldg(bptr);
+        const int ne = __ldg(bptr + nbo) - ebase;
+        int* sb = reinterpret_cast<int*>(smem + Y.rec);
+        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(bptr + k);
+        unsigned char* q = smem + Y.rec + (((size_t)nbo + 1) * 4 + 15) / 16 * 16;
+        if constexpr (sizeof(Real) == 4) {
+            float4* sr = reinterpret_cast<float4*>(q);
+            const float4* gr = reinterpret_cast<const float4*>(A.bcoef) + ebase;
+            for (int e = threadIdx.x; e < ne; e += kClThreads) sr[e] = __ldg(gr + e);
+            rec = sr;
+        } else {
+            int* scol = reinterpret_cast<int*>(q);
+            Real* sr = reinterpret_cast<Real*>(q + ((size_t)ne * 4 + 15) / 16 * 16);
+            const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)ebase * R;
+            for (int e = threadIdx.x; e < ne; e += kClThreads) scol[e] = __ldg(A.bcol + ebase + e);
+            for (int e = threadIdx.x; e < ne * R; e += kClThreads) sr[e] = __ldg(gr + e);
+            col = scol;
+            rec = sr;
+        }
+        bptr = sb;
+    }
+
+    // ---- r_1 = psi over the window, the diagonal (noise of this step, or as it is)
+    if (act) {
+        const int step = *A.S.step;
+        const double* D = A.noise == DQ_NOISE_ZZ && (A.flags & kClNoise)
+                              ? A.zzD + (size_t)(step - *A.zz_start) * n * B : nullptr;
+        Real* dg = reinterpret_cast<Real*>(A.diag);
+        for (int row = rl - hlo; row < nrow + hhi; row += RL) {
+            const size_t x = ((ptrdiff_t)r0 + row) * B + bb;
+            stv<Real, TPT>(cur + (ptrdiff_t)row * rowr, tl * TPT, ldv<Real, TPT, false>(slab(1), x));
+            if (row < 0 || row >= nrow) continue;
+            const size_t l = loc(row);
+            if (!(A.flags & kClNoise)) {
+#pragma unroll
+                for (int t = 0; t < TPT; ++t) dsm[l + t] = dg[x + t];
+                continue;
+            }
+            const int site = r0 + row;
+            double v[TPT];
+            if (A.noise == DQ_NOISE_OU) {
+                if constexpr (TPT == 2) {
+                    double u0 = A.deps[x], u1 = A.deps[x + 1];
+                    ou_update_pair(u0, u1, A.invtau[site], A.coeff[site], A.subdt, A.sqrt_subdt, A.ns, A.seed,
+                                   (A.traj0 + bb) >> 1, step, site);
+                    A.deps[x] = u0;
+                    A.deps[x + 1] = u1;
+                    v[0] = __dadd_rn(u0, A.eps[x]);
+                    v[TPT - 1] = __dadd_rn(u1, A.eps[x + 1]);
+                } else {
+                    const double u = ou_update(A.deps[x], A.invtau[site], A.coeff[site], A.subdt, A.sqrt_subdt, A.ns,
+                                               A.seed, A.traj0 + bb, step, site);
+                    A.deps[x] = u;
+                    v[0] = __dadd_rn(u, A.eps[x]);
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < TPT; ++t) {
+                    if (A.noise == DQ_NOISE_GAUSS)
+                        v[t] = __dadd_rn(__dmul_rn(normal(A.seed, P_GAUSS, A.traj0 + bb + t, step, site, 0),
+                                                   A.sigma[site]), A.eps[x + t]);
+                    else if (A.noise == DQ_NOISE_ZZ)
+                        v[t] = __dadd_rn(D[x + t], A.eps[x + t]);
+                    else
+                        v[t] = A.eps[x + t];
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) {
+                dg[x + t] = (Real)v[t];
+                dsm[l + t] = (Real)v[t];
+            }
+        }
+    }
+    if (threadIdx.x < TC) {
+        const double s1 = c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
+        scs[TC + threadIdx.x] = s1;
+        par[TC + threadIdx.x] = make_double2(s1, 0.0);
+        mtr[threadIdx.x] = 0;
+    }
+    sum.sync();   // every CTA of the cluster runs; the window is in place
+
+    const Real* wcol = cur - (ptrdiff_t)r0 * rowr + 2 * tl * TPT;   // this thread's values of global row 0
+    // H_off r_j of block k
+    auto product = [&](int k, CV<Real, TPT> (&acc)[R]) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+            for (int v = 0; v < 2 * TPT; ++v) acc[i].v[v] = 0;
+        cl_gather<Real, TPT, R>(bptr[k] - ebase, bptr[k + 1] - ebase, col, rec, wcol, rowr, acc);
+    };
+    // the neighbours' rows of the window's margins, as they are in their shared memory
+    auto margins = [&]() {
+        if constexpr (!kLocal) {
+            const int nh = act ? hlo + hhi : 0;
+            for (int h0 = rl; h0 < nh; h0 += 4 * RL) {
+                T v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int h = h0 + q * RL;
+                    if (h >= nh) break;
+                    const int g = r0 + (h < hlo ? h - hlo : nrow + h - hlo), own = g / A.rpc;
+                    v[q] = cl_load(reinterpret_cast<const T*>(cur + (size_t)(g - own * A.rpc) * rowr) + tl, own);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int h = h0 + q * RL;
+                    if (h >= nh) break;
+                    const int row = h < hlo ? h - hlo : nrow + h - hlo;
+                    reinterpret_cast<T*>(cur + (ptrdiff_t)row * rowr)[tl] = v[q];
+                }
+            }
+        }
+    };
+
+    const bool adaptive = A.S.mtraj != nullptr;
+    int jl = A.m;   // iterations done
+    for (int j = 1; j <= A.m; ++j) {
+        // u = H r_j - (beta_{j-1} sc_{j-1} / sc_j) r_{j-1} over r_{j-1} (w = sc_j u); alpha_j
+        double x2[TPT], y2[TPT], sc[TPT];
+        Real fm[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+            const double2 p = par[TC + tl * TPT + t];
+            sc[t] = p.x;
+            fm[t] = (Real)p.y;
+            x2[t] = y2[t] = 0.0;
+        }
+        for (int k = rl; k < nbk; k += RL) {
+            CV<Real, TPT> acc[R];
+            product(k, acc);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = k * R + i;
+                if (row >= nrow) break;
+                const size_t l = loc(row);
+                const CV<Real, TPT> x = ldv<Real, TPT, false>(cur, l);
+                CV<Real, TPT> o = x;
+                if (j > 1) o = ldv<Real, TPT, false>(prev, l);
+#pragma unroll
+                for (int t = 0; t < TPT; ++t) {
+                    const Real dv = dsm[l + t];
+                    const Real ur = fma(dv, x.v[2 * t], fma(-fm[t], o.v[2 * t], acc[i].v[2 * t]));
+                    const Real ui = fma(dv, x.v[2 * t + 1], fma(-fm[t], o.v[2 * t + 1], acc[i].v[2 * t + 1]));
+                    o.v[2 * t] = ur;
+                    o.v[2 * t + 1] = ui;
+                    const double xr = x.v[2 * t], xi = x.v[2 * t + 1], dr = ur, di = ui;
+                    if (A.bil) {
+                        x2[t] += xr * dr - xi * di;
+                        y2[t] += xr * di + xi * dr;
+                    } else {
+                        x2[t] += xr * dr + xi * di;
+                        y2[t] += xr * di - xi * dr;
+                    }
+                }
+                stv<Real, TPT>(prev, l, o);
+            }
+        }
+        sum.template part<true>(0, x2, y2);
+        sum.sync();
+        if (threadIdx.x < TC) {
+            const int t = threadIdx.x;
+            const double2 a = sum.get(0, t);
+            const double s = scs[j * TC + t], ar = a.x * s * s, ai = a.y * s * s;
+            al[j * TC + t] = make_double2(ar, ai);
+            par[t] = make_double2(ar * s, ai * s);
+        }
+        __syncthreads();
+        // r_{j+1} = w - alpha_j q_j over r_j, r_j over r_{j-1}; beta_j
+        double2 aj[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) {
+            aj[t] = par[tl * TPT + t];
+            x2[t] = 0.0;
+        }
+        Real* out = slab(j + 1);
+        for (int k = rl; k < nbk; k += RL)
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = k * R + i;
+                if (row >= nrow) break;
+                const size_t l = loc(row);
+                const CV<Real, TPT> x = ldv<Real, TPT, false>(cur, l);
+                CV<Real, TPT> o = ldv<Real, TPT, false>(prev, l);
+#pragma unroll
+                for (int t = 0; t < TPT; ++t) {
+                    const double xr = x.v[2 * t], xi = x.v[2 * t + 1];
+                    o.v[2 * t] = (Real)(sc[t] * (double)o.v[2 * t] - (aj[t].x * xr - aj[t].y * xi));
+                    o.v[2 * t + 1] = (Real)(sc[t] * (double)o.v[2 * t + 1] - (aj[t].x * xi + aj[t].y * xr));
+                    const double rr = o.v[2 * t], ri = o.v[2 * t + 1];
+                    x2[t] += rr * rr + ri * ri;
+                }
+                stv<Real, TPT>(prev, l, x);
+                stv<Real, TPT>(cur, l, o);
+                stv<Real, TPT>(out, glo(row), o);
+            }
+        sum.template part<false>(1, x2, y2);
+        sum.sync();
+        if (threadIdx.x < TC) {
+            const int t = threadIdx.x;
+            const double b2 = sum.get(1, t).x;
+            // 1 / beta and beta; sqrt only where the reciprocal has no value
+            double s1 = rsqrt(b2), bt = b2 * s1;
+            if (!(b2 > 1e-290) || !(b2 < 1e290)) {
+                bt = sqrt(b2);
+                s1 = bt > 0.0 ? 1.0 / bt : 0.0;
+            }
+            if (!isfinite(bt) && c0 + t < B && rank == 0) atomicCAS(A.S.status, 0, DQ_ERR_NAN);
+            // lucky breakdown: invariant Krylov space, continue with q_{j+1} = 0
+            const double bp = j > 1 ? be[(j - 1) * TC + t] : 0.0;
+            const double2 a = al[j * TC + t];
+            if (bt <= 2.0 * kBreakdownRel * (fabs(a.x) + fabs(a.y) + bp) &&
+                bt <= kBreakdownRel * (sqrt(a.x * a.x + a.y * a.y) + bp)) {
+                bt = 0.0;
+                s1 = 0.0;
+            }
+            be[j * TC + t] = bt;
+            scs[(j + 1) * TC + t] = s1;
+            // beta_j sc_j / sc_{j+1} = beta_j^2 sc_j
+            par[TC + t] = make_double2(s1, bt * (bt * scs[j * TC + t]));
+        }
+        margins();
+        __syncthreads();
+        if (adaptive && j >= A.m_min && j < A.m && (j - A.m_min) % kMCheckStride == 0) {
+            // EXPOKIT's first term per undecided trajectory; every CTA decides alike
+            if (threadIdx.x == 0) flag = 0;
+            __syncthreads();
+            for (int t = warp; t < TC; t += kClWarps) {
+                if (c0 + t >= B || mtr[t]) continue;
+                const int q = (min(lane, j - 1) + 1) * TC + t;
+                cd y, f1, f2;
+                int s;
+                const bool ok = series_exp_tbar(j, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
+                if (ok && s >= 0 && lane == j - 1 && fabs(be[q]) * sqrt(cabs2(f1)) <= A.tol) mtr[t] = j;
+                if (!ok && lane == 0) atomicOr(&flag, 1);
+            }
+            __syncthreads();
+            if (flag) {
+                // the dense form on rank 0, the choices through global memory
+                __shared__ cd ald[kMaxL], bed[kMaxL];
+                if (rank == 0) {
+                    for (int t = 0; t < TC && c0 + t < B; ++t) {
+                        int mt = mtr[t];
+                        __syncthreads();
+                        if (mt == 0) {
+                            for (int i = threadIdx.x; i <= j + 1; i += kClThreads) {
+                                ald[i] = i >= 1 && i <= j ? cmk(al[i * TC + t].x, al[i * TC + t].y) : cmk(0, 0);
+                                bed[i] = i >= 1 && i <= j ? cmk(be[i * TC + t], 0.0) : cmk(0, 0);
+                            }
+                            __syncthreads();
+                            const PadeOut o = cl_dense(j, ald, bed, A.tau_im, A.norm_mode, nullptr,
+                                                       A.scratch + chunk * A.scratch_stride);
+                            if (o.s >= 0 && fabs(bed[j].x) * sqrt(cabs2(o.e_m1_m)) <= A.tol) mt = j;
+                            __syncthreads();
+                        }
+                        if (threadIdx.x == 0) A.S.mtraj[c0 + t] = mt;
+                    }
+                }
+                sum.sync();
+                if (threadIdx.x < TC && c0 + (int)threadIdx.x < B) mtr[threadIdx.x] = A.S.mtraj[c0 + threadIdx.x];
+                sum.sync();   // rank 0 may write the choices again only after all have read them
+            }
+            bool done = true;
+            for (int t = 0; t < TC && c0 + t < B; ++t) done = done && mtr[t] != 0;
+            if (done) {
+                jl = j;
+                break;
+            }
+        }
+    }
+    // ---- the recurrence's scalars (the adjoint and the getters read them) ----
+    __syncthreads();
+    if (rank == 0) {
+        for (int e = threadIdx.x; e < jl * TC; e += kClThreads) {
+            const int j = 1 + e / TC, t = e % TC;
+            if (c0 + t >= B) continue;
+            const size_t k = (size_t)j * B + c0 + t;
+            A.S.alpha[2 * k] = al[j * TC + t].x;
+            A.S.alpha[2 * k + 1] = al[j * TC + t].y;
+            A.S.beta[k] = be[j * TC + t];
+            A.S.sc[k + B] = scs[(j + 1) * TC + t];
+        }
+    }
+    if (!(A.flags & kClFinish)) {
+        // the neighbours may still read this CTA's rows of the last window
+        if constexpr (!kLocal) cl_sync();
+        return;
+    }
+    // ---- ||H q_{m+1}|| ---------------------------------------------------------
+    double nav = 0.0;   // set where it is used, per trajectory
+    if (!adaptive) {
+        double x2[TPT];
+#pragma unroll
+        for (int t = 0; t < TPT; ++t) x2[t] = 0.0;
+        for (int k = rl; k < nbk; k += RL) {
+            CV<Real, TPT> acc[R];
+            product(k, acc);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int row = k * R + i;
+                if (row >= nrow) break;
+                const size_t l = loc(row);
+                const CV<Real, TPT> x = ldv<Real, TPT, false>(cur, l);
+#pragma unroll
+                for (int t = 0; t < TPT; ++t) {
+                    const Real dv = dsm[l + t];
+                    const double ur = fma(dv, x.v[2 * t], acc[i].v[2 * t]);
+                    const double ui = fma(dv, x.v[2 * t + 1], acc[i].v[2 * t + 1]);
+                    x2[t] += ur * ur + ui * ui;
+                }
+            }
+        }
+        sum.template part<false>(0, x2, x2);
+        sum.sync();
+    }
+    // ---- exp(tau Tbar) e_1: one warp per trajectory, in every CTA -------------
+    if (threadIdx.x == 0) flag = 0;
+    __syncthreads();
+    auto estimate = [&](int m, int t, cd e1, cd e2) {
+        const double bmm = be[m * TC + t];
+        // with the adaptive dimension only err1 (||H q_{m+1}|| belongs to the largest m)
+        return adaptive ? fmax(fabs(bmm) * sqrt(cabs2(e1)), 1.110223e-16) : expokit_error(bmm, nav, e1, e2);
+    };
+    int mmax = adaptive ? 0 : A.m;
+    for (int t = 0; t < TC && c0 + t < B; ++t)
+        if (adaptive) mmax = max(mmax, mtr[t] ? mtr[t] : A.m);
+    __syncthreads();   // before a warp below marks its trajectory
+    for (int t = warp; t < TC; t += kClWarps) {
+        if (c0 + t >= B) continue;
+        const int m = adaptive && mtr[t] ? mtr[t] : A.m;
+        const int q = (min(lane, m - 1) + 1) * TC + t;
+        cd y, f1, f2;
+        int s;
+        const bool ok = series_exp_tbar(m, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
+        if (!ok) {
+            if (lane == 0) atomicOr(&flag, 1);
+            if (lane == 0) mtr[t] = -m;   // dense below
+            continue;
+        }
+        if (lane < mmax) {
+            const cd v = lane < m ? cscale(y, scs[(lane + 1) * TC + t]) : cmk(0.0, 0.0);
+            yts[lane * TC + t] = make_double2(v.x, v.y);
+        }
+        if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
+        if (rank == 0 && lane == m - 1) {
+            if (s < 0) atomicCAS(A.S.status, 0, DQ_ERR_SCALING);
+            else A.erracc[c0 + t] += estimate(m, t, f1, f2);
+        }
+        if (adaptive && rank == 0 && lane == 0) A.S.mtraj[c0 + t] = m;
+    }
+    __syncthreads();
+    if (flag) {
+        __shared__ cd ald[kMaxL], bed[kMaxL], yd[kMaxM];
+        if (rank == 0) {
+            for (int t = 0; t < TC && c0 + t < B; ++t) {
+                if (mtr[t] >= 0) continue;
+                const int m = -mtr[t];
+                for (int i = threadIdx.x; i <= m + 1; i += kClThreads) {
+                    ald[i] = i >= 1 && i <= m ? cmk(al[i * TC + t].x, al[i * TC + t].y) : cmk(0, 0);
+                    bed[i] = i >= 1 && i <= m ? cmk(be[i * TC + t], 0.0) : cmk(0, 0);
+                }
+                __syncthreads();
+                const PadeOut o = cl_dense(m, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
+                __syncthreads();
+                if (o.s < 0 && threadIdx.x == 0)
+                    atomicCAS(A.S.status, 0, o.s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
+                for (int j = threadIdx.x; j < mmax; j += kClThreads) {
+                    const cd v = j < m && o.s >= 0 ? cscale(yd[j], scs[(j + 1) * TC + t]) : cmk(0.0, 0.0);
+                    const size_t k = (size_t)(j + 1) * B + c0 + t;
+                    A.S.yt[2 * k] = v.x;
+                    A.S.yt[2 * k + 1] = v.y;
+                }
+                if (threadIdx.x == 0 && o.s >= 0) {
+                    if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
+                    A.erracc[c0 + t] += estimate(m, t, o.e_m1_m, o.e_m1_mp1);
+                }
+                if (adaptive && threadIdx.x == 0) A.S.mtraj[c0 + t] = m;
+                __syncthreads();
+            }
+        }
+        sum.sync();
+        for (int e = threadIdx.x; e < mmax * TC; e += kClThreads) {
+            const int j = e / TC, t = e % TC;
+            if (c0 + t >= B || mtr[t] >= 0) continue;
+            const size_t k = (size_t)(j + 1) * B + c0 + t;
+            yts[e] = make_double2(A.S.yt[2 * k], A.S.yt[2 * k + 1]);
+        }
+        __syncthreads();
+    }
+    // ---- psi = sum_j yt_j r_j over slab 1, its norm, <bra|psi> -----------------
+    double nn[TPT], cr[TPT], ci[TPT];
+#pragma unroll
+    for (int t = 0; t < TPT; ++t) nn[t] = cr[t] = ci[t] = 0.0;
+    for (int k = rl; k < nbk; k += RL)
+        for (int row = k * R; row < min(nrow, k * R + R); ++row) {
+            const size_t x = glo(row);
+            double pr[TPT], pi[TPT];
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) pr[t] = pi[t] = 0.0;
+            for (int j0 = 1; j0 <= mmax; j0 += 8) {
+                CV<Real, TPT> v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (j0 + q <= mmax) v[q] = ldv<Real, TPT, false>(slab(j0 + q), x);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    if (j0 + q > mmax) break;
+#pragma unroll
+                    for (int t = 0; t < TPT; ++t) {
+                        const double2 yv = yts[(j0 + q - 1) * TC + tl * TPT + t];
+                        pr[t] += yv.x * v[q].v[2 * t] - yv.y * v[q].v[2 * t + 1];
+                        pi[t] += yv.x * v[q].v[2 * t + 1] + yv.y * v[q].v[2 * t];
+                    }
+                }
+            }
+            const cd p0 = A.bra[r0 + row];
+            CV<Real, TPT> o;
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) {
+                o.v[2 * t] = (Real)pr[t];
+                o.v[2 * t + 1] = (Real)pi[t];
+                const double vr = o.v[2 * t], vi = o.v[2 * t + 1];
+                nn[t] += vr * vr + vi * vi;
+                cr[t] += p0.x * vr + p0.y * vi;   // conj(bra) * psi
+                ci[t] += p0.x * vi - p0.y * vr;
+            }
+            stv<Real, TPT>(slab(1), x, o);
+        }
+    // ex[0] still holds ||H q_{m+1}||, which slower CTAs may be reading
+    sum.sync();
+    sum.template part<true>(0, cr, ci);
+    sum.template part<false>(1, nn, nn);
+    sum.sync();
+    if (rank == 0) {
+        double* cs = reinterpret_cast<double*>(sum.red);   // free again: the chunk's correlation terms
+        if (threadIdx.x < TC) {
+            const int t = threadIdx.x, b = c0 + t;
+            double sr = 0.0, si = 0.0;
+            if (b < B) {
+                const double n2 = sum.get(1, t).x;
+                const double2 c = sum.get(0, t);
+                const double s1 = 1.0 / sqrt(n2);
+                A.S.norm2[b] = n2;
+                A.S.sc[(size_t)B + b] = s1;   // next step's q_1 = psi / ||psi||
+                if (!(n2 > 0.0) || !isfinite(n2)) atomicCAS(A.S.status, 0, DQ_ERR_NAN);
+                sr = c.x * s1;
+                si = c.y * s1;
+            }
+            cs[2 * t] = sr;
+            cs[2 * t + 1] = si;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sr = 0.0, si = 0.0;
+            for (int t = 0; t < TC; ++t) {
+                sr += cs[2 * t];
+                si += cs[2 * t + 1];
+            }
+            double* cp = A.S.corr + ((size_t)(*A.S.step + 1) * A.chunks + chunk) * 2;
+            cp[0] = sr;
+            cp[1] = si;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+using ClKernel = void (*)(const ClusterArgs);
+
+template <typename Real, int TPT>
+static ClKernel cl_pick(int R, bool local) {
+    switch (R) {
+        case 1: return local ? k_cluster_step<Real, TPT, 1, true> : k_cluster_step<Real, TPT, 1, false>;
+        case 2: return local ? k_cluster_step<Real, TPT, 2, true> : k_cluster_step<Real, TPT, 2, false>;
+        case 3:
+            if constexpr (sizeof(Real) == 4)
+                return local ? k_cluster_step<Real, TPT, 3, true> : k_cluster_step<Real, TPT, 3, false>;
+            return nullptr;
+        case 4:
+            if constexpr (sizeof(Real) == 8)
+                return local ? k_cluster_step<Real, TPT, 4, true> : k_cluster_step<Real, TPT, 4, false>;
+            return nullptr;
+        default: return nullptr;
+    }
+}
+
+static ClKernel cl_kernel(bool mixed, int tpt, int R, bool local) {
+    if (!mixed) return cl_pick<double, 1>(R, local);
+    return tpt == 2 ? cl_pick<float, 2>(R, local) : nullptr;
+}
+
+static const ::BlockFmt& cl_fmt(const BatchedState* bs, int R) {
+    return bs->fmt[R == 1 ? 0 : R == 2 ? 1 : R == 3 ? 2 : 3];
+}
+
+static int cl_rows(int n, int CS, int R) {
+    const int rpc = (n + CS - 1) / CS;
+    return (rpc + R - 1) / R * R;
+}
+
+static cudaLaunchConfig_t cl_config(int chunks, int CS, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(chunks * CS);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = CS;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Bytes of the largest CTA's coupling records (block starts, columns, coefficients).
+static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R) {
+    const size_t nb = rpc / R, ne = nb * (size_t)f.max_block;
+    const size_t head = ((nb + 1) * 4 + 15) / 16 * 16;
+    if (mixed) return head + ne * 16;
+    return head + (ne * 4 + 15) / 16 * 16 + ne * R * sizeof(double);
+}
+
+// Clusters of this shape that the device holds at once (0: it cannot run);
+// *smem its dynamic shared memory, *rec the part that holds the records (0
+// when they do not fit).
+static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::BlockFmt& f, size_t* smem, size_t* rec) {
+    const BatchedState* bs = c->bat;
+    const int n = c->n, m = c->cfg.m;
+    if (CS < 1 || CS > kClMaxCtas || (CS & (CS - 1))) return 0;
+    if (tc < tpt || tc > kMaxTC || tc % tpt || ((tc / tpt) & (tc / tpt - 1)) || tc / tpt > 32) return 0;
+    ClKernel k = cl_kernel(bs->mixed, tpt, R, CS == 1);
+    if (!k) return 0;
+    const size_t rsz = bs->mixed ? sizeof(float) : sizeof(double);
+    const int rpc = cl_rows(n, CS, R);
+    size_t rb = cl_rec_bytes(f, bs->mixed, rpc, R);
+    size_t sm = cl_layout(CS, tc, m, rpc, c->bw, rsz, rb).total;
+    if (sm > kClSmemMax) {
+        rb = 0;
+        sm = cl_layout(CS, tc, m, rpc, c->bw, rsz, 0).total;
+    }
+    if (sm > kClSmemMax) return 0;
+    int found = 0;
+    if (raise_smem_limit(k, (int)kClSmemMax) == cudaSuccess &&
+        (CS <= 8 || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = cl_config(1, CS, sm, nullptr, &at);
+        if (cudaOccupancyMaxActiveClusters(&found, k, &cfg) != cudaSuccess) found = 0;
+    }
+    cudaGetLastError();
+    *smem = sm;
+    *rec = rb;
+    return found;
+}
+
+// One cluster launch: the whole step (flags kClNoise | kClFinish), or the
+// Lanczos iterations of a given slab 1 and diagonal alone (flags 0).
+cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
+    BatchedState* bs = c->bat;
+    const ::BlockFmt& f = cl_fmt(bs, bs->R);
+    ClusterArgs a = {};
+    a.n = c->n;
+    a.B = bs->B;
+    a.TC = bs->TC;
+    a.rpc = bs->rpc;
+    a.bw = c->bw;
+    a.rec_smem = (int)bs->cl_rec;
+    a.m = c->cfg.m;
+    a.flags = whole_step ? kClNoise | kClFinish : 0;
+    a.bil = c->cfg.dot_mode == DQ_DOT_BILINEAR;
+    a.chunks = bs->chunks;
+    a.bptr = f.bptr;
+    a.bcol = f.bcol;
+    a.bcoef = f.bcoef;
+    a.slabs = bs->slabs;
+    a.slab = (size_t)c->n * bs->B;
+    a.diag = bs->diag;
+    a.S = bs->s;
+    a.noise = c->cfg.noise_model;
+    a.ns = c->cfg.ka_substeps > 0 ? c->cfg.ka_substeps : 1;
+    a.traj0 = c->traj0;
+    a.subdt = c->cfg.dt / (double)a.ns;
+    a.sqrt_subdt = sqrt(a.subdt);
+    a.seed = c->cfg.seed;
+    a.sigma = c->d_sigma;
+    a.invtau = c->d_invtau;
+    a.coeff = c->d_coeff;
+    a.eps = bs->eps;
+    a.deps = bs->deps;
+    a.zzD = zz.D;
+    a.zz_start = zz.start;
+    a.norm_mode = c->cfg.norm_mode;
+    a.m_min = c->cfg.m_min;
+    a.tol = c->cfg.m_tol > 0 ? c->cfg.m_tol : 1e-7;
+    a.tau_im = c->tau_im;
+    a.erracc = c->d_erracc;
+    a.bra = corr_bra(c);
+    a.scratch = static_cast<unsigned char*>(bs->cl_scratch);
+    a.scratch_stride = pade_smem_bytes(c->cfg.m + 2);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cl_config(bs->chunks, bs->ctas_per_sm, bs->win_smem, c->stream, &at);
+    return cudaLaunchKernelEx(&cfg, cl_kernel(bs->mixed, bs->TPT, bs->R, bs->ctas_per_sm == 1), a);
+}
+
+// Shapes `bs` for the cluster form (its coupling blocks of R rows exist).
+dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R) {
+    BatchedState* bs = c->bat;
+    size_t smem = 0, rec = 0;
+    if (cluster_resident(c, tc, tpt, CS, R, cl_fmt(bs, R), &smem, &rec) < 1) return DQ_ERR_ARG;
+    const int chunks = (bs->B + tc - 1) / tc;
+    const size_t need = (size_t)chunks * pade_smem_bytes(c->cfg.m + 2);
+    if (need > bs->cl_scratch_bytes) {
+        cudaFree(bs->cl_scratch);
+        bs->cl_scratch = nullptr;
+        bs->cl_scratch_bytes = 0;
+        dq_status st = check_cuda(c, cudaMalloc(&bs->cl_scratch, need), "cluster scratch");
+        if (st) return st;
+        bs->cl_scratch_bytes = need;
+    }
+    bs->TC = tc;
+    bs->TPT = tpt;
+    bs->chunks = chunks;
+    bs->ctas_per_sm = CS;
+    bs->R = R;
+    bs->rpc = cl_rows(c->n, CS, R);
+    bs->gx = bs->gxs = CS;
+    bs->win_smem = smem;
+    bs->cl_rec = rec;
+    bs->staged = kStagedCluster;
+    bs->groups = 1;
+    return DQ_OK;
+}
+
+}  // namespace dq
