@@ -43,6 +43,21 @@ constexpr int kAdjMaxClasses = 8; // coupling classes with a gradient of their o
 // contiguous head of a workspace's scalar block
 inline size_t scal_block(int B) { return (size_t)4 * kMaxL * B; }
 
+// Slabs 2.. of a Krylov basis hold chunks of `tc` trajectories one after
+// another, [chunk][site][trajectory of the chunk] (tc = B: plain
+// [site][trajectory]); the state itself (slab 1) is always plain.  A thread's
+// trajectory b on row i is at base + i * stride.
+struct BasisLane {
+    size_t base;
+    int stride;
+    __device__ __forceinline__ BasisLane(int n, int B, int tc, int b) {
+        const int c0 = b / tc * tc;
+        base = (size_t)c0 * n + (b - c0);
+        stride = min(tc, B - c0);
+    }
+    __device__ __forceinline__ size_t at(int row) const { return base + (size_t)row * stride; }
+};
+
 template <typename Real> struct R2;
 template <> struct R2<float> { using T = float2; };
 template <> struct R2<double> { using T = double2; };
@@ -67,6 +82,7 @@ struct AdjointState {
     // the next segment is recomputed into the other on a second stream
     // (absent when the memory is short; the sweep then waits for each recompute)
     unsigned char* seg_V2 = nullptr;
+    int seg_tc = 0, seg_tc2 = 0;         // basis layout of each set (the tiling may change between the passes)
     double* seg_sc2 = nullptr;
     unsigned char* seg_diag2 = nullptr;
     cudaStream_t rstream = nullptr;
@@ -319,7 +335,7 @@ __global__ void __launch_bounds__(256) k_adj_small(int m, int B, double tau_im, 
 // Sums over the CTA's trajectories go to gsite/gcpl[row][traj group] (one
 // writer each, deterministic); |lambda|^2 partials to lpart[cta][b].
 template <typename Real, int MM>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m, int rows_per_cta, int G,
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m, int tcv, int tcw, int rows_per_cta, int G,
                                                          const Real* __restrict__ sV, Real* sW, size_t slab_reals,
                                                          const Real* __restrict__ d, const cd* __restrict__ psi0,
                                                          const cd* __restrict__ Gt, double invB, int write_lam,
@@ -344,18 +360,20 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m
     const cd g = Gt[0];
     const double sr = g.x * invB, si = -g.y * invB;
     const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
+    const BasisLane bv(n, B, tcv, b), bw(n, B, tcw, b);
     double lnn = 0.0;
     // uniform trip count across the warp: the trajectory-lane shuffles below
     // need every lane
     for (int base = r0; base < r1; base += kRowLanes) {
         const int row = base + rl;
         const bool valid = row < r1;
-        const size_t x = (size_t)(valid ? row : r0) * B + b;
+        const size_t x = (size_t)(valid ? row : r0) * B + b, xv = bv.at(valid ? row : r0),
+                     xw = bw.at(valid ? row : r0);
         Real vr[MM + 1], vi[MM + 1];
 #pragma unroll
         for (int c = 0; c <= MM; ++c) {
             if (c <= m) {
-                const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * x);
+                const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * (c ? xv : x));
                 vr[c] = v.x;
                 vi[c] = v.y;
             } else {
@@ -370,7 +388,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m
         // loads overlap the products
         auto ldw = [&](int a) {
             T2 v;
-            if (a < m) v = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * x);
+            if (a < m) v = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * (a ? xw : x));
             else { v.x = 0; v.y = 0; }
             return v;
         };
@@ -446,7 +464,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m
 // skip0, class-0 entries are left out: their sum follows on the host from the
 // total off-diagonal form (free from the Lanczos relation in k_adj_grad).
 template <typename Real, int MM>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m, int rows_per_cta, int G, int C,
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m, int tcv, int tcw, int rows_per_cta, int G, int C,
                                                         const Real* __restrict__ sV, const Real* __restrict__ sW,
                                                         size_t slab_reals, const int* __restrict__ rowptr,
                                                         const int* __restrict__ col, const int* __restrict__ cls,
@@ -466,15 +484,17 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m,
     }
     __syncthreads();
     const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
+    const BasisLane bv(n, B, tcv, b), bw(n, B, tcw, b);
     for (int base = r0; base < r1; base += kRowLanes) {
         const int row = base + rl;
         const bool valid = row < r1;
-        const size_t x = (size_t)(valid ? row : r0) * B + b;
+        const int own = valid ? row : r0;
+        const size_t x = (size_t)own * B + b, xw = bw.at(own);
         Real tr[MM], ti[MM];
 #pragma unroll
         for (int c = 0; c < MM; ++c) { tr[c] = 0; ti[c] = 0; }
         for (int a = 0; a < m; ++a) {
-            const T2 w = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * x);
+            const T2 w = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * (a ? xw : x));
 #pragma unroll
             for (int c = 0; c < MM; ++c) {
                 if (c < m) {
@@ -497,16 +517,16 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m,
             const int pe = rowptr[row + 1];
             int p = rowptr[row];
             while (p < pe) {
-                size_t xk[KP];
+                int xk[KP];
                 int qk[KP];
                 double vk[KP];
 #pragma unroll
-                for (int k = 0; k < KP; ++k) { xk[k] = x; qk[k] = 0; vk[k] = 0.0; }
+                for (int k = 0; k < KP; ++k) { xk[k] = own; qk[k] = 0; vk[k] = 0.0; }
                 int nk = 0;
                 for (; p < pe && nk < KP; ++p) {
                     const int q = cls[p];
                     if (skip0 && q == 0) continue;
-                    const size_t xv = (size_t)col[p] * B + b;
+                    const int xv = col[p];
                     const double vv = vbase[p];
 #pragma unroll
                     for (int k = 0; k < KP; ++k)   // register slots, no indexed local array
@@ -522,7 +542,8 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m,
                     if (c < m) {
 #pragma unroll
                         for (int k = 0; k < KP; ++k) {   // unused slots read the own row, weight 0
-                            const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * xk[k]);
+                            const size_t xv = c ? bv.at(xk[k]) : (size_t)xk[k] * B + b;
+                            const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * xv);
                             rr[k] = fma(tr[c], v.x, fma(-ti[c], v.y, rr[k]));   // Re(t v)
                         }
                     }
@@ -633,6 +654,7 @@ static cudaError_t grad_attr(int bytes) {
 static void use_set(AdjointState* a, int k) {
     if (!a->seg_V2 || a->cur_set == k) return;
     std::swap(a->seg_V, a->seg_V2);
+    std::swap(a->seg_tc, a->seg_tc2);
     std::swap(a->seg_sc, a->seg_sc2);
     std::swap(a->seg_diag, a->seg_diag2);
     a->cur_set = k;
@@ -653,7 +675,7 @@ static void launch_grad(dq_ctx* c, AdjointState* a, int t, int slot, int write_l
     using T2 = typename R2<Real>::T;
 #define DQ_GRAD(MMV)                                                                                               \
     k_adj_grad<Real, MMV><<<grid, kAdjThreads, smem, c->stream>>>(                                                  \
-        n, B, m, a->rows_per_cta, G, (const Real*)slot_V(a, m, slot), (Real*)a->ws2->slabs, slab_reals,          \
+        n, B, m, a->seg_tc, batched_basis_chunk(a->ws2), a->rows_per_cta, G, (const Real*)slot_V(a, m, slot), (Real*)a->ws2->slabs, slab_reals,          \
         (const Real*)(a->seg_diag + (size_t)slot * a->diag_bytes),                                                 \
         c->d_psi0, a->d_G + t, a->inv_norm, write_lam, (const T2*)a->d_coef, a->d_lpart, a->d_gsite, a->d_gcpl)
     switch (mm_bucket(m)) {
@@ -673,7 +695,7 @@ static void launch_cls(dq_ctx* c, AdjointState* a, int slot) {
     const dim3 grid(a->row_ctas, G);
     using T2 = typename R2<Real>::T;
 #define DQ_CLS(MMV)                                                                                                  \
-    k_adj_cls<Real, MMV><<<grid, kAdjThreads, smem, c->stream>>>(n, B, m, a->rows_per_cta, G, a->n_cls,                \
+    k_adj_cls<Real, MMV><<<grid, kAdjThreads, smem, c->stream>>>(n, B, m, a->seg_tc, batched_basis_chunk(a->ws2), a->rows_per_cta, G, a->n_cls,                \
                                                                (const Real*)slot_V(a, m, slot),                      \
                                                                (const Real*)a->ws2->slabs,                           \
                                                                slab_reals, c->d_rowptr, c->d_col, a->d_cls,           \
@@ -716,6 +738,7 @@ static dq_status run_segment(dq_ctx* c, AdjointState* a, int s0, int s1, bool re
     BatchedState* bs = c->bat;
     const int m = c->cfg.m;
     dq_status hook_st = DQ_OK;
+    a->seg_tc = batched_basis_chunk(bs);
     for (int k = s0; k < s1; ++k) {
         const int slot = k - s0;
         unsigned char* V = slot_V(a, m, slot);
@@ -1047,8 +1070,7 @@ dq_status dq_backward(dq_ctx* c, double* grad_sites, double* grad_classes) {
             const int slot = t - s0;
             DQ_CU(cudaMemcpyAsync(w2->diag, a->seg_diag + (size_t)slot * a->diag_bytes, a->diag_bytes,
                                   cudaMemcpyDeviceToDevice, c->stream));
-            for (int j = 1; j <= m; ++j)
-                if ((st = batched_iteration(c, w2, j))) return st;
+            if ((st = batched_krylov(c, w2))) return st;
             // the kept step's tridiagonal and scales, in the workspace layout
             BatchedScalars SV = bs->s;
             SV.alpha = a->seg_sc + (size_t)slot * scal_block(B);

@@ -726,10 +726,11 @@ extern "C" dq_status dq_autotune(dq_ctx* c, int reps, double* best_ms) {
     double best = 1e30;
     const int vecs[2] = {2, 1};
     for (int groups = 1; groups <= 8; groups <<= 1)
-        for (int staged = 0; staged <= 12; ++staged)
+        for (int staged = 0; staged <= 13; ++staged)
             for (int vi = 0; vi < 2; ++vi)
-                for (int tc = 4; tc <= 64; tc <<= 1)
-                    for (int cps = 1; cps <= 8; cps <<= 1)
+                for (int tc = staged == 13 ? 1 : 4; tc <= 64; tc <<= 1)
+                    // form 13: CTAs per cluster, any number up to 16
+                    for (int cps = 1; cps <= (staged == 13 ? 16 : 8); cps += staged == 13 ? 1 : cps)
                         for (int R : {1, 2, 3, 4, 8}) {
                             if (batched_set_tiling(c, tc, vecs[vi], cps, R, staged, groups) != DQ_OK) continue;
                             double ms = 0.0;

@@ -3229,6 +3229,7 @@ static dq_status build_fmt(dq_ctx* c, int R, BlockFmt& f) {
     }
     if (R == 3) return DQ_ERR_ARG;   // three rows per block only in the packed (complex64) form
     f.nunion = bcol.size();
+    for (int k = 0; k < nb; ++k) f.max_block = std::max(f.max_block, bptr[k + 1] - bptr[k]);
     const size_t nu = std::max<size_t>(f.nunion, 1);
     DQ_CU(cudaMalloc(&f.bptr, sizeof(int) * (nb + 1)));
     DQ_CU(cudaMalloc(&f.bcol, sizeof(int) * nu));
@@ -3480,6 +3481,19 @@ dq_status batched_set_tiling(dq_ctx* c, int tc, int tpt, int ctas_per_sm, int R,
     const int B = bs->B, n = c->n;
     if (tpt != 1 && tpt != 2) return DQ_ERR_ARG;
     if (!bs->mixed && tpt != 1) return DQ_ERR_ARG;
+    if (staged == kStagedCluster) {
+        // one launch per step: ctas_per_sm is the CTAs of a cluster; no reorthogonalisation
+        const int ri = r_index(R);
+        if (groups != 1 || c->cfg.reorth || ri < 0 || tc < 1) return DQ_ERR_ARG;
+        if (bs->mixed ? R > 3 : R == 3 || R > 4) return DQ_ERR_ARG;
+        if (!bs->fmt[ri].bptr) {
+            dq_status st = build_fmt(c, R, bs->fmt[ri]);
+            if (st) return st;
+        }
+        dq_status st = cluster_set(c, tc, tpt, ctas_per_sm, R);
+        if (st == DQ_OK) drop_graph(bs);
+        return st;
+    }
     if (tc < tpt || tc > kMaxTC || (tc & (tc - 1)) || B % tc || tc / tpt > kBThreads) return DQ_ERR_ARG;
     if (ctas_per_sm < 1 || ctas_per_sm > 16) return DQ_ERR_ARG;
     if (staged < 0 || staged > 12) return DQ_ERR_ARG;
@@ -3749,7 +3763,8 @@ dq_status batched_invalidate_blocks(dq_ctx* c) {
     drop_graph(bs);
     if (!bs->TC) return DQ_OK;
     dq_status st = batched_set_tiling(c, bs->TC, bs->TPT, bs->ctas_per_sm, bs->R, bs->staged, bs->groups);
-    if (st && bs->staged) st = batched_set_tiling(c, bs->TC, bs->TPT, bs->ctas_per_sm, bs->R, 0, bs->groups);
+    if (st && bs->staged == kStagedCluster) st = batched_default_tiling(c);
+    else if (st && bs->staged) st = batched_set_tiling(c, bs->TC, bs->TPT, bs->ctas_per_sm, bs->R, 0, bs->groups);
     if (st) c->err = "batched: could not rebuild the coupling blocks";
     return st;
 }
@@ -3770,7 +3785,7 @@ dq_status batched_mirror_tiling(dq_ctx* c, BatchedState* dst) {
     dst->staged = src->staged; dst->groups = src->groups; dst->halo = src->halo; dst->wmask = src->wmask;
     dst->rpc_win = src->rpc_win; dst->gxw = src->gxw; dst->bw = src->bw; dst->win_smem = src->win_smem;
     dst->f_sr = src->f_sr; dst->f_hb = src->f_hb; dst->f_D = src->f_D; dst->f_rpc = src->f_rpc;
-    dst->f_gx = src->f_gx; dst->f_smem = src->f_smem; dst->f_rb = src->f_rb;
+    dst->f_gx = src->f_gx; dst->f_smem = src->f_smem; dst->f_rb = src->f_rb; dst->cl_rec = src->cl_rec;
     dst->tmaps.clear();
     dst->fmaps.clear();
     if (src->staged == 2 || src->staged == 4) {
@@ -3854,10 +3869,37 @@ static dq_status alloc_ws_into(dq_ctx* c, BatchedState* bs, int B, bool mixed, b
     return batched_default_tiling(c);
 }
 
+// The tiling of an ensemble that no one tuned, by size: the cluster form where
+// its estimated iteration beats the grid-wide form's estimate.  On a B200, a
+// step: 1,024 sites x 64 FP64 224 us grid-wide, 81 us as clusters; 4,731 x 100
+// with 28 couplings a row 739 and 331; 4,096 x 128 with 8, 375 and 169; 30,000 x
+// 256 does not fit the chip and stays grid-wide.
 dq_status batched_default_tiling(dq_ctx* c) {
     BatchedState* bs = c->bat;
     const int B = bs->B;
-    int tpt = bs->mixed ? 2 : 1;
+    const int tpt = bs->mixed ? 2 : 1;
+    if (!c->cfg.reorth) {
+        // rows per block: three (complex128: two) share a gathered row, one where rows have few couplings
+        const bool wide = c->nnz_off >= 6 * (size_t)c->n;
+        const int R = !wide ? 1 : bs->mixed ? 3 : 2;
+        const double elems = (double)c->n * B, z = (double)c->nnz_off / c->n;
+        // grid-wide forms, cycles per iteration: two launches with their reductions, then the data
+        // (with an adaptive dimension also the checks, and the launches past the chosen one)
+        const double grid = (28000.0 + elems * (bs->mixed ? 0.0075 + 0.00075 * z : 0.02 + 0.0015 * z)) *
+                            (c->cfg.m_min > 0 ? 1.6 : 1.0);
+        // what the cluster form takes at least (the union of R rows' columns has z entries or more),
+        // before any block is built
+        const double least = 5500.0 + elems / bs->sms * (bs->mixed ? 1.2 + 0.13 * z / R : 0.8 + 0.26 * z / R);
+        if (least < grid) {
+            BlockFmt& f = bs->fmt[r_index(R)];
+            dq_status st = DQ_OK;
+            if (!f.bptr && (st = build_fmt(c, R, f))) return st;
+            int tc = 0, cs = 0;
+            if (cluster_plan(c, R, &tc, &cs) < grid &&
+                batched_set_tiling(c, tc, tpt, cs, R, kStagedCluster, 1) == DQ_OK)
+                return DQ_OK;
+        }
+    }
     int tc = 16;
     while (tc > tpt && B % tc) tc >>= 1;
     if (B % tc) tc = tpt;
@@ -3897,6 +3939,7 @@ void batched_free_ws(BatchedState* bs) {
     if (!bs->fmt_borrowed)
         for (auto& f : bs->fmt) free_fmt(f);
     cudaFree(bs->wB);
+    cudaFree(bs->cl_scratch);
     cudaFree(bs->slabs); cudaFree(bs->diag); cudaFree(bs->eps); cudaFree(bs->deps);
     cudaFree(bs->zzD); cudaFree(bs->zz_start);
     cudaFree(bs->scal_mem); cudaFree(bs->s.tickets); cudaFree(bs->s.status); cudaFree(bs->s.mtraj);
@@ -4375,12 +4418,22 @@ static dq_status enqueue_step(dq_ctx* c, StepTimer* tm, const std::function<void
             n, B, c->traj0, c->cfg.seed, zz_params(c), bs->s, bs->zz_start, bs->zzD);
         k_zz_mark<<<1, 1, 0, st>>>(bs->s, bs->zz_start);
     }
-    k_noise_b<Real, TPT><<<grid, kBThreads, 0, st>>>(n, B, c->traj0, TC, rpc, c->cfg.noise_model, ns, subdt, sqrt_subdt,
-                                                     c->cfg.seed, c->d_sigma, c->d_invtau, c->d_coeff, bs->eps,
-                                                     bs->deps, (Real*)bs->diag, bs->s, bs->zzD, bs->zz_start);
+    const bool cluster = bs->staged == kStagedCluster;
+    if (cluster) {
+        // noise to correlation in one launch
+        mark(DQ_KIND_FUSED);
+        dq_status cst = check_cuda(c, cluster_launch(c, true, ZZBlockRef{bs->zzD, bs->zz_start}), "cluster step launch");
+        if (cst) return cst;
+    } else {
+        k_noise_b<Real, TPT><<<grid, kBThreads, 0, st>>>(n, B, c->traj0, TC, rpc, c->cfg.noise_model, ns, subdt,
+                                                         sqrt_subdt, c->cfg.seed, c->d_sigma, c->d_invtau, c->d_coeff,
+                                                         bs->eps, bs->deps, (Real*)bs->diag, bs->s, bs->zzD,
+                                                         bs->zz_start);
+    }
     if (after_noise) (*after_noise)();
     const bool adaptive = bs->s.mtraj != nullptr;
-    if (adaptive) {
+    if (cluster) {
+    } else if (adaptive) {
         // adaptive Krylov dimension: checks after iterations m_min, m_min + 4, ...;
         // chunks whose trajectories all chose skip their remaining iterations
         const int m_min = c->cfg.m_min;
@@ -4407,10 +4460,12 @@ static dq_status enqueue_step(dq_ctx* c, StepTimer* tm, const std::function<void
             }
         }
     }
+    if (!cluster) {
     mark(DQ_KIND_PADE);
     k_pade_b<<<(B + kPadeWarps - 1) / kPadeWarps, 32 * kPadeWarps, pade_smem_bytes(m + 2), st>>>(m, B, c->tau_im, c->cfg.norm_mode, bs->s, c->d_erracc);
     mark(DQ_KIND_COMBINE);
     k_combine_b<Real, TPT><<<grid, kBThreads, 0, st>>>(n, B, TC, rpc, m, slabs, se, corr_bra(c), bs->s);
+    }
     const int pblocks = std::max(1, std::min(bs->sms * 4, (n + 7) / 8));
     mark(DQ_KIND_POP);
     if (c->ipr_on && !skip_pop)
@@ -4450,10 +4505,13 @@ static dq_status enqueue_iteration_any(dq_ctx* c, int j) {
     return DQ_OK;
 }
 
-dq_status batched_iteration(dq_ctx* c, BatchedState* ws, int j) {
+dq_status batched_krylov(dq_ctx* c, BatchedState* ws) {
     BatchedState* saved = c->bat;
     c->bat = ws;
-    dq_status st = enqueue_iteration_any(c, j);
+    dq_status st = DQ_OK;
+    if (ws->staged == kStagedCluster) st = check_cuda(c, cluster_launch(c, false, ZZBlockRef{}), "cluster launch");
+    else
+        for (int j = 1; j <= c->cfg.m && st == DQ_OK; ++j) st = enqueue_iteration_any(c, j);
     c->bat = saved;
     return st;
 }
@@ -4532,12 +4590,14 @@ dq_status batched_time_iteration(dq_ctx* c, int reps, double* ms) {
     // the standard forms are timed on iteration 2 (after one of iteration 1),
     // whose SpMM also streams q_{j-1} like every later one
     const int js = std::min(2, c->cfg.m);
+    const bool cluster = c->bat->staged == kStagedCluster;
     auto one = [&]() {
-        if (fused) fused_iteration_any(c, jt);
+        if (cluster) batched_krylov(c, c->bat);
+        else if (fused) fused_iteration_any(c, jt);
         else if (pform) pf(jt);
         else enqueue_iteration_any(c, js);
     };
-    if (!fused && !pform && js == 2) enqueue_iteration_any(c, 1);
+    if (!fused && !pform && !cluster && js == 2) enqueue_iteration_any(c, 1);
     if (fused) {
         enqueue_iteration_any(c, 1);
         if (jt == 3) fused_iteration_any(c, 2);
@@ -4555,7 +4615,8 @@ dq_status batched_time_iteration(dq_ctx* c, int reps, double* ms) {
     cudaEventElapsedTime(&t, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    *ms = t / reps;
+    // the cluster form runs all m iterations in one launch
+    *ms = t / reps / (cluster ? c->cfg.m : 1);
     return check_cuda(c, cudaGetLastError(), "time iteration");
 }
 
@@ -4597,7 +4658,7 @@ __global__ void __launch_bounds__(512, 1) k_gather_floor(int n, int B, int TC, i
 dq_status batched_time_gather_floor(dq_ctx* c, int reps, double* ms) {
     BatchedState* bs = c->bat;
     const BlockFmt& f = bs->fmt[r_index(bs->R)];
-    if (!bs->mixed || bs->TPT != 2 || bs->R > 3 || !f.packed) {
+    if (!bs->mixed || bs->TPT != 2 || bs->R > 3 || !f.packed || bs->staged == kStagedCluster) {
         c->err = "gather floor: needs the complex64 packed form (vec 2, rows_per_block <= 3)";
         return DQ_ERR_STATE;
     }

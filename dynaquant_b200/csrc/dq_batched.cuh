@@ -19,6 +19,7 @@ constexpr int kMaxCtasPerChunk = 4096;
 // SM); measured on the tube, 2, 3, 8 and 16 were all slower (small systems
 // take twice as many, see batched_set_tiling)
 constexpr int kStreamCtasPerSm = 4;
+constexpr int kStagedCluster = 13;   // tiling form of dq_cluster.cu
 constexpr int kMCheckStride = 4;   // adaptive Krylov dimension: checks at m_min, m_min + 4, ... below m
 
 // ---- vector access of TPT consecutive complex values ----------------------
@@ -193,6 +194,10 @@ struct dq::BatchedState {
     // fused iteration (staged = 2): second SpMM output buffer, tensor maps of
     // slabs 0..m and of wB (boxes of f_sr rows), halo blocks, stages, grid
     void* wB = nullptr;
+    // cluster form: the dense exponential's matrices, one set per chunk
+    void* cl_scratch = nullptr;
+    size_t cl_scratch_bytes = 0;
+    size_t cl_rec = 0;          // its records' share of the shared memory
     std::vector<CUtensorMap> fmaps;
     int f_sr = 0, f_hb = 0, f_D = 2, f_rpc = 0, f_gx = 0, f_rb = 1;   // f_rb: blocks per warp (staged = 4)
     size_t f_smem = 0;
@@ -292,7 +297,18 @@ namespace dq {
 // host functions of dq_batched.cu used by the adjoint
 BatchedState* batched_alloc_ws(dq_ctx* c, int B, bool mixed, dq_status* st);
 void batched_free_ws(BatchedState* bs);
-dq_status batched_iteration(dq_ctx* c, BatchedState* ws, int j);
+// the m Lanczos iterations of a workspace (without ||H q_{m+1}||)
+dq_status batched_krylov(dq_ctx* c, BatchedState* ws);
 dq_status batched_mirror_tiling(dq_ctx* c, BatchedState* dst);
 dq_status batched_step_eager(dq_ctx* c, const std::function<void()>* after_noise, bool skip_pop);
+// trajectories per chunk of the layout of slabs 2.. ([chunk][site][trajectory]; B: plain [site][trajectory])
+inline int batched_basis_chunk(const BatchedState* bs) { return bs->staged == kStagedCluster ? bs->TC : bs->B; }
+// dq_cluster.cu: one launch per step
+struct ZZBlockRef {   // ZZ noise sums of a block of steps and its first step (null for other noise)
+    const double* D = nullptr;
+    const int* start = nullptr;
+};
+double cluster_plan(dq_ctx* c, int R, int* tc_out, int* cs_out);
+dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R);
+cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz);
 }  // namespace dq

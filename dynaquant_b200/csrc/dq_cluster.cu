@@ -41,6 +41,7 @@ enum { kClNoise = 1, kClFinish = 2 };
 struct ClusterArgs {
     int n, B, TC, rpc, bw, m, flags, bil, chunks;
     int rec_smem;             // bytes of coupling records kept in shared memory (0: read through L1)
+    int max_block;            // most records of one row block
     const int* bptr;
     const int* bcol;
     const void* bcoef;
@@ -78,7 +79,7 @@ static __host__ __device__ inline ClLayout cl_layout(int CS, int TC, int m, int 
     L.red = p; p += sizeof(double2) * 2 * kClWarps * TC;
     L.al = p; p += sizeof(double2) * (m + 2) * TC;
     L.y = p; p += sizeof(double2) * m * TC;
-    L.par = p; p += sizeof(double2) * 2 * TC;
+    L.par = p; p += sizeof(double2) * 3 * TC;
     L.be = p; p += sizeof(double) * (m + 2) * TC;
     L.sc = p; p += sizeof(double) * (m + 2) * TC;
     p = (p + 127) & ~(size_t)127;
@@ -142,6 +143,7 @@ struct ClSum {
     double2* red;   // [2][warps][TC]
     int TC, CS;
     unsigned rank;
+    int pt, pd;     // threadIdx.x % TC, threadIdx.x / TC
 
     __device__ __forceinline__ void sync() const {
         if constexpr (kLocal) __syncthreads();
@@ -170,8 +172,8 @@ struct ClSum {
             for (int t = 0; t < TPT; ++t) red[(buf * kClWarps + warp) * TC + lane * TPT + t] = make_double2(a[t], b[t]);
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < TC * CS; e += kClThreads) {
-            const int t = e % TC, dst = e / TC;
+        for (int dst = pd; dst < CS; dst += kClThreads / TC) {
+            const int t = pt;
             double2 v[kClWarps];
 #pragma unroll
             for (int w = 0; w < kClWarps; ++w) v[w] = red[(buf * kClWarps + w) * TC + t];
@@ -202,53 +204,124 @@ struct ClSum {
     }
 };
 
-// Four coupling entries of one row block: window row and R coefficients each.
+__device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float4 lds_f4(unsigned a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ double2 lds_d2(unsigned a) {
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+    return v;
+}
+
+// The power of two at or below |s| (0 for 0), as a float, and 1 over it.
+__device__ __forceinline__ float cl_pow2(double s) {
+    if (s == 0.0) return 0.f;
+    return ldexpf(1.f, max(-120, min(120, ilogb(s))));
+}
+__device__ __forceinline__ double cl_pow2_inv(double s) { return ldexp(1.0, -max(-120, min(120, ilogb(s)))); }
+
+// Where a thread's coupling records are.  In global memory (lg < 0) the
+// records of a block are contiguous from bptr[k]; in shared memory those of
+// the 2^lg = 32 / TL blocks a warp works on are interleaved entry by entry, so
+// the warp's loads of one entry are one contiguous run instead of one
+// bank-conflicting piece per block.
+struct ClRecs {
+    const int* bptr;     // starts of the own blocks
+    const int* col;      // FP64 form: columns
+    const void* rec;     // packed records, or FP64 coefficients
+    unsigned scol, srec; // the same in shared memory
+    int lg, maxb;
+};
+
+// Four coupling entries of one row block: column and R coefficients each.
 template <typename Real, int R>
 struct ClRec {
     int c[4];
     Real cf[4][R];
-    // entries [e, e + 4) of a block that ends at pe; col/rec in shared memory or global
-    __device__ __forceinline__ void load(int e, int pe, const int* col, const void* rec) {
+    __device__ __forceinline__ void put(int u, float4 r) {
+        c[u] = __float_as_int(r.x);
+        cf[u][0] = r.y;
+        if constexpr (R > 1) cf[u][R > 1 ? 1 : 0] = r.z;
+        if constexpr (R > 2) cf[u][R > 2 ? 2 : 0] = r.w;
+    }
+    // entries [e, e + 4) of a block of `len` entries; `off` is the block's
+    // first slot (kShared: byte offset of its 16-byte records)
+    template <bool kShared>
+    __device__ __forceinline__ void load(const ClRecs& Q, int off, int e, int len) {
         if constexpr (sizeof(Real) == 4) {
             // packed records {col, c0, c1, c2}, a multiple of 4 per block
-            const float4* r4 = reinterpret_cast<const float4*>(rec) + e;
+            if constexpr (kShared) {
+                const unsigned a = Q.srec + off + (e << (Q.lg + 4));
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 r = r4[u];
-                c[u] = __float_as_int(r.x);
-                cf[u][0] = r.y;
-                if constexpr (R > 1) cf[u][R > 1 ? 1 : 0] = r.z;
-                if constexpr (R > 2) cf[u][R > 2 ? 2 : 0] = r.w;
+                for (int u = 0; u < 4; ++u) put(u, lds_f4(a + (u << (Q.lg + 4))));
+            } else {
+                const float4* r4 = reinterpret_cast<const float4*>(Q.rec) + off + e;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) put(u, __ldg(r4 + u));
             }
         } else {
-            const Real* cb = reinterpret_cast<const Real*>(rec);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int p = min(e + u, pe - 1);
-                c[u] = col[p];
+                const int p = min(e + u, len - 1);
+                if constexpr (kShared) {
+                    // columns [slot], coefficients by pairs in planes of 2^lg (R = 1: singles)
+                    const int g = off >> Q.lg, i = off & ((1 << Q.lg) - 1), slot = ((g + p) << Q.lg) + i;
+                    asm volatile("ld.shared.s32 %0, [%1];" : "=r"(c[u]) : "r"(Q.scol + 4 * slot));
+                    if constexpr (R == 1) {
+                        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(cf[u][0]) : "r"(Q.srec + 8 * slot));
+                    } else {
 #pragma unroll
-                for (int i = 0; i < R; ++i) cf[u][i] = e + u < pe ? cb[(size_t)p * R + i] : Real(0);
+                        for (int h = 0; h < R / 2; ++h) {
+                            const double2 v = lds_d2(Q.srec + 16 * ((((g + p) * (R / 2) + h) << Q.lg) + i));
+                            cf[u][2 * h] = v.x;
+                            cf[u][2 * h + 1] = v.y;
+                        }
+                    }
+                } else {
+                    c[u] = __ldg(Q.col + off + p);
+                    const Real* cb = reinterpret_cast<const Real*>(Q.rec) + (size_t)(off + p) * R;
+#pragma unroll
+                    for (int i = 0; i < R; ++i) cf[u][i] = __ldg(cb + i);
+                }
+                if (e + u >= len)
+#pragma unroll
+                    for (int i = 0; i < R; ++i) cf[u][i] = Real(0);
             }
         }
     }
 };
 
-// acc += the couplings of one row block, entries [pb, pe), times the window's
-// rows (`win` points at this thread's trajectories of global row 0); the next
-// four entries load while the current four gather.
-template <typename Real, int TPT, int R>
-__device__ __forceinline__ void cl_gather(int pb, int pe, const int* col, const void* rec, const Real* win, int row,
+// acc += the couplings of one row block times the window's rows (`win`: shared
+// address of this thread's trajectories of global row 0, `row` bytes a row);
+// the next four entries load while the current four gather.
+template <typename Real, int TPT, int R, bool kShared>
+__device__ __forceinline__ void cl_gather(const ClRecs& Q, int off, int len, unsigned win, int row,
                                           CV<Real, TPT> (&acc)[R]) {
-    if (pb >= pe) return;
     ClRec<Real, R> A;
-    A.load(pb, pe, col, rec);
-    for (int e = pb;; e += 4) {
-        const bool more = e + 4 < pe;
+    A.template load<kShared>(Q, off, 0, len);
+    for (int e = 0;; e += 4) {
+        const bool more = e + 4 < len;
         ClRec<Real, R> N;
-        if (more) N.load(e + 4, pe, col, rec);
+        if (more) N.template load<kShared>(Q, off, e + 4, len);
         CV<Real, TPT> y[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) y[u] = ldv<Real, TPT, false>(win + (ptrdiff_t)A.c[u] * row, 0);
+        for (int u = 0; u < 4; ++u) {
+            const unsigned a = win + A.c[u] * row;
+            if constexpr (TPT == 2) {
+                const float4 v = lds_f4(a);
+                y[u].v[0] = v.x;
+                y[u].v[1] = v.y;
+                y[u].v[2 * TPT - 2] = v.z;
+                y[u].v[2 * TPT - 1] = v.w;
+            } else {
+                const double2 v = lds_d2(a);
+                y[u].v[0] = (Real)v.x;
+                y[u].v[1] = (Real)v.y;
+            }
+        }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -271,7 +344,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const ClLayout Y = cl_layout(CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem);
     double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
     double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
-    double2* par = reinterpret_cast<double2*>(smem + Y.par);   // [0][t] alpha_j sc_j, [1][t] (sc_j, the factor of r_{j-1})
+    // [0][t] the update's coefficients, [1][t] (sc_j, the factor of r_{j-1}), [2][t] complex64: Im alpha's low part
+    double2* par = reinterpret_cast<double2*>(smem + Y.par);
     double* be = reinterpret_cast<double*>(smem + Y.be);
     double* scs = reinterpret_cast<double*>(smem + Y.sc);
     const int rowr = TC * 2;                                   // Reals of one row
@@ -280,7 +354,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     Real* prev = reinterpret_cast<Real*>(smem + Y.prev);
     Real* dsm = reinterpret_cast<Real*>(smem + Y.d);
     const ClSum<TPT, kLocal> sum{reinterpret_cast<double2*>(smem + Y.ex), reinterpret_cast<double2*>(smem + Y.red),
-                                 TC, CS, rank};
+                                 TC, CS, rank, (int)threadIdx.x % TC, (int)threadIdx.x / TC};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tl = threadIdx.x % TL, rl = threadIdx.x / TL, RL = kClThreads / TL;
     const int chunk = blockIdx.x / CS, c0 = chunk * TC;
@@ -296,34 +370,50 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     auto loc = [&](int row) { return (size_t)row * TC + tl * TPT; };
     auto glo = [&](int row) { return (size_t)(r0 + row) * B + bb; };
 
+    // slab j >= 2: [chunk][site][trajectory of the chunk], so a CTA's rows are one contiguous run
+    const int tca = min(TC, B - c0);
+    auto basis = [&](int j, int row) {
+        return slab(j) + 2 * ((size_t)c0 * n + (size_t)(r0 + row) * tca + (act ? tl * TPT : 0));
+    };
+
     // ---- the coupling records of the own row blocks --------------------------
     const int kb0 = r0 / R, nbo = (nrow + R - 1) / R;
-    const int* bptr = A.bptr + kb0;
-    const int* col = A.bcol;
-    const void* rec = A.bcoef;
-    int ebase = 0;
+    ClRecs Q{A.bptr + kb0, A.bcol, A.bcoef, 0u, 0u, -1, A.max_block};
     if (A.rec_smem) {
         // block starts, columns (FP64), coefficients
-        ebase = __ldg(bptr);
-        const int ne = __ldg(bptr + nbo) - ebase;
+        const int lg = __ffs(32 / TL) - 1, per = 1 << lg;
+        const int slots = (nbo + per - 1) / per * per * A.max_block;
         int* sb = reinterpret_cast<int*>(smem + Y.rec);
-        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(bptr + k);
+        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(A.bptr + kb0 + k);
         unsigned char* q = smem + Y.rec + (((size_t)nbo + 1) * 4 + 15) / 16 * 16;
-        if constexpr (sizeof(Real) == 4) {
-            float4* sr = reinterpret_cast<float4*>(q);
-            const float4* gr = reinterpret_cast<const float4*>(A.bcoef) + ebase;
-            for (int e = threadIdx.x; e < ne; e += kClThreads) sr[e] = __ldg(gr + e);
-            rec = sr;
-        } else {
-            int* scol = reinterpret_cast<int*>(q);
-            Real* sr = reinterpret_cast<Real*>(q + ((size_t)ne * 4 + 15) / 16 * 16);
-            const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)ebase * R;
-            for (int e = threadIdx.x; e < ne; e += kClThreads) scol[e] = __ldg(A.bcol + ebase + e);
-            for (int e = threadIdx.x; e < ne * R; e += kClThreads) sr[e] = __ldg(gr + e);
-            col = scol;
-            rec = sr;
+        int* scol = reinterpret_cast<int*>(q);
+        if constexpr (sizeof(Real) == 8) q += ((size_t)slots * 4 + 15) / 16 * 16;
+        // a warp per block, a lane per entry
+        for (int k = warp; k < nbo; k += kClWarps) {
+            const int p0 = __ldg(A.bptr + kb0 + k), ne = __ldg(A.bptr + kb0 + k + 1) - p0;
+            const int g = (k >> lg) * A.max_block, i = k & (per - 1);
+            for (int e = lane; e < ne; e += 32) {
+                if constexpr (sizeof(Real) == 4) {
+                    reinterpret_cast<float4*>(q)[(g + e) * per + i] =
+                        __ldg(reinterpret_cast<const float4*>(A.bcoef) + p0 + e);
+                } else {
+                    const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)(p0 + e) * R;
+                    scol[(g + e) * per + i] = __ldg(A.bcol + p0 + e);
+                    if constexpr (R == 1) {
+                        reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < R / 2; ++h)
+                            reinterpret_cast<double2*>(q)[((g + e) * (R / 2) + h) * per + i] =
+                                __ldg(reinterpret_cast<const double2*>(gr) + h);
+                    }
+                }
+            }
         }
-        bptr = sb;
+        Q.bptr = sb;
+        Q.scol = sm_addr(scol);
+        Q.srec = sm_addr(q);
+        Q.lg = lg;
     }
 
     // ---- r_1 = psi over the window, the diagonal (noise of this step, or as it is)
@@ -386,14 +476,22 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     sum.sync();   // every CTA of the cluster runs; the window is in place
 
-    const Real* wcol = cur - (ptrdiff_t)r0 * rowr + 2 * tl * TPT;   // this thread's values of global row 0
+    const int rowb = rowr * (int)sizeof(Real);
+    const unsigned wcol = sm_addr(cur) - (unsigned)(r0 * rowb) + tl * TPT * 2 * (int)sizeof(Real);   // global row 0
     // H_off r_j of block k
     auto product = [&](int k, CV<Real, TPT> (&acc)[R]) {
 #pragma unroll
         for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int v = 0; v < 2 * TPT; ++v) acc[i].v[v] = 0;
-        cl_gather<Real, TPT, R>(bptr[k] - ebase, bptr[k + 1] - ebase, col, rec, wcol, rowr, acc);
+        const int p0 = Q.bptr[k], len = Q.bptr[k + 1] - p0;
+        if (len <= 0) return;
+        if (Q.lg < 0) {
+            cl_gather<Real, TPT, R, false>(Q, p0, len, wcol, rowb, acc);
+        } else {
+            const int slot = ((k >> Q.lg) * Q.maxb << Q.lg) + (k & ((1 << Q.lg) - 1));
+            cl_gather<Real, TPT, R, true>(Q, sizeof(Real) == 4 ? slot << 4 : slot, len, wcol, rowb, acc);
+        }
     };
     // the neighbours' rows of the window's margins, as they are in their shared memory
     auto margins = [&]() {
@@ -405,7 +503,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 for (int q = 0; q < 4; ++q) {
                     const int h = h0 + q * RL;
                     if (h >= nh) break;
-                    const int g = r0 + (h < hlo ? h - hlo : nrow + h - hlo), own = g / A.rpc;
+                    const int g = r0 + (h < hlo ? h - hlo : nrow + h - hlo);
+                    int own = (int)rank;
+                    while (g < own * A.rpc) --own;
+                    while (g >= (own + 1) * A.rpc) ++own;
                     v[q] = cl_load(reinterpret_cast<const T*>(cur + (size_t)(g - own * A.rpc) * rowr) + tl, own);
                 }
 #pragma unroll
@@ -420,6 +521,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     };
 
     const bool adaptive = A.S.mtraj != nullptr;
+    // the last warp's lanes take the sums' scalars: the margins' loads start with the first warps
+    const int last = warp == kClWarps - 1 ? lane : kMaxTC;
     int jl = A.m;   // iterations done
     for (int j = 1; j <= A.m; ++j) {
         // u = H r_j - (beta_{j-1} sc_{j-1} / sc_j) r_{j-1} over r_{j-1} (w = sc_j u); alpha_j
@@ -450,36 +553,47 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     const Real ui = fma(dv, x.v[2 * t + 1], fma(-fm[t], o.v[2 * t + 1], acc[i].v[2 * t + 1]));
                     o.v[2 * t] = ur;
                     o.v[2 * t + 1] = ui;
-                    const double xr = x.v[2 * t], xi = x.v[2 * t + 1], dr = ur, di = ui;
-                    if (A.bil) {
-                        x2[t] += xr * dr - xi * di;
-                        y2[t] += xr * di + xi * dr;
-                    } else {
-                        x2[t] += xr * dr + xi * di;
-                        y2[t] += xr * di - xi * dr;
-                    }
+                    // the bilinear dot takes q_j itself, the Hermitian one its conjugate
+                    const double xr = x.v[2 * t], xi = A.bil ? -x.v[2 * t + 1] : x.v[2 * t + 1], dr = ur, di = ui;
+                    x2[t] += xr * dr + xi * di;
+                    y2[t] += xr * di - xi * dr;
                 }
                 stv<Real, TPT>(prev, l, o);
             }
         }
         sum.template part<true>(0, x2, y2);
         sum.sync();
-        if (threadIdx.x < TC) {
-            const int t = threadIdx.x;
+        for (int t = last; t < TC; t += 32) {
             const double2 a = sum.get(0, t);
             const double s = scs[j * TC + t], ar = a.x * s * s, ai = a.y * s * s;
             al[j * TC + t] = make_double2(ar, ai);
-            par[t] = make_double2(ar * s, ai * s);
+            if constexpr (sizeof(Real) == 4) {
+                const float p2 = cl_pow2(s), h = (float)ar, g = (float)ai;
+                *reinterpret_cast<float4*>(par + t) = make_float4(p2, -p2 * h, -p2 * (float)(ar - h), p2 * g);
+                par[2 * TC + t].x = p2 * (float)(ai - g);
+            } else {
+                par[t] = make_double2(ar * s, ai * s);
+            }
         }
         __syncthreads();
-        // r_{j+1} = w - alpha_j q_j over r_j, r_j over r_{j-1}; beta_j
+        // r_{j+1} over r_j, r_j over r_{j-1}; beta_j.  complex128: r_{j+1} = sc_j (u - alpha_j r_j).
+        // complex64: the scale is the power of two below sc_j and alpha a pair of floats, so that
+        // fma(-alpha_lo, r, fma(-alpha_hi, r, u)) is within an ulp of the exact difference without
+        // a conversion to FP64 (16 a clock and SM: eight of them a value bound this pass)
         double2 aj[TPT];
+        float4 af[TPT];
+        float aq[TPT];
 #pragma unroll
         for (int t = 0; t < TPT; ++t) {
-            aj[t] = par[tl * TPT + t];
+            if constexpr (sizeof(Real) == 4) {
+                af[t] = *reinterpret_cast<const float4*>(par + tl * TPT + t);
+                aq[t] = (float)par[2 * TC + tl * TPT + t].x;
+            } else {
+                aj[t] = par[tl * TPT + t];
+            }
             x2[t] = 0.0;
         }
-        Real* out = slab(j + 1);
+        Real* out = basis(j + 1, 0);
         for (int k = rl; k < nbk; k += RL)
 #pragma unroll
             for (int i = 0; i < R; ++i) {
@@ -490,27 +604,41 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 CV<Real, TPT> o = ldv<Real, TPT, false>(prev, l);
 #pragma unroll
                 for (int t = 0; t < TPT; ++t) {
-                    const double xr = x.v[2 * t], xi = x.v[2 * t + 1];
-                    o.v[2 * t] = (Real)(sc[t] * (double)o.v[2 * t] - (aj[t].x * xr - aj[t].y * xi));
-                    o.v[2 * t + 1] = (Real)(sc[t] * (double)o.v[2 * t + 1] - (aj[t].x * xi + aj[t].y * xr));
+                    if constexpr (sizeof(Real) == 4) {
+                        const float xr = x.v[2 * t], xi = x.v[2 * t + 1];
+                        float2 v = make_float2(af[t].x * o.v[2 * t], af[t].x * o.v[2 * t + 1]);   // exact
+                        v = __ffma2_rn(make_float2(af[t].y, af[t].y), make_float2(xr, xi), v);
+                        v = __ffma2_rn(make_float2(af[t].z, af[t].z), make_float2(xr, xi), v);
+                        v = __ffma2_rn(make_float2(af[t].w, -af[t].w), make_float2(xi, xr), v);
+                        if (A.bil) v = __ffma2_rn(make_float2(aq[t], -aq[t]), make_float2(xi, xr), v);
+                        o.v[2 * t] = v.x;
+                        o.v[2 * t + 1] = v.y;
+                    } else {
+                        const double xr = x.v[2 * t], xi = x.v[2 * t + 1];
+                        o.v[2 * t] = (Real)(sc[t] * (double)o.v[2 * t] - (aj[t].x * xr - aj[t].y * xi));
+                        o.v[2 * t + 1] = (Real)(sc[t] * (double)o.v[2 * t + 1] - (aj[t].x * xi + aj[t].y * xr));
+                    }
                     const double rr = o.v[2 * t], ri = o.v[2 * t + 1];
                     x2[t] += rr * rr + ri * ri;
                 }
                 stv<Real, TPT>(prev, l, x);
                 stv<Real, TPT>(cur, l, o);
-                stv<Real, TPT>(out, glo(row), o);
+                stv<Real, TPT>(out + (size_t)row * tca * 2, 0, o);
             }
         sum.template part<false>(1, x2, y2);
         sum.sync();
-        if (threadIdx.x < TC) {
-            const int t = threadIdx.x;
+        for (int t = last; t < TC; t += 32) {
             const double b2 = sum.get(1, t).x;
-            // 1 / beta and beta; sqrt only where the reciprocal has no value
-            double s1 = rsqrt(b2), bt = b2 * s1;
+            // 1 / ||r_{j+1}|| and ||r_{j+1}||; sqrt only where the reciprocal has no value
+            double s1 = rsqrt(b2), nr = b2 * s1;
             if (!(b2 > 1e-290) || !(b2 < 1e290)) {
-                bt = sqrt(b2);
-                s1 = bt > 0.0 ? 1.0 / bt : 0.0;
+                nr = sqrt(b2);
+                s1 = nr > 0.0 ? 1.0 / nr : 0.0;
             }
+            // beta_j = ||H q_j - ..|| = sc_j ||r_{j+1}|| / scale (complex128: scale = sc_j)
+            const double scj = scs[j * TC + t];
+            double bt = nr;
+            if constexpr (sizeof(Real) == 4) bt = scj != 0.0 ? nr * (scj * cl_pow2_inv(scj)) : 0.0;
             if (!isfinite(bt) && c0 + t < B && rank == 0) atomicCAS(A.S.status, 0, DQ_ERR_NAN);
             // lucky breakdown: invariant Krylov space, continue with q_{j+1} = 0
             const double bp = j > 1 ? be[(j - 1) * TC + t] : 0.0;
@@ -522,8 +650,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             }
             be[j * TC + t] = bt;
             scs[(j + 1) * TC + t] = s1;
-            // beta_j sc_j / sc_{j+1} = beta_j^2 sc_j
-            par[TC + t] = make_double2(s1, bt * (bt * scs[j * TC + t]));
+            // beta_j sc_j / sc_{j+1}
+            par[TC + t] = make_double2(s1, bt * scj * (s1 > 0.0 ? nr : 0.0));
         }
         margins();
         __syncthreads();
@@ -707,7 +835,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 CV<Real, TPT> v[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (j0 + q <= mmax) v[q] = ldv<Real, TPT, false>(slab(j0 + q), x);
+                    if (j0 + q <= mmax)
+                        v[q] = j0 + q == 1 ? ldv<Real, TPT, false>(slab(1), x)
+                                           : ldv<Real, TPT, false>(basis(j0 + q, row), 0);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     if (j0 + q > mmax) break;
@@ -819,11 +949,11 @@ static cudaLaunchConfig_t cl_config(int chunks, int CS, size_t smem, cudaStream_
 }
 
 // Bytes of the largest CTA's coupling records (block starts, columns, coefficients).
-static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R) {
-    const size_t nb = rpc / R, ne = nb * (size_t)f.max_block;
+static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R, int TL) {
+    const size_t per = 32 / TL, nb = rpc / R, slots = (nb + per - 1) / per * per * (size_t)f.max_block;
     const size_t head = ((nb + 1) * 4 + 15) / 16 * 16;
-    if (mixed) return head + ne * 16;
-    return head + (ne * 4 + 15) / 16 * 16 + ne * R * sizeof(double);
+    if (mixed) return head + slots * 16;
+    return head + (slots * 4 + 15) / 16 * 16 + slots * R * sizeof(double);
 }
 
 // Clusters of this shape that the device holds at once (0: it cannot run);
@@ -832,13 +962,13 @@ static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R) {
 static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::BlockFmt& f, size_t* smem, size_t* rec) {
     const BatchedState* bs = c->bat;
     const int n = c->n, m = c->cfg.m;
-    if (CS < 1 || CS > kClMaxCtas || (CS & (CS - 1))) return 0;
+    if (CS < 1 || CS > kClMaxCtas) return 0;
     if (tc < tpt || tc > kMaxTC || tc % tpt || ((tc / tpt) & (tc / tpt - 1)) || tc / tpt > 32) return 0;
     ClKernel k = cl_kernel(bs->mixed, tpt, R, CS == 1);
     if (!k) return 0;
     const size_t rsz = bs->mixed ? sizeof(float) : sizeof(double);
     const int rpc = cl_rows(n, CS, R);
-    size_t rb = cl_rec_bytes(f, bs->mixed, rpc, R);
+    size_t rb = cl_rec_bytes(f, bs->mixed, rpc, R, tc / tpt);
     size_t sm = cl_layout(CS, tc, m, rpc, c->bw, rsz, rb).total;
     if (sm > kClSmemMax) {
         rb = 0;
@@ -858,6 +988,51 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
     return found;
 }
 
+// Estimated SM cycles of one Lanczos iteration of this shape, and the shape
+// with the least over CTAs per cluster and trajectories per chunk (R rows per
+// block, its blocks built).  An iteration is a fixed part (two reductions with
+// their barriers, the margins' round trip), the shared-memory wavefronts of
+// the gathers and records (records read through L1: a wavefront each) and the
+// elementwise part, bound by FP64 arithmetic and, in complex64, by
+// conversions; times the waves of clusters that the device needs.  Measured
+// against it on a B200 (us per iteration): 4096 sites x 128, 8 couplings per
+// row, 4 CTAs x 4 trajectories 8.0 (model 8.1); 4731 x 100, 28 couplings, 9 x 8
+// 13.8 (13.0); 8100 x 64, 6 x 4 in an adaptive run.  The order of shapes is what it
+// is used for; those within 10 % change places with the matrix.
+double cluster_plan(dq_ctx* c, int R, int* tc_out, int* cs_out) {
+    const BatchedState* bs = c->bat;
+    const ::BlockFmt& f = cl_fmt(bs, R);
+    const int n = c->n, B = bs->B, tpt = bs->mixed ? 2 : 1;
+    const double len = (double)f.nunion / std::max(1, f.nb), csz = bs->mixed ? 8.0 : 16.0;
+    double best = 1e30;
+    for (int CS = 1; CS <= kClMaxCtas; ++CS) {
+        const int rpc = cl_rows(n, CS, R);
+        if (CS > 1 && (size_t)rpc * (CS - 1) >= (size_t)n) continue;   // a CTA without rows
+        for (int tc = tpt; tc <= 32 && tc < 2 * B; tc *= 2) {
+            const int chunks = (B + tc - 1) / tc, TL = tc / tpt;
+            // threads with a block to do set the pace when there are fewer than the CTA has
+            const double nbk = rpc / R, rounds = std::ceil(nbk * TL / kClThreads) * kClThreads / (nbk * TL);
+            const double gather = nbk * len * tc * csz / 128.0 * 1.3;
+            const double elem = (double)rpc * tc * (bs->mixed ? 1.2 : 0.8) * std::min(rounds, 1.5);
+            auto cycles = [&](bool in_smem) {
+                return 5500.0 + 60.0 * CS + 1.6 * (gather + nbk * len * (in_smem ? 0.125 * (bs->mixed ? 1 : R) : 0.8)) +
+                       elem;
+            };
+            if (cycles(true) >= best) continue;
+            size_t smem = 0, rec = 0;
+            const int fit = cluster_resident(c, tc, tpt, CS, R, f, &smem, &rec);
+            if (fit < 1) continue;
+            const double t = (double)((chunks + fit - 1) / fit) * cycles(rec > 0);
+            if (t < best) {
+                best = t;
+                *tc_out = tc;
+                *cs_out = CS;
+            }
+        }
+    }
+    return best;
+}
+
 // One cluster launch: the whole step (flags kClNoise | kClFinish), or the
 // Lanczos iterations of a given slab 1 and diagonal alone (flags 0).
 cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
@@ -870,6 +1045,7 @@ cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
     a.rpc = bs->rpc;
     a.bw = c->bw;
     a.rec_smem = (int)bs->cl_rec;
+    a.max_block = f.max_block;
     a.m = c->cfg.m;
     a.flags = whole_step ? kClNoise | kClFinish : 0;
     a.bil = c->cfg.dot_mode == DQ_DOT_BILINEAR;

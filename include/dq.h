@@ -231,7 +231,8 @@ DQ_API dq_status dq_krylov_step_static(int n, const int *rowptr, const int *col,
  * fused combine/observables), the step loop captured in a CUDA graph. */
 DQ_API dq_status dq_run(dq_ctx *ctx, int n_steps);
 
-/* Tiling of the ensemble kernels: traj_chunk trajectories per CTA column
+/* Tiling of the ensemble kernels (without this call or dq_autotune a default
+ * by size is taken): traj_chunk trajectories per CTA column
  * (a power of two dividing n_traj, <= 64), vec 1 or 2 complex values per
  * thread (8- or 16-byte loads; 1 in FP64), about ctas_per_sm CTAs per SM,
  * each owning a contiguous range of sites, and rows_per_block (1, 2, 4 or 8)
@@ -262,7 +263,12 @@ DQ_API dq_status dq_run(dq_ctx *ctx, int n_steps);
  * still in L2 (no reorthogonalisation or adaptive m), 12 is the L1 form at
  * 32 warps per SM and at most 64 registers a thread (complex64, vec 2,
  * rows_per_block <= 3; ctas_per_sm 1: one 1024-thread CTA per SM, 2: two
- * 512-thread CTAs).  groups splits the trajectory chunks
+ * 512-thread CTAs), 13 runs a whole step in one launch: a thread-block
+ * cluster of ctas_per_sm CTAs (1 to 16) per traj_chunk trajectories (vec times
+ * a power of two; it need not divide n_traj), each CTA's rows with their
+ * neighbours, within the matrix bandwidth, in shared memory (vec 2 in
+ * complex64; rows_per_block up to 3, 4 in FP64 but not 3; groups 1, no
+ * reorthogonalisation; refused when it does not fit).  groups splits the trajectory chunks
  * into groups whose m Lanczos iterations run one group after another, so a
  * group's Krylov slabs stay resident in L2 (must divide n_traj / traj_chunk).  Changing it restarts the ensemble at the next dq_run
  * (as dq_reset does). */
