@@ -186,6 +186,7 @@ dq_status dq_set_hamiltonian_csr(dq_ctx* c, int n, const int* rowptr, const int*
     }
     c->rows_sorted = sorted;
     c->bw = bw;
+    c->plain = plain_cluster_plan(n, c->cfg.m, bw, (double)cl.size() / n);
     c->nnz_off = (int)cl.size();
     c->rowptr = std::move(rp);
     c->col = std::move(cl);

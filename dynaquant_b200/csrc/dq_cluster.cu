@@ -36,12 +36,14 @@ constexpr int kClMaxCtas = 16;            // CTAs per cluster (above 8: not port
 // dynamic shared memory of one CTA (one CTA per SM: 128 registers a thread)
 constexpr size_t kClSmemMax = 224 * 1024;
 
+// margins above this are read through L2 instead of the neighbours' shared memory
+constexpr size_t kClWideMargin = 32 * 1024;
+
 enum { kClNoise = 1, kClFinish = 2 };
 
 struct ClusterArgs {
     int n, B, TC, rpc, bw, m, flags, bil, chunks;
     int rec_smem;             // bytes of coupling records kept in shared memory (0: read through L1)
-    int max_block;            // most records of one row block
     const int* bptr;
     const int* bcol;
     const void* bcoef;
@@ -49,7 +51,7 @@ struct ClusterArgs {
     size_t slab;              // complex values per slab
     void* diag;
     BatchedScalars S;
-    int noise, ns, traj0;
+    int noise, ns, traj0, step;   // step: kPlain
     double subdt, sqrt_subdt;
     uint64_t seed;
     const double* sigma;
@@ -63,6 +65,13 @@ struct ClusterArgs {
     double tau_im, tol;
     double* erracc;
     const cd* bra;
+    // one trajectory through the drop-in step (kPlain): the state comes from psi_in as it is (q_1) and
+    // goes to psi_out normalised; the sums of the record may be null
+    const cd* psi_in;
+    cd* psi_out;
+    double* pops_row;
+    cd* corr_pt;
+    PlainScalars* ps;
     unsigned char* scratch;   // per chunk, for the dense exponential
     size_t scratch_stride;
 };
@@ -72,7 +81,8 @@ struct ClLayout {
     size_t ex, red, al, y, par, be, sc, win, prev, d, rec, total;
 };
 
-static __host__ __device__ inline ClLayout cl_layout(int CS, int TC, int m, int rpc, int bw, size_t rsz, size_t rec) {
+static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int m, int rpc, int bw, size_t rsz,
+                                                     size_t rec) {
     ClLayout L;
     size_t p = 0;
     L.ex = p; p += sizeof(double2) * 2 * CS * TC;
@@ -84,7 +94,8 @@ static __host__ __device__ inline ClLayout cl_layout(int CS, int TC, int m, int 
     L.sc = p; p += sizeof(double) * (m + 2) * TC;
     p = (p + 127) & ~(size_t)127;
     const size_t row = (size_t)TC * 2 * rsz;
-    L.win = p; p += (rpc + (CS > 1 ? 2 * (size_t)bw : 0)) * row;
+    const size_t wide = rpc + 2 * (size_t)bw;   // never more than the rows there are (bw may be n)
+    L.win = p; p += (CS > 1 ? (wide < (size_t)n ? wide : (size_t)(n > rpc ? n : rpc)) : rpc) * row;
     L.prev = p; p += rpc * row;
     L.d = p; p += rpc * row / 2;
     p = (p + 15) & ~(size_t)15;
@@ -233,7 +244,8 @@ struct ClRecs {
     const int* col;      // FP64 form: columns
     const void* rec;     // packed records, or FP64 coefficients
     unsigned scol, srec; // the same in shared memory
-    int lg, maxb;
+    const int* goff;     // first entry of each interleaved group of 2^lg blocks
+    int lg;
 };
 
 // Four coupling entries of one row block: column and R coefficients each.
@@ -331,7 +343,18 @@ __device__ __forceinline__ void cl_gather(const ClRecs& Q, int off, int len, uns
     }
 }
 
-template <typename Real, int TPT, int R, bool kLocal>
+// Trajectory b's error estimate of the step.
+template <bool kPlain>
+__device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double est) {
+    if (kPlain) {
+        A.ps->err = est;
+        if (A.erracc) *A.erracc += est;
+    } else {
+        A.erracc[b] += est;
+    }
+}
+
+template <typename Real, int TPT, int R, bool kLocal, bool kPlain = false>
 __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArgs A) {
     using T = typename VL<Real, TPT>::T;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -341,7 +364,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const int CS = kLocal ? 1 : (int)cl_size();
     const unsigned rank = kLocal ? 0u : cl_rank();
     const int bw = kLocal ? 0 : A.bw;
-    const ClLayout Y = cl_layout(CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem);
+    const ClLayout Y = cl_layout(n, CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem);
     double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
     double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
     // [0][t] the update's coefficients, [1][t] (sc_j, the factor of r_{j-1}), [2][t] complex64: Im alpha's low part
@@ -350,7 +373,6 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     double* scs = reinterpret_cast<double*>(smem + Y.sc);
     const int rowr = TC * 2;                                   // Reals of one row
     Real* win = reinterpret_cast<Real*>(smem + Y.win);
-    Real* cur = win + (size_t)bw * rowr;                       // the own rows of the window
     Real* prev = reinterpret_cast<Real*>(smem + Y.prev);
     Real* dsm = reinterpret_cast<Real*>(smem + Y.d);
     const ClSum<TPT, kLocal> sum{reinterpret_cast<double2*>(smem + Y.ex), reinterpret_cast<double2*>(smem + Y.red),
@@ -363,9 +385,12 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const int bb = act ? b0 : 0;
     const int r0 = min((int)rank * A.rpc, n), nrow = min(n - r0, A.rpc);
     const int nbk = act ? (nrow + R - 1) / R : 0;
-    const int hlo = kLocal ? 0 : min(bw, r0), hhi = kLocal ? 0 : min(bw, n - (r0 + nrow));
+    const int hlo = kLocal ? 0 : min(bw, r0);
+    Real* cur = win + (size_t)hlo * rowr;                      // the own rows of the window
+    const int hhi = kLocal ? 0 : min(bw, n - (r0 + nrow));
     Real* slabs = reinterpret_cast<Real*>(A.slabs);
     auto slab = [&](int j) { return slabs + 2 * A.slab * j; };
+    const Real* first = kPlain ? reinterpret_cast<const Real*>(A.psi_in) : slab(1);
     // own row `row` (within the CTA) of this thread's trajectories
     auto loc = [&](int row) { return (size_t)row * TC + tl * TPT; };
     auto glo = [&](int row) { return (size_t)(r0 + row) * B + bb; };
@@ -378,53 +403,69 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
 
     // ---- the coupling records of the own row blocks --------------------------
     const int kb0 = r0 / R, nbo = (nrow + R - 1) / R;
-    ClRecs Q{A.bptr + kb0, A.bcol, A.bcoef, 0u, 0u, -1, A.max_block};
+    ClRecs Q{A.bptr + kb0, A.bcol, A.bcoef, 0u, 0u, nullptr, -1};
     if (A.rec_smem) {
-        // block starts, columns (FP64), coefficients
-        const int lg = __ffs(32 / TL) - 1, per = 1 << lg;
-        const int slots = (nbo + per - 1) / per * per * A.max_block;
+        // block starts, group starts (a group is as long as its longest block), columns (FP64), coefficients
+        const int lg = __ffs(32 / TL) - 1, per = 1 << lg, ng = (nbo + per - 1) >> lg;
         int* sb = reinterpret_cast<int*>(smem + Y.rec);
+        int* sg = sb + nbo + 1;
         for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(A.bptr + kb0 + k);
-        unsigned char* q = smem + Y.rec + (((size_t)nbo + 1) * 4 + 15) / 16 * 16;
-        int* scol = reinterpret_cast<int*>(q);
-        if constexpr (sizeof(Real) == 8) q += ((size_t)slots * 4 + 15) / 16 * 16;
-        // a warp per block, a lane per entry
-        for (int k = warp; k < nbo; k += kClWarps) {
-            const int p0 = __ldg(A.bptr + kb0 + k), ne = __ldg(A.bptr + kb0 + k + 1) - p0;
-            const int g = (k >> lg) * A.max_block, i = k & (per - 1);
-            for (int e = lane; e < ne; e += 32) {
-                if constexpr (sizeof(Real) == 4) {
-                    reinterpret_cast<float4*>(q)[(g + e) * per + i] =
-                        __ldg(reinterpret_cast<const float4*>(A.bcoef) + p0 + e);
-                } else {
-                    const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)(p0 + e) * R;
-                    scol[(g + e) * per + i] = __ldg(A.bcol + p0 + e);
-                    if constexpr (R == 1) {
-                        reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
+        __syncthreads();
+        for (int g = warp; g < ng; g += kClWarps) {
+            const int k = (g << lg) + lane;
+            int len = lane < per && k < nbo ? sb[k + 1] - sb[k] : 0;
+            len = __reduce_max_sync(0xffffffffu, len);
+            if (lane == 0) sg[g + 1] = len;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            sg[0] = 0;
+            for (int g = 0; g < ng; ++g) sg[g + 1] += sg[g];
+        }
+        __syncthreads();
+        const size_t slots = (size_t)sg[ng] << lg, head = (((size_t)nbo + ng + 2) * 4 + 15) / 16 * 16;
+        const size_t cols = sizeof(Real) == 8 ? (slots * 4 + 15) / 16 * 16 : 0;
+        unsigned char* q = smem + Y.rec + head + cols;
+        Q.bptr = sb;
+        if (head + cols + slots * (sizeof(Real) == 8 ? R * 8 : 16) <= (size_t)A.rec_smem) {
+            int* scol = reinterpret_cast<int*>(smem + Y.rec + head);
+            // a warp per block, a lane per entry
+            for (int k = warp; k < nbo; k += kClWarps) {
+                const int p0 = sb[k], ne = sb[k + 1] - p0, g = sg[k >> lg], i = k & (per - 1);
+                for (int e = lane; e < ne; e += 32) {
+                    if constexpr (sizeof(Real) == 4) {
+                        reinterpret_cast<float4*>(q)[(g + e) * per + i] =
+                            __ldg(reinterpret_cast<const float4*>(A.bcoef) + p0 + e);
                     } else {
+                        const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)(p0 + e) * R;
+                        scol[(g + e) * per + i] = __ldg(A.bcol + p0 + e);
+                        if constexpr (R == 1) {
+                            reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
+                        } else {
 #pragma unroll
-                        for (int h = 0; h < R / 2; ++h)
-                            reinterpret_cast<double2*>(q)[((g + e) * (R / 2) + h) * per + i] =
-                                __ldg(reinterpret_cast<const double2*>(gr) + h);
+                            for (int h = 0; h < R / 2; ++h)
+                                reinterpret_cast<double2*>(q)[((g + e) * (R / 2) + h) * per + i] =
+                                    __ldg(reinterpret_cast<const double2*>(gr) + h);
+                        }
                     }
                 }
             }
+            Q.scol = sm_addr(scol);
+            Q.srec = sm_addr(q);
+            Q.goff = sg;
+            Q.lg = lg;
         }
-        Q.bptr = sb;
-        Q.scol = sm_addr(scol);
-        Q.srec = sm_addr(q);
-        Q.lg = lg;
     }
 
     // ---- r_1 = psi over the window, the diagonal (noise of this step, or as it is)
     if (act) {
-        const int step = *A.S.step;
+        const int step = kPlain ? A.step : *A.S.step;
         const double* D = A.noise == DQ_NOISE_ZZ && (A.flags & kClNoise)
                               ? A.zzD + (size_t)(step - *A.zz_start) * n * B : nullptr;
         Real* dg = reinterpret_cast<Real*>(A.diag);
         for (int row = rl - hlo; row < nrow + hhi; row += RL) {
             const size_t x = ((ptrdiff_t)r0 + row) * B + bb;
-            stv<Real, TPT>(cur + (ptrdiff_t)row * rowr, tl * TPT, ldv<Real, TPT, false>(slab(1), x));
+            stv<Real, TPT>(cur + (ptrdiff_t)row * rowr, tl * TPT, ldv<Real, TPT, false>(first, x));
             if (row < 0 || row >= nrow) continue;
             const size_t l = loc(row);
             if (!(A.flags & kClNoise)) {
@@ -469,7 +510,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     }
     if (threadIdx.x < TC) {
-        const double s1 = c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
+        const double s1 = kPlain ? 1.0 : c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
         scs[TC + threadIdx.x] = s1;
         par[TC + threadIdx.x] = make_double2(s1, 0.0);
         mtr[threadIdx.x] = 0;
@@ -489,14 +530,19 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         if (Q.lg < 0) {
             cl_gather<Real, TPT, R, false>(Q, p0, len, wcol, rowb, acc);
         } else {
-            const int slot = ((k >> Q.lg) * Q.maxb << Q.lg) + (k & ((1 << Q.lg) - 1));
+            const int slot = (Q.goff[k >> Q.lg] << Q.lg) + (k & ((1 << Q.lg) - 1));
             cl_gather<Real, TPT, R, true>(Q, sizeof(Real) == 4 ? slot << 4 : slot, len, wcol, rowb, acc);
         }
     };
-    // the neighbours' rows of the window's margins, as they are in their shared memory
-    auto margins = [&]() {
+    // The window's margins of r_j (j >= 2): the neighbours' rows from their shared memory, or, when
+    // the margins are wide, from the slab that the barrier has just published (a window of all 5,278
+    // rows in 11 CTAs: a step of 12 iterations took 232 us by DSMEM, 199 us this way)
+    const bool wide = (size_t)(hlo + hhi) * rowr * sizeof(Real) > kClWideMargin;
+    auto margins = [&](int j) {
         if constexpr (!kLocal) {
             const int nh = act ? hlo + hhi : 0;
+            const T* src = reinterpret_cast<const T*>(slab(j) + 2 * ((size_t)c0 * n + (act ? tl * TPT : 0)));
+            const int stride = tca / TPT;
             for (int h0 = rl; h0 < nh; h0 += 4 * RL) {
                 T v[4];
 #pragma unroll
@@ -504,10 +550,14 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     const int h = h0 + q * RL;
                     if (h >= nh) break;
                     const int g = r0 + (h < hlo ? h - hlo : nrow + h - hlo);
-                    int own = (int)rank;
-                    while (g < own * A.rpc) --own;
-                    while (g >= (own + 1) * A.rpc) ++own;
-                    v[q] = cl_load(reinterpret_cast<const T*>(cur + (size_t)(g - own * A.rpc) * rowr) + tl, own);
+                    if (wide) {
+                        v[q] = src[(size_t)g * stride];
+                    } else {
+                        const int own = g / A.rpc;
+                        // the owner's own rows start after its lower margin
+                        const int at = min(bw, own * A.rpc) + g - own * A.rpc;
+                        v[q] = cl_load(reinterpret_cast<const T*>(win + (size_t)at * rowr) + tl, own);
+                    }
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -520,7 +570,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     };
 
-    const bool adaptive = A.S.mtraj != nullptr;
+    const bool adaptive = !kPlain && A.S.mtraj != nullptr;
     // the last warp's lanes take the sums' scalars: the margins' loads start with the first warps
     const int last = warp == kClWarps - 1 ? lane : kMaxTC;
     int jl = A.m;   // iterations done
@@ -549,10 +599,20 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
 #pragma unroll
                 for (int t = 0; t < TPT; ++t) {
                     const Real dv = dsm[l + t];
-                    const Real ur = fma(dv, x.v[2 * t], fma(-fm[t], o.v[2 * t], acc[i].v[2 * t]));
-                    const Real ui = fma(dv, x.v[2 * t + 1], fma(-fm[t], o.v[2 * t + 1], acc[i].v[2 * t + 1]));
-                    o.v[2 * t] = ur;
-                    o.v[2 * t + 1] = ui;
+                    Real ur = acc[i].v[2 * t], ui = acc[i].v[2 * t + 1];
+                    if constexpr (kPlain) {
+                        // the reference's order: alpha_j from H q_j alone (the unconjugated dot of
+                        // complex states does not make q_j orthogonal to q_{j-1})
+                        ur = fma(dv, x.v[2 * t], ur);
+                        ui = fma(dv, x.v[2 * t + 1], ui);
+                        o.v[2 * t] = fma(-fm[t], o.v[2 * t], ur);
+                        o.v[2 * t + 1] = fma(-fm[t], o.v[2 * t + 1], ui);
+                    } else {
+                        ur = fma(dv, x.v[2 * t], fma(-fm[t], o.v[2 * t], ur));
+                        ui = fma(dv, x.v[2 * t + 1], fma(-fm[t], o.v[2 * t + 1], ui));
+                        o.v[2 * t] = ur;
+                        o.v[2 * t + 1] = ui;
+                    }
                     // the bilinear dot takes q_j itself, the Hermitian one its conjugate
                     const double xr = x.v[2 * t], xi = A.bil ? -x.v[2 * t + 1] : x.v[2 * t + 1], dr = ur, di = ui;
                     x2[t] += xr * dr + xi * di;
@@ -653,7 +713,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             // beta_j sc_j / sc_{j+1}
             par[TC + t] = make_double2(s1, bt * scj * (s1 > 0.0 ? nr : 0.0));
         }
-        margins();
+        margins(j + 1);
         __syncthreads();
         if (adaptive && j >= A.m_min && j < A.m && (j - A.m_min) % kMCheckStride == 0) {
             // EXPOKIT's first term per undecided trajectory; every CTA decides alike
@@ -704,7 +764,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     // ---- the recurrence's scalars (the adjoint and the getters read them) ----
     __syncthreads();
-    if (rank == 0) {
+    if (!kPlain && rank == 0) {
         for (int e = threadIdx.x; e < jl * TC; e += kClThreads) {
             const int j = 1 + e / TC, t = e % TC;
             if (c0 + t >= B) continue;
@@ -778,7 +838,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
         if (rank == 0 && lane == m - 1) {
             if (s < 0) atomicCAS(A.S.status, 0, DQ_ERR_SCALING);
-            else A.erracc[c0 + t] += estimate(m, t, f1, f2);
+            else cl_estimate<kPlain>(A, c0 + t, estimate(m, t, f1, f2));
         }
         if (adaptive && rank == 0 && lane == 0) A.S.mtraj[c0 + t] = m;
     }
@@ -801,12 +861,13 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 for (int j = threadIdx.x; j < mmax; j += kClThreads) {
                     const cd v = j < m && o.s >= 0 ? cscale(yd[j], scs[(j + 1) * TC + t]) : cmk(0.0, 0.0);
                     const size_t k = (size_t)(j + 1) * B + c0 + t;
-                    A.S.yt[2 * k] = v.x;
-                    A.S.yt[2 * k + 1] = v.y;
+                    double* yt = kPlain ? reinterpret_cast<double*>(A.ps->yt) : A.S.yt;
+                    yt[2 * k] = v.x;
+                    yt[2 * k + 1] = v.y;
                 }
                 if (threadIdx.x == 0 && o.s >= 0) {
                     if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
-                    A.erracc[c0 + t] += estimate(m, t, o.e_m1_m, o.e_m1_mp1);
+                    cl_estimate<kPlain>(A, c0 + t, estimate(m, t, o.e_m1_m, o.e_m1_mp1));
                 }
                 if (adaptive && threadIdx.x == 0) A.S.mtraj[c0 + t] = m;
                 __syncthreads();
@@ -817,7 +878,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             const int j = e / TC, t = e % TC;
             if (c0 + t >= B || mtr[t] >= 0) continue;
             const size_t k = (size_t)(j + 1) * B + c0 + t;
-            yts[e] = make_double2(A.S.yt[2 * k], A.S.yt[2 * k + 1]);
+            const double* yt = kPlain ? reinterpret_cast<const double*>(A.ps->yt) : A.S.yt;
+            yts[e] = make_double2(yt[2 * k], yt[2 * k + 1]);
         }
         __syncthreads();
     }
@@ -836,7 +898,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
                     if (j0 + q <= mmax)
-                        v[q] = j0 + q == 1 ? ldv<Real, TPT, false>(slab(1), x)
+                        v[q] = j0 + q == 1 ? ldv<Real, TPT, false>(first, x)
                                            : ldv<Real, TPT, false>(basis(j0 + q, row), 0);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
@@ -849,7 +911,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     }
                 }
             }
-            const cd p0 = A.bra[r0 + row];
+            const cd p0 = !kPlain || A.corr_pt ? A.bra[r0 + row] : cmk(0.0, 0.0);
             CV<Real, TPT> o;
 #pragma unroll
             for (int t = 0; t < TPT; ++t) {
@@ -860,14 +922,34 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 cr[t] += p0.x * vr + p0.y * vi;   // conj(bra) * psi
                 ci[t] += p0.x * vi - p0.y * vr;
             }
-            stv<Real, TPT>(slab(1), x, o);
+            if (kPlain) stv<Real, TPT>(prev, loc(row), o);   // its norm is not known yet
+            else stv<Real, TPT>(slab(1), x, o);
         }
     // ex[0] still holds ||H q_{m+1}||, which slower CTAs may be reading
     sum.sync();
     sum.template part<true>(0, cr, ci);
     sum.template part<false>(1, nn, nn);
     sum.sync();
-    if (rank == 0) {
+    if constexpr (kPlain) {
+        const double n2 = sum.get(1, 0).x, nrm = sqrt(n2), inv = 1. / nrm;
+        for (int k = rl; k < nbk; k += RL)
+            for (int row = k * R; row < min(nrow, k * R + R); ++row) {
+                const CV<Real, TPT> v = ldv<Real, TPT, false>(prev, loc(row));
+                const cd o = cmk(v.v[0] * inv, v.v[1] * inv);
+                A.psi_out[r0 + row] = o;
+                if (A.pops_row) A.pops_row[r0 + row] += cabs2(o);
+            }
+        if (rank == 0 && threadIdx.x == 0) {
+            A.ps->norm = nrm;
+            A.ps->invnorm = inv;
+            if (!(nrm > 0.0) || !isfinite(nrm)) atomicCAS(&A.ps->status, 0, DQ_ERR_NAN);
+            if (A.corr_pt) {
+                const double2 c = sum.get(0, 0);
+                A.corr_pt->x += c.x * inv;
+                A.corr_pt->y += c.y * inv;
+            }
+        }
+    } else if (rank == 0) {
         double* cs = reinterpret_cast<double*>(sum.red);   // free again: the chunk's correlation terms
         if (threadIdx.x < TC) {
             const int t = threadIdx.x, b = c0 + t;
@@ -951,7 +1033,7 @@ static cudaLaunchConfig_t cl_config(int chunks, int CS, size_t smem, cudaStream_
 // Bytes of the largest CTA's coupling records (block starts, columns, coefficients).
 static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R, int TL) {
     const size_t per = 32 / TL, nb = rpc / R, slots = (nb + per - 1) / per * per * (size_t)f.max_block;
-    const size_t head = ((nb + 1) * 4 + 15) / 16 * 16;
+    const size_t head = ((nb + (nb + per - 1) / per + 2) * 4 + 15) / 16 * 16;
     if (mixed) return head + slots * 16;
     return head + (slots * 4 + 15) / 16 * 16 + slots * R * sizeof(double);
 }
@@ -969,10 +1051,10 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
     const size_t rsz = bs->mixed ? sizeof(float) : sizeof(double);
     const int rpc = cl_rows(n, CS, R);
     size_t rb = cl_rec_bytes(f, bs->mixed, rpc, R, tc / tpt);
-    size_t sm = cl_layout(CS, tc, m, rpc, c->bw, rsz, rb).total;
+    size_t sm = cl_layout(n, CS, tc, m, rpc, c->bw, rsz, rb).total;
     if (sm > kClSmemMax) {
         rb = 0;
-        sm = cl_layout(CS, tc, m, rpc, c->bw, rsz, 0).total;
+        sm = cl_layout(n, CS, tc, m, rpc, c->bw, rsz, 0).total;
     }
     if (sm > kClSmemMax) return 0;
     int found = 0;
@@ -1045,7 +1127,6 @@ cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
     a.rpc = bs->rpc;
     a.bw = c->bw;
     a.rec_smem = (int)bs->cl_rec;
-    a.max_block = f.max_block;
     a.m = c->cfg.m;
     a.flags = whole_step ? kClNoise | kClFinish : 0;
     a.bil = c->cfg.dot_mode == DQ_DOT_BILINEAR;
@@ -1110,6 +1191,96 @@ dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R) {
     bs->staged = kStagedCluster;
     bs->groups = 1;
     return DQ_OK;
+}
+
+// ---- the drop-in step ------------------------------------------------------
+// A single trajectory: rows of the off-diagonal CSR as they are (R = 1), a
+// thread each, the records in shared memory where a CTA's turn out to fit (the
+// kernel looks).  `bw` is the matrix bandwidth, or n where only the device
+// knows the columns (then every CTA's window is the whole vector); `z` the
+// couplings of a row, 0 when unknown.  ctas = 0: too large for 16 CTAs.
+// Estimated cycles of an iteration: rounds of rows by the CTA's threads, the
+// wavefronts of the records and gathers (7 per 32 entries), the barriers.
+PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
+    PlainCluster best;
+    double t_best = 1e30;
+    for (int CS = 1; CS <= kClMaxCtas; ++CS) {
+        const int rpc = cl_rows(n, CS, 1);
+        if (CS > 1 && ((size_t)rpc * (CS - 1) >= (size_t)n || rpc < 32)) continue;
+        const size_t fixed = cl_layout(n, CS, 1, m, rpc, bw, sizeof(double), 0).total;
+        if (fixed + 4096 > kClSmemMax) continue;
+        const size_t room = (kClSmemMax - fixed) / 16 * 16 - 16;
+        const double zz = z > 0.0 ? z : 8.0;
+        if (rpc * (zz * 1.15 + 2.0) * 12.0 > (double)room) continue;
+        // unknown rows may be long: as many CTAs as there are rows for, so that their records fit
+        const double t = z > 0.0 ? std::ceil((double)rpc / kClThreads) * (400.0 + 75.0 * z) + 0.25 * rpc * z +
+                                       (CS > 1 ? 700.0 + 60.0 * CS : 0.0)
+                                 : std::abs(rpc - 128.0);
+        if (t < t_best) {
+            t_best = t;
+            best.ctas = CS;
+            best.rpc = rpc;
+            best.smem = fixed + room;
+            best.rec = room;
+        }
+    }
+    return best;
+}
+
+cudaError_t plain_cluster_attributes() {
+    cudaError_t e = raise_smem_limit(k_cluster_step<double, 1, 1, true, true>, (int)kClSmemMax);
+    if (e == cudaSuccess) e = raise_smem_limit(k_cluster_step<double, 1, 1, false, true>, (int)kClSmemMax);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_cluster_step<double, 1, 1, false, true>,
+                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cudaStream_t st) {
+    ClusterArgs a = {};
+    a.n = q.n;
+    a.B = 1;
+    a.TC = 1;
+    a.rpc = P.rpc;
+    a.bw = q.bw;
+    a.m = q.m;
+    a.flags = kClFinish | (q.draw ? kClNoise : 0);
+    a.bil = q.dot_mode == DQ_DOT_BILINEAR;
+    a.chunks = 1;
+    a.rec_smem = (int)P.rec;
+    a.bptr = q.rowptr;
+    a.bcol = q.col;
+    a.bcoef = q.val;
+    a.slabs = q.Q;
+    a.slab = (size_t)q.n;
+    a.diag = q.diag;
+    a.S.status = &q.ps->status;
+    a.noise = q.noise;
+    a.ns = q.ns;
+    a.traj0 = q.traj;
+    a.step = q.step;
+    a.subdt = q.subdt;
+    a.sqrt_subdt = sqrt(q.subdt);
+    a.seed = q.seed;
+    a.sigma = q.sigma;
+    a.invtau = q.invtau;
+    a.coeff = q.coeff;
+    a.eps = q.eps;
+    a.deps = q.deps;
+    a.norm_mode = q.norm_mode;
+    a.tau_im = q.tau_im;
+    a.erracc = q.erracc;
+    a.bra = q.bra;
+    a.psi_in = q.psi_in;
+    a.psi_out = q.psi_out;
+    a.pops_row = q.pops_row;
+    a.corr_pt = q.corr_pt;
+    a.ps = q.ps;
+    a.scratch = q.scratch;
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cl_config(1, P.ctas, P.smem, st, &at);
+    return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, true>
+                                                : k_cluster_step<double, 1, 1, false, true>, a);
 }
 
 }  // namespace dq

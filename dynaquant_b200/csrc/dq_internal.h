@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <string>
 #include <vector>
 
@@ -34,6 +35,40 @@ constexpr int kPlainThreads = 256;
 constexpr int kMaxPartials = 4096;
 constexpr int kMaxZZOsc = 1024;   // oscillators of one ZZ spectral density
 constexpr int kIprRowGroups = 296; // row groups of the ensemble IPR reduction (2 per SM)
+
+// The one-launch drop-in step (dq_cluster.cu): CTAs of its cluster (0: the
+// system is too large for it), rows per CTA, shared memory.
+struct PlainCluster {
+    int ctas = 0, rpc = 0;
+    size_t smem = 0, rec = 0;
+};
+
+// What one such step reads and writes (device pointers).
+struct PlainStep {
+    int n, m, bw, dot_mode, norm_mode;
+    const int* rowptr;       // off-diagonal CSR
+    const int* col;
+    const double* val;
+    double* diag;            // written when the step draws its noise, else read
+    const cd* psi_in;
+    cd* psi_out;
+    cd* Q;                   // m + 2 vectors of n
+    PlainScalars* ps;
+    double tau_im;
+    // noise of the step (draw): trajectory, step and the parameters of k_noise
+    bool draw;
+    int noise, ns, traj, step;
+    double subdt;
+    uint64_t seed;
+    const double *sigma, *invtau, *coeff, *eps;
+    double* deps;
+    // records (may be null)
+    double* erracc;
+    double* pops_row;
+    cd* corr_pt;
+    const cd* bra;
+    unsigned char* scratch;  // pade_smem_bytes(m + 2)
+};
 
 struct BatchedState;   // dq_batched.cu
 struct TkEnsemble;     // dq_tk_ensemble.cu
@@ -91,6 +126,8 @@ struct dq_ctx {
     dq::cd* d_psi_b = nullptr;
     double* d_partial = nullptr;  // kMaxPartials x 2
     dq::PlainScalars* d_ps = nullptr;
+    unsigned char* d_pade = nullptr;       // the one-launch step's dense exponential
+    dq::PlainCluster plain;                // its shape for the Hamiltonian that is set
 
     // observables (sums over trajectories; divided by n_traj on read)
     int n_rec_max = 0;
@@ -169,6 +206,10 @@ dq_status plain_clear_observables(dq_ctx* c);
 dq_status plain_observe_initial(dq_ctx* c);
 dq_status check_cuda(dq_ctx* c, cudaError_t e, const char* what);
 dq_status read_status(dq_ctx* c, int code, const char* what);
+// implemented in dq_cluster.cu
+PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
+cudaError_t plain_cluster_attributes();
+cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cudaStream_t st);
 // implemented in dq_batched.cu
 // default_tiling = false leaves the tiling unset (TC = 0) for a caller that
 // sets one at once (batched_set_tiling, or batched_default_tiling)

@@ -484,6 +484,7 @@ dq_status plain_alloc(dq_ctx* c) {
     DQ_CU(cudaMalloc(&c->d_psi_b, sizeof(cd) * n));
     DQ_CU(cudaMalloc(&c->d_partial, sizeof(double) * 2 * kMaxPartials));
     DQ_CU(cudaMalloc(&c->d_ps, sizeof(PlainScalars)));
+    DQ_CU(cudaMalloc(&c->d_pade, pade_smem_bytes(m + 2)));
     DQ_CU(cudaMemsetAsync(c->d_ps, 0, sizeof(PlainScalars), c->stream));
     DQ_CU(cudaMemsetAsync(c->d_Q, 0, sizeof(cd) * (size_t)n * (m + 2), c->stream));
     // the limit is a per-function attribute shared by every context (and by
@@ -493,12 +494,14 @@ dq_status plain_alloc(dq_ctx* c) {
     (void)m;
     DQ_CU(raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL)));
     DQ_CU(raise_smem_limit(k_pade_tk, (int)pade_smem_bytes(kMaxL)));
+    DQ_CU(plain_cluster_attributes());
     return DQ_OK;
 }
 
 void plain_free(dq_ctx* c) {
     cudaFree(c->d_eps_p); cudaFree(c->d_deps_p); cudaFree(c->d_diag); cudaFree(c->d_Q); cudaFree(c->d_w);
-    cudaFree(c->d_psi_a); cudaFree(c->d_psi_b); cudaFree(c->d_partial); cudaFree(c->d_ps);
+    cudaFree(c->d_psi_a); cudaFree(c->d_psi_b); cudaFree(c->d_partial); cudaFree(c->d_ps); cudaFree(c->d_pade);
+    c->d_pade = nullptr;
     c->d_eps_p = c->d_deps_p = c->d_diag = c->d_partial = nullptr;
     c->d_Q = c->d_w = c->d_psi_a = c->d_psi_b = nullptr;
     c->d_ps = nullptr;
@@ -586,7 +589,11 @@ dq_status plain_step(dq_ctx* c, int traj, int step, const cd* psi_in, cd* psi_ou
     const double sqrt_subdt = sqrt(subdt);
     const double* eps = c->d_eps_p + (size_t)traj * n;
     double* deps = c->d_deps_p + (size_t)traj * n;
-    if (c->cfg.noise_model == DQ_NOISE_ZZ) {
+    // small systems: noise to normalisation in one launch of one cluster (the ZZ sums have their own)
+    // that launch reads psi_in 16 bytes at a time; a caller's pointer is only promised 8
+    const bool one = c->plain.ctas > 0 && c->tk_p == 0 && !c->cfg.reorth && ((uintptr_t)psi_in & 15) == 0;
+    if (one && c->cfg.noise_model != DQ_NOISE_ZZ) {
+    } else if (c->cfg.noise_model == DQ_NOISE_ZZ) {
         ZZParams zz;
         zz.n_osc = c->zz_n_osc;
         zz.omega = c->d_zz_omega;
@@ -596,6 +603,44 @@ dq_status plain_step(dq_ctx* c, int traj, int step, const cd* psi_in, cd* psi_ou
     } else {
         k_noise<<<G, T, 0, st>>>(n, c->traj0 + traj, step, c->cfg.noise_model, ns, subdt, sqrt_subdt, c->cfg.seed, c->d_sigma,
                                  c->d_invtau, c->d_coeff, eps, deps, c->d_diag, c->d_ps);
+    }
+    if (one) {
+        PlainStep q;
+        q.n = n;
+        q.m = m;
+        q.bw = c->bw;
+        q.dot_mode = c->cfg.dot_mode;
+        q.norm_mode = c->cfg.norm_mode;
+        q.rowptr = c->d_rowptr;
+        q.col = c->d_col;
+        q.val = c->d_val;
+        q.diag = c->d_diag;
+        q.psi_in = psi_in;
+        q.psi_out = psi_out;
+        q.Q = c->d_Q;
+        q.ps = c->d_ps;
+        q.tau_im = c->tau_im;
+        q.draw = c->cfg.noise_model != DQ_NOISE_ZZ;
+        q.noise = c->cfg.noise_model;
+        q.ns = ns;
+        q.traj = c->traj0 + traj;
+        q.step = step;
+        q.subdt = subdt;
+        q.seed = c->cfg.seed;
+        q.sigma = c->d_sigma;
+        q.invtau = c->d_invtau;
+        q.coeff = c->d_coeff;
+        q.eps = eps;
+        q.deps = deps;
+        q.erracc = observe ? c->d_erracc + traj : nullptr;
+        q.pops_row = (observe && rec >= 0) ? c->d_pops + (size_t)rec * n : nullptr;
+        q.corr_pt = observe ? c->d_corr + (step + 1) : nullptr;
+        q.bra = corr_bra(c);
+        q.scratch = c->d_pade;
+        DQ_CU(plain_cluster_launch(c->plain, q, st));
+        if (observe && c->ipr_on) k_ipr_plain<<<G, T, 0, st>>>(n, psi_out, c->d_ipr + step + 1, c->d_partial, c->d_ps);
+        DQ_CU(cudaGetLastError());
+        return DQ_OK;
     }
     if (c->tk_p > 0) return plain_tk_tail(c, traj, step, psi_in, psi_out, observe, rec);
     plain_lanczos(c, m, c->d_rowptr, c->d_col, c->d_val, c->d_diag, psi_in, c->d_Q);
@@ -730,6 +775,11 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
     const size_t off_w = off_partial + align256(sizeof(double) * 2 * kMaxPartials);
     const size_t off_q = off_w + align256(sizeof(cd) * (size_t)n);
     const size_t need = off_q + sizeof(cd) * (size_t)n * (size_t)(m + 2);
+    // one launch where the whole vector fits every CTA's window (the columns are known on the device
+    // only) and the dense exponential's matrices the rest of the array
+    const size_t off_pade = align256(need);
+    PlainCluster shape;
+    if (off_pade + pade_smem_bytes(m + 2) <= kStaticScratchBytes && ((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0);
     if (G > kMaxPartials || need > kStaticScratchBytes) {
         char msg[200];
         snprintf(msg, sizeof msg,
@@ -756,6 +806,7 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
             cudaError_t e = cudaGetSymbolAddress(&p, g_dq_static_scratch);
             if (e == cudaSuccess)
                 e = raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL));
+            if (e == cudaSuccess) e = plain_cluster_attributes();
             if (e != cudaSuccess) {
                 write_err(errbuf, errbuf_len, cudaGetErrorString(e));
                 return DQ_ERR_CUDA;
@@ -778,22 +829,43 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
         hbar = (1 / 100.) * (1e15) * 1. / (299792548. * 2 * pi);   // cppUtility.cpp:19-22
     }
     const double tau_im = -dt / hbar;
-    k_static_begin<<<1, 32, 0, st>>>(ps);
-    for (int j = 1; j <= m; ++j) {
-        const cd* rj = (j == 1) ? pin : Q + (size_t)j * n;
-        const cd* rjm = (j <= 1) ? nullptr : (j == 2 ? pin : Q + (size_t)(j - 1) * n);
-        cd* rjp = Q + (size_t)(j + 1) * n;
-        if (dot_mode == DQ_DOT_BILINEAR)
-            k_spmv_alpha<true><<<G, T, 0, st>>>(n, j, rowptr, col, val, diag, rj, w, partial, ps);
-        else
-            k_spmv_alpha<false><<<G, T, 0, st>>>(n, j, rowptr, col, val, diag, rj, w, partial, ps);
-        k_axpy_norm<<<G, T, 0, st>>>(n, j, w, rj, rjm, rjp, partial, ps);
+    cudaError_t e = cudaSuccess;
+    if (shape.ctas > 0) {
+        PlainStep q = {};
+        q.n = n;
+        q.m = m;
+        q.bw = n;
+        q.dot_mode = dot_mode;
+        q.norm_mode = norm_mode;
+        q.rowptr = rowptr;
+        q.col = col;
+        q.val = val;
+        q.diag = const_cast<double*>(diag);   // read only: the step draws no noise
+        q.psi_in = pin;
+        q.psi_out = pout;
+        q.Q = Q;
+        q.ps = ps;
+        q.tau_im = tau_im;
+        q.scratch = base + off_pade;
+        e = plain_cluster_launch(shape, q, st);
+    } else {
+        k_static_begin<<<1, 32, 0, st>>>(ps);
+        for (int j = 1; j <= m; ++j) {
+            const cd* rj = (j == 1) ? pin : Q + (size_t)j * n;
+            const cd* rjm = (j <= 1) ? nullptr : (j == 2 ? pin : Q + (size_t)(j - 1) * n);
+            cd* rjp = Q + (size_t)(j + 1) * n;
+            if (dot_mode == DQ_DOT_BILINEAR)
+                k_spmv_alpha<true><<<G, T, 0, st>>>(n, j, rowptr, col, val, diag, rj, w, partial, ps);
+            else
+                k_spmv_alpha<false><<<G, T, 0, st>>>(n, j, rowptr, col, val, diag, rj, w, partial, ps);
+            k_axpy_norm<<<G, T, 0, st>>>(n, j, w, rj, rjm, rjp, partial, ps);
+        }
+        k_spmv_norm<<<G, T, 0, st>>>(n, m + 1, rowptr, col, val, diag, Q + (size_t)(m + 1) * n, partial, ps);
+        k_pade_plain<<<1, 256, pade_smem_bytes(m + 2), st>>>(m, tau_im, norm_mode, ps, nullptr, 0);
+        k_combine<<<G, T, 0, st>>>(n, m, pin, Q, pout, partial, ps);
+        k_renorm<<<G, T, 0, st>>>(n, pout, nullptr, nullptr, nullptr, partial, ps);
+        e = cudaGetLastError();
     }
-    k_spmv_norm<<<G, T, 0, st>>>(n, m + 1, rowptr, col, val, diag, Q + (size_t)(m + 1) * n, partial, ps);
-    k_pade_plain<<<1, 256, pade_smem_bytes(m + 2), st>>>(m, tau_im, norm_mode, ps, nullptr, 0);
-    k_combine<<<G, T, 0, st>>>(n, m, pin, Q, pout, partial, ps);
-    k_renorm<<<G, T, 0, st>>>(n, pout, nullptr, nullptr, nullptr, partial, ps);
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         write_err(errbuf, errbuf_len, cudaGetErrorString(e));
         return DQ_ERR_CUDA;
