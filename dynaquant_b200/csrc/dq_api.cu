@@ -291,13 +291,18 @@ dq_status dq_set_taylor_krylov(dq_ctx* c, int p, int m_b, const int* rowptr, con
     // split B into its diagonal and off-diagonal CSR like the Hamiltonian
     std::vector<int> rp(n + 1, 0), cl;
     std::vector<double> vb, dg(n, 0.0);
+    int bw = 0;
     for (int i = 0; i < n; ++i) {
         for (int q = rowptr[i]; q < rowptr[i + 1]; ++q) {
             const int j = col[q];
             if (j < 0 || j >= n) return fail(c, DQ_ERR_ARG, "taylor_krylov: column index out of range");
             if (!std::isfinite(val[q])) return fail(c, DQ_ERR_ARG, "taylor_krylov: non-finite value");
             if (j == i) dg[i] += val[q];
-            else { cl.push_back(j); vb.push_back(val[q]); }
+            else {
+                cl.push_back(j);
+                vb.push_back(val[q]);
+                bw = std::max(bw, std::abs(j - i));
+            }
         }
         rp[i + 1] = (int)cl.size();
     }
@@ -325,6 +330,8 @@ dq_status dq_set_taylor_krylov(dq_ctx* c, int p, int m_b, const int* rowptr, con
     }
     c->tk_p = p;
     c->tk_m = m_b;
+    c->tk_bw = bw;
+    c->tk_nnz = rp[n];
     c->ready = false;
     return DQ_OK;
 }

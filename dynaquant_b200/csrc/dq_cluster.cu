@@ -72,17 +72,26 @@ struct ClusterArgs {
     double* pops_row;
     cd* corr_pt;
     PlainScalars* ps;
+    // Taylor-Krylov step (kTaylor): psi_in and psi_out are the ensemble's states, the matrix above is the
+    // step's Hamiltonian, the Lanczos iterations run on B; per trajectory <bra|psi> and sum |psi|^4
+    int tk_p;
+    const int* b_ptr;
+    const int* b_col;
+    const double* b_val;
+    const double* b_diag;
+    cd tk_coef[kMaxL];        // tau^k / k!
+    double* tk_obs;           // [3][B]
     unsigned char* scratch;   // per chunk, for the dense exponential
     size_t scratch_stride;
 };
 
 // Shared memory of a CTA: reductions, the chunk's scalars, the vectors, the records.
 struct ClLayout {
-    size_t ex, red, al, y, par, be, sc, win, prev, d, rec, total;
+    size_t ex, red, al, y, par, be, sc, win, prev, d, acc, rec, total;
 };
 
 static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int m, int rpc, int bw, size_t rsz,
-                                                     size_t rec) {
+                                                     size_t rec, bool taylor = false) {
     ClLayout L;
     size_t p = 0;
     L.ex = p; p += sizeof(double2) * 2 * CS * TC;
@@ -98,6 +107,8 @@ static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int 
     L.win = p; p += (CS > 1 ? (wide < (size_t)n ? wide : (size_t)(n > rpc ? n : rpc)) : rpc) * row;
     L.prev = p; p += rpc * row;
     L.d = p; p += rpc * row / 2;
+    p = (p + 15) & ~(size_t)15;
+    L.acc = p; p += taylor ? rpc * row : 0;   // the Taylor sum of the own rows
     p = (p + 15) & ~(size_t)15;
     L.rec = p; p += rec;
     L.total = (p + 15) & ~(size_t)15;
@@ -145,6 +156,37 @@ __device__ __forceinline__ T cl_load(const T* p, unsigned rank) {
 __device__ __noinline__ PadeOut cl_dense(int m, const cd* al, const cd* be, double tau_im, int norm_mode, cd* y,
                                          unsigned char* scratch) {
     return pade_exp_tbar(m, al, be, cmk(0.0, tau_im), norm_mode, y, scratch);
+}
+
+// the same for Taylor-Krylov's augmented matrix: y is its last column
+__device__ __noinline__ PadeOut cl_dense_tk(int mb, int p, const cd* al, const cd* be, double tau_im, int norm_mode,
+                                            cd* y, unsigned char* scratch) {
+    const int L = mb + p;
+    cd* A = reinterpret_cast<cd*>(scratch);
+    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
+        const int i = e / L, j = e % L;
+        cd v = cmk(0.0, 0.0);
+        if (i < mb && j < mb) {
+            if (i == j) v = al[i + 1];
+            else if (j == i + 1) v = be[i + 1];
+            else if (i == j + 1) v = be[j + 1];
+        } else if ((i == 0 && j == mb) || (i >= mb && j == i + 1)) {
+            v = cmk(1.0, 0.0);
+        }
+        A[e] = cmul(cmk(0.0, tau_im), v);
+    }
+    __syncthreads();
+    cd* E = nullptr;
+    PadeOut o;
+    o.s = pade_exp_sm(L, norm_mode, scratch, &E);
+    o.e_m1_m = o.e_m1_mp1 = cmk(0.0, 0.0);
+    if (o.s >= 0) {
+        for (int j = threadIdx.x; j < mb; j += blockDim.x) y[j] = E[j * L + L - 1];
+        o.e_m1_m = E[(mb - 1) * L + mb];
+        o.e_m1_mp1 = E[(mb - 1) * L + mb + 1];
+    }
+    __syncthreads();
+    return o;
 }
 
 // One CTA's view of its cluster's sums.
@@ -354,8 +396,12 @@ __device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double 
     }
 }
 
-template <typename Real, int TPT, int R, bool kLocal, bool kPlain = false>
+// What a launch carries through its step.
+enum { kEnsemble = 0, kDropIn = 1, kTaylor = 2 };
+
+template <typename Real, int TPT, int R, bool kLocal, int kMode = kEnsemble>
 __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArgs A) {
+    constexpr bool kPlain = kMode == kDropIn, kTk = kMode == kTaylor;
     using T = typename VL<Real, TPT>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int mtr[kMaxTC];
@@ -364,7 +410,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const int CS = kLocal ? 1 : (int)cl_size();
     const unsigned rank = kLocal ? 0u : cl_rank();
     const int bw = kLocal ? 0 : A.bw;
-    const ClLayout Y = cl_layout(n, CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem);
+    const ClLayout Y = cl_layout(n, CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem, kTk);
     double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
     double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
     // [0][t] the update's coefficients, [1][t] (sc_j, the factor of r_{j-1}), [2][t] complex64: Im alpha's low part
@@ -390,7 +436,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const int hhi = kLocal ? 0 : min(bw, n - (r0 + nrow));
     Real* slabs = reinterpret_cast<Real*>(A.slabs);
     auto slab = [&](int j) { return slabs + 2 * A.slab * j; };
-    const Real* first = kPlain ? reinterpret_cast<const Real*>(A.psi_in) : slab(1);
+    const Real* first = kPlain || kTk ? reinterpret_cast<const Real*>(A.psi_in) : slab(1);
     // own row `row` (within the CTA) of this thread's trajectories
     auto loc = [&](int row) { return (size_t)row * TC + tl * TPT; };
     auto glo = [&](int row) { return (size_t)(r0 + row) * B + bb; };
@@ -403,13 +449,15 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
 
     // ---- the coupling records of the own row blocks --------------------------
     const int kb0 = r0 / R, nbo = (nrow + R - 1) / R;
-    ClRecs Q{A.bptr + kb0, A.bcol, A.bcoef, 0u, 0u, nullptr, -1};
-    if (A.rec_smem) {
+    ClRecs Q;
+    auto load_records = [&](const int* gptr, const int* gcol, const void* gcoef) {
+        Q = ClRecs{gptr + kb0, gcol, gcoef, 0u, 0u, nullptr, -1};
+        if (!A.rec_smem) return;
         // block starts, group starts (a group is as long as its longest block), columns (FP64), coefficients
         const int lg = __ffs(32 / TL) - 1, per = 1 << lg, ng = (nbo + per - 1) >> lg;
         int* sb = reinterpret_cast<int*>(smem + Y.rec);
         int* sg = sb + nbo + 1;
-        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(A.bptr + kb0 + k);
+        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(gptr + kb0 + k);
         __syncthreads();
         for (int g = warp; g < ng; g += kClWarps) {
             const int k = (g << lg) + lane;
@@ -435,10 +483,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 for (int e = lane; e < ne; e += 32) {
                     if constexpr (sizeof(Real) == 4) {
                         reinterpret_cast<float4*>(q)[(g + e) * per + i] =
-                            __ldg(reinterpret_cast<const float4*>(A.bcoef) + p0 + e);
+                            __ldg(reinterpret_cast<const float4*>(gcoef) + p0 + e);
                     } else {
-                        const Real* gr = reinterpret_cast<const Real*>(A.bcoef) + (size_t)(p0 + e) * R;
-                        scol[(g + e) * per + i] = __ldg(A.bcol + p0 + e);
+                        const Real* gr = reinterpret_cast<const Real*>(gcoef) + (size_t)(p0 + e) * R;
+                        scol[(g + e) * per + i] = __ldg(gcol + p0 + e);
                         if constexpr (R == 1) {
                             reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
                         } else {
@@ -455,11 +503,12 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             Q.goff = sg;
             Q.lg = lg;
         }
-    }
+    };
+    load_records(A.bptr, A.bcol, A.bcoef);
 
     // ---- r_1 = psi over the window, the diagonal (noise of this step, or as it is)
     if (act) {
-        const int step = kPlain ? A.step : *A.S.step;
+        const int step = kMode != kEnsemble ? A.step : *A.S.step;
         const double* D = A.noise == DQ_NOISE_ZZ && (A.flags & kClNoise)
                               ? A.zzD + (size_t)(step - *A.zz_start) * n * B : nullptr;
         Real* dg = reinterpret_cast<Real*>(A.diag);
@@ -510,7 +559,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     }
     if (threadIdx.x < TC) {
-        const double s1 = kPlain ? 1.0 : c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
+        const double s1 = kPlain || kTk ? 1.0 : c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
         scs[TC + threadIdx.x] = s1;
         par[TC + threadIdx.x] = make_double2(s1, 0.0);
         mtr[threadIdx.x] = 0;
@@ -570,9 +619,61 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     };
 
-    const bool adaptive = !kPlain && A.S.mtraj != nullptr;
+    const bool adaptive = kMode == kEnsemble && A.S.mtraj != nullptr;
     // the last warp's lanes take the sums' scalars: the margins' loads start with the first warps
     const int last = warp == kClWarps - 1 ? lane : kMaxTC;
+    if constexpr (kTk) {
+        // the Taylor sum over k < p of tau^k / k! A^k psi, and r_1 = A^p psi with its norm
+        Real* tsum = reinterpret_cast<Real*>(smem + Y.acc);
+        for (int k = rl; k < nbk; k += RL) stv<Real, TPT>(tsum, loc(k), ldv<Real, TPT, false>(cur, loc(k)));
+        double b2[TPT];
+        for (int q = 1; q <= A.tk_p; ++q) {
+            for (int k = rl; k < nbk; k += RL) {
+                CV<Real, TPT> acc[R];
+                product(k, acc);
+                const size_t l = loc(k);
+                const CV<Real, TPT> x = ldv<Real, TPT, false>(cur, l);
+#pragma unroll
+                for (int v = 0; v < 2 * TPT; ++v) acc[0].v[v] = fma(dsm[l + v / 2], x.v[v], acc[0].v[v]);
+                stv<Real, TPT>(prev, l, acc[0]);
+            }
+            sum.sync();   // the neighbours have read these rows into their margins
+            const cd c = q < A.tk_p ? A.tk_coef[q] : cmk(0.0, 0.0);
+            b2[0] = 0.0;
+            for (int k = rl; k < nbk; k += RL) {
+                const size_t l = loc(k);
+                const CV<Real, TPT> y = ldv<Real, TPT, false>(prev, l);
+                stv<Real, TPT>(cur, l, y);
+                stv<Real, TPT>(basis(1, k), 0, y);
+                if (q < A.tk_p) {
+                    CV<Real, TPT> a = ldv<Real, TPT, false>(tsum, l);
+                    a.v[0] += c.x * y.v[0] - c.y * y.v[1];
+                    a.v[1] += c.x * y.v[1] + c.y * y.v[0];
+                    stv<Real, TPT>(tsum, l, a);
+                } else {
+                    b2[0] += (double)y.v[0] * y.v[0] + (double)y.v[1] * y.v[1];
+                }
+            }
+            if (q == A.tk_p) sum.template part<false>(1, b2, b2);
+            sum.sync();
+            margins(1);
+            if (q == A.tk_p) {
+                for (int t = last; t < TC; t += 32) {
+                    const double nb = sqrt(sum.get(1, t).x);
+                    if ((!(nb > 0.0) || !isfinite(nb)) && c0 + t < B && rank == 0) atomicCAS(A.S.status, 0, DQ_ERR_NAN);
+                    const double s1 = 1.0 / nb;
+                    scs[TC + t] = s1;
+                    par[TC + t] = make_double2(s1, 0.0);
+                }
+                // the Lanczos iterations run on B
+                for (int k = rl; k < nbk; k += RL)
+#pragma unroll
+                    for (int t = 0; t < TPT; ++t) dsm[loc(k) + t] = (Real)A.b_diag[r0 + k];
+                load_records(A.b_ptr, A.b_col, A.b_val);
+            }
+            __syncthreads();
+        }
+    }
     int jl = A.m;   // iterations done
     for (int j = 1; j <= A.m; ++j) {
         // u = H r_j - (beta_{j-1} sc_{j-1} / sc_j) r_{j-1} over r_{j-1} (w = sc_j u); alpha_j
@@ -600,7 +701,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 for (int t = 0; t < TPT; ++t) {
                     const Real dv = dsm[l + t];
                     Real ur = acc[i].v[2 * t], ui = acc[i].v[2 * t + 1];
-                    if constexpr (kPlain) {
+                    if constexpr (kMode != kEnsemble) {
                         // the reference's order: alpha_j from H q_j alone (the unconjugated dot of
                         // complex states does not make q_j orthogonal to q_{j-1})
                         ur = fma(dv, x.v[2 * t], ur);
@@ -764,7 +865,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     // ---- the recurrence's scalars (the adjoint and the getters read them) ----
     __syncthreads();
-    if (!kPlain && rank == 0) {
+    if (kMode == kEnsemble && rank == 0) {
         for (int e = threadIdx.x; e < jl * TC; e += kClThreads) {
             const int j = 1 + e / TC, t = e % TC;
             if (c0 + t >= B) continue;
@@ -824,8 +925,15 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         const int m = adaptive && mtr[t] ? mtr[t] : A.m;
         const int q = (min(lane, m - 1) + 1) * TC + t;
         cd y, f1, f2;
-        int s;
-        const bool ok = series_exp_tbar(m, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
+        int s = 0;
+        bool ok;
+        if constexpr (kTk) {
+            // the weights are the last column's, times ||A^p psi|| = 1 / sc_1
+            ok = series_exp_tk(m, A.tk_p, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2);
+            y = cscale(y, 1.0 / scs[TC + t]);
+        } else {
+            ok = series_exp_tbar(m, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
+        }
         if (!ok) {
             if (lane == 0) atomicOr(&flag, 1);
             if (lane == 0) mtr[t] = -m;   // dense below
@@ -838,6 +946,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
         if (rank == 0 && lane == m - 1) {
             if (s < 0) atomicCAS(A.S.status, 0, DQ_ERR_SCALING);
+            else if constexpr (kTk) A.tk_obs[c0 + t] = estimate(m, t, f1, f2);   // completed with the norm below
             else cl_estimate<kPlain>(A, c0 + t, estimate(m, t, f1, f2));
         }
         if (adaptive && rank == 0 && lane == 0) A.S.mtraj[c0 + t] = m;
@@ -854,20 +963,27 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     bed[i] = i >= 1 && i <= m ? cmk(be[i * TC + t], 0.0) : cmk(0, 0);
                 }
                 __syncthreads();
-                const PadeOut o = cl_dense(m, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
+                PadeOut o;
+                if constexpr (kTk) {
+                    o = cl_dense_tk(m, A.tk_p, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
+                    for (int j = threadIdx.x; j < m; j += kClThreads) yd[j] = cscale(yd[j], 1.0 / scs[TC + t]);
+                } else {
+                    o = cl_dense(m, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
+                }
                 __syncthreads();
                 if (o.s < 0 && threadIdx.x == 0)
                     atomicCAS(A.S.status, 0, o.s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
                 for (int j = threadIdx.x; j < mmax; j += kClThreads) {
                     const cd v = j < m && o.s >= 0 ? cscale(yd[j], scs[(j + 1) * TC + t]) : cmk(0.0, 0.0);
                     const size_t k = (size_t)(j + 1) * B + c0 + t;
-                    double* yt = kPlain ? reinterpret_cast<double*>(A.ps->yt) : A.S.yt;
+                    double* yt = kPlain ? reinterpret_cast<double*>(A.ps->yt) : A.S.yt;   // [j][trajectory]
                     yt[2 * k] = v.x;
                     yt[2 * k + 1] = v.y;
                 }
                 if (threadIdx.x == 0 && o.s >= 0) {
                     if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
-                    cl_estimate<kPlain>(A, c0 + t, estimate(m, t, o.e_m1_m, o.e_m1_mp1));
+                    if constexpr (kTk) A.tk_obs[c0 + t] = estimate(m, t, o.e_m1_m, o.e_m1_mp1);
+                    else cl_estimate<kPlain>(A, c0 + t, estimate(m, t, o.e_m1_m, o.e_m1_mp1));
                 }
                 if (adaptive && threadIdx.x == 0) A.S.mtraj[c0 + t] = m;
                 __syncthreads();
@@ -884,9 +1000,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         __syncthreads();
     }
     // ---- psi = sum_j yt_j r_j over slab 1, its norm, <bra|psi> -----------------
-    double nn[TPT], cr[TPT], ci[TPT];
+    double nn[TPT], cr[TPT], ci[TPT], q4[TPT];
 #pragma unroll
-    for (int t = 0; t < TPT; ++t) nn[t] = cr[t] = ci[t] = 0.0;
+    for (int t = 0; t < TPT; ++t) nn[t] = cr[t] = ci[t] = q4[t] = 0.0;
     for (int k = rl; k < nbk; k += RL)
         for (int row = k * R; row < min(nrow, k * R + R); ++row) {
             const size_t x = glo(row);
@@ -898,7 +1014,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
                     if (j0 + q <= mmax)
-                        v[q] = j0 + q == 1 ? ldv<Real, TPT, false>(first, x)
+                        v[q] = j0 + q == 1 && !kTk ? ldv<Real, TPT, false>(first, x)
                                            : ldv<Real, TPT, false>(basis(j0 + q, row), 0);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
@@ -911,6 +1027,11 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     }
                 }
             }
+            if constexpr (kTk) {
+                const CV<Real, TPT> a = ldv<Real, TPT, false>(reinterpret_cast<const Real*>(smem + Y.acc), loc(row));
+                pr[0] += a.v[0];
+                pi[0] += a.v[1];
+            }
             const cd p0 = !kPlain || A.corr_pt ? A.bra[r0 + row] : cmk(0.0, 0.0);
             CV<Real, TPT> o;
 #pragma unroll
@@ -921,16 +1042,38 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 nn[t] += vr * vr + vi * vi;
                 cr[t] += p0.x * vr + p0.y * vi;   // conj(bra) * psi
                 ci[t] += p0.x * vi - p0.y * vr;
+                if (kTk) q4[t] += (vr * vr + vi * vi) * (vr * vr + vi * vi);
             }
-            if (kPlain) stv<Real, TPT>(prev, loc(row), o);   // its norm is not known yet
+            if (kPlain || kTk) stv<Real, TPT>(prev, loc(row), o);   // its norm is not known yet
             else stv<Real, TPT>(slab(1), x, o);
         }
     // ex[0] still holds ||H q_{m+1}||, which slower CTAs may be reading
     sum.sync();
     sum.template part<true>(0, cr, ci);
-    sum.template part<false>(1, nn, nn);
+    sum.template part<kTk>(1, nn, q4);
     sum.sync();
-    if constexpr (kPlain) {
+    if constexpr (kTk) {
+        if (act) {
+            const double inv = 1.0 / sqrt(sum.get(1, tl).x);
+            for (int k = rl; k < nbk; k += RL) {
+                const CV<Real, TPT> v = ldv<Real, TPT, false>(prev, loc(k));
+                A.psi_out[glo(k)] = cmk(v.v[0] * inv, v.v[1] * inv);
+            }
+        }
+        if (rank == 0 && threadIdx.x < TC && c0 + (int)threadIdx.x < B) {
+            const int t = threadIdx.x, b = c0 + t;
+            const double2 n2 = sum.get(1, t), c = sum.get(0, t);
+            const double nrm = sqrt(n2.x), inv = 1.0 / nrm;
+            if (!(nrm > 0.0) || !isfinite(nrm)) atomicCAS(A.S.status, 0, DQ_ERR_NAN);
+            // taylorKrylovClass.cu:417-434: the B part's estimate plus |1 - norm|
+            double est = A.tk_obs[b] + fabs(1.0 - nrm);
+            if (est < 1.110223e-16) est = 1.110223e-16;
+            A.erracc[b] += est;
+            A.tk_obs[b] = c.x * inv;
+            A.tk_obs[B + b] = c.y * inv;
+            A.tk_obs[2 * B + b] = n2.y * (inv * inv) * (inv * inv);
+        }
+    } else if constexpr (kPlain) {
         const double n2 = sum.get(1, 0).x, nrm = sqrt(n2), inv = 1. / nrm;
         for (int k = rl; k < nbk; k += RL)
             for (int row = k * R; row < min(nrow, k * R + R); ++row) {
@@ -1228,10 +1371,10 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
 }
 
 cudaError_t plain_cluster_attributes() {
-    cudaError_t e = raise_smem_limit(k_cluster_step<double, 1, 1, true, true>, (int)kClSmemMax);
-    if (e == cudaSuccess) e = raise_smem_limit(k_cluster_step<double, 1, 1, false, true>, (int)kClSmemMax);
+    cudaError_t e = raise_smem_limit(k_cluster_step<double, 1, 1, true, kDropIn>, (int)kClSmemMax);
+    if (e == cudaSuccess) e = raise_smem_limit(k_cluster_step<double, 1, 1, false, kDropIn>, (int)kClSmemMax);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_cluster_step<double, 1, 1, false, true>,
+        e = cudaFuncSetAttribute(k_cluster_step<double, 1, 1, false, kDropIn>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
@@ -1279,8 +1422,113 @@ cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cuda
     a.scratch = q.scratch;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cl_config(1, P.ctas, P.smem, st, &at);
-    return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, true>
-                                                : k_cluster_step<double, 1, 1, false, true>, a);
+    return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, kDropIn>
+                                                : k_cluster_step<double, 1, 1, false, kDropIn>, a);
+}
+
+// ---- Taylor-Krylov steps of an ensemble --------------------------------------
+// CTAs and trajectories of a cluster for n sites x B trajectories, z couplings
+// per row of the larger matrix and bandwidth bw, by cluster_plan's estimate;
+// ctas = 0: nothing fits.
+TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z) {
+    TaylorCluster best;
+    double t_best = 1e30;
+    ClKernel local = k_cluster_step<double, 1, 1, true, kTaylor>, wide = k_cluster_step<double, 1, 1, false, kTaylor>;
+    if (raise_smem_limit(local, (int)kClSmemMax) != cudaSuccess || raise_smem_limit(wide, (int)kClSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(wide, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return best;
+    }
+    for (int CS = 1; CS <= kClMaxCtas; ++CS) {
+        const int rpc = cl_rows(n, CS, 1);
+        if (CS > 1 && (size_t)rpc * (CS - 1) >= (size_t)n) continue;
+        int fit = 0;   // one CTA per SM whatever its shared memory: resident clusters depend on CS alone
+        for (int tc = 1; tc <= 32 && tc < 2 * B; tc *= 2) {
+            const size_t fixed = cl_layout(n, CS, tc, mb, rpc, bw, sizeof(double), 0, true).total;
+            if (fixed + 4096 > kClSmemMax) continue;
+            const size_t room = (kClSmemMax - fixed) / 16 * 16 - 16;
+            const bool in_smem = rpc * (z * 1.15 + 2.0) * 12.0 <= (double)room;
+            const int chunks = (B + tc - 1) / tc;
+            const double cycles = 5500.0 + 60.0 * CS +
+                                  1.6 * (rpc * z * tc * 16.0 / 128.0 * 1.3 + rpc * z * (in_smem ? 0.125 : 1.6)) +
+                                  0.8 * rpc * tc;
+            if (cycles >= t_best) continue;
+            if (!fit) {
+                cudaLaunchAttribute at;
+                const cudaLaunchConfig_t cfg = cl_config(1, CS, kClSmemMax, nullptr, &at);
+                if (cudaOccupancyMaxActiveClusters(&fit, CS == 1 ? local : wide, &cfg) != cudaSuccess || fit < 1) {
+                    cudaGetLastError();
+                    fit = -1;
+                }
+            }
+            if (fit < 1) continue;
+            const double t = cycles * ((chunks + fit - 1) / fit);
+            if (t < t_best) {
+                t_best = t;
+                best.ctas = CS;
+                best.tc = tc;
+                best.rpc = rpc;
+                best.chunks = chunks;
+                best.smem = fixed + room;
+                best.rec = room;
+            }
+        }
+    }
+    return best;
+}
+
+cudaError_t taylor_cluster_launch(const TaylorCluster& P, const TaylorStep& q, cudaStream_t st) {
+    ClusterArgs a = {};
+    a.n = q.n;
+    a.B = q.B;
+    a.TC = P.tc;
+    a.rpc = P.rpc;
+    a.bw = q.bw;
+    a.m = q.mb;
+    a.flags = kClFinish | kClNoise;
+    a.bil = q.dot_mode == DQ_DOT_BILINEAR;
+    a.chunks = P.chunks;
+    a.rec_smem = (int)P.rec;
+    a.bptr = q.rowptr;
+    a.bcol = q.col;
+    a.bcoef = q.val;
+    a.slabs = q.Q;
+    a.slab = (size_t)q.n * q.B;
+    a.diag = q.diag;
+    a.S.status = q.status;
+    a.S.yt = q.yt;
+    a.noise = q.noise;
+    a.ns = q.ns;
+    a.traj0 = q.traj0;
+    a.step = q.step;
+    a.subdt = q.subdt;
+    a.sqrt_subdt = sqrt(q.subdt);
+    a.seed = q.seed;
+    a.sigma = q.sigma;
+    a.invtau = q.invtau;
+    a.coeff = q.coeff;
+    a.eps = q.eps;
+    a.deps = q.deps;
+    if (q.noise == DQ_NOISE_ZZ) a.flags = kClFinish;   // the diagonal is drawn by a launch of its own
+    a.norm_mode = q.norm_mode;
+    a.tau_im = q.tau_im;
+    a.erracc = q.erracc;
+    a.bra = q.bra;
+    a.psi_in = q.psi;
+    a.psi_out = q.psi;
+    a.tk_p = q.p;
+    a.b_ptr = q.b_rowptr;
+    a.b_col = q.b_col;
+    a.b_val = q.b_val;
+    a.b_diag = q.b_diag;
+    for (int k = 0; k < q.p; ++k) a.tk_coef[k] = q.coef[k];
+    a.tk_obs = q.obs;
+    a.scratch = q.scratch;
+    a.scratch_stride = pade_smem_bytes(q.mb + q.p);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = cl_config(P.chunks, P.ctas, P.smem, st, &at);
+    return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, kTaylor>
+                                                : k_cluster_step<double, 1, 1, false, kTaylor>, a);
 }
 
 }  // namespace dq

@@ -70,6 +70,37 @@ struct PlainStep {
     unsigned char* scratch;  // pade_smem_bytes(m + 2)
 };
 
+// A Taylor-Krylov step of an ensemble as one cluster launch: CTAs (0: nothing
+// fits) and trajectories per cluster, rows per CTA, chunks, shared memory.
+struct TaylorCluster {
+    int ctas = 0, tc = 0, rpc = 0, chunks = 0;
+    size_t smem = 0, rec = 0;
+};
+
+struct TaylorStep {
+    int n, B, mb, p, bw, dot_mode, norm_mode;
+    const int *rowptr, *col;         // the Hamiltonian's off-diagonal CSR
+    const double* val;
+    const int *b_rowptr, *b_col;     // the auxiliary matrix's, and its diagonal
+    const double *b_val, *b_diag;
+    const cd* coef;                  // tau^k / k!, k < p (host)
+    double* diag;                    // [site][trajectory]: written (ZZ noise: read)
+    cd* psi;                         // [site][trajectory], replaced by the normalised next states
+    cd* Q;                           // mb + 2 slabs
+    double* yt;                      // kMaxL x B complex
+    int* status;
+    double* obs;                     // [3][B]: <bra|psi> and sum |psi|^4 of every trajectory
+    double tau_im;
+    int noise, ns, traj0, step;
+    double subdt;
+    uint64_t seed;
+    const double *sigma, *invtau, *coeff, *eps;
+    double* deps;
+    double* erracc;
+    const cd* bra;
+    unsigned char* scratch;          // chunks x pade_smem_bytes(mb + p)
+};
+
 struct BatchedState;   // dq_batched.cu
 struct TkEnsemble;     // dq_tk_ensemble.cu
 struct AdjointState;   // dq_adjoint.cu
@@ -144,6 +175,7 @@ struct dq_ctx {
     // Taylor-Krylov mode (tk_p > 0): the auxiliary matrix B (off-diagonal
     // CSR + diagonal), its Krylov basis and the Taylor work vectors
     int tk_p = 0, tk_m = 0;
+    int tk_bw = 0, tk_nnz = 0;    // B's bandwidth and off-diagonal entries
     int* d_tk_rowptr = nullptr;
     int* d_tk_col = nullptr;
     double* d_tk_val = nullptr;
@@ -209,6 +241,8 @@ dq_status read_status(dq_ctx* c, int code, const char* what);
 // implemented in dq_cluster.cu
 PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
 cudaError_t plain_cluster_attributes();
+TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z);
+cudaError_t taylor_cluster_launch(const TaylorCluster& P, const TaylorStep& q, cudaStream_t st);
 cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cudaStream_t st);
 // implemented in dq_batched.cu
 // default_tiling = false leaves the tiling unset (TC = 0) for a caller that

@@ -48,6 +48,12 @@ struct TkEnsemble {
     double* scal_mem = nullptr;
     TkScal s{};
     int mb_alloc = 0;
+    // the one-launch form (ctas = 0: the launches below), its trajectories' observables, the
+    // dense exponential's matrices
+    TaylorCluster cluster;
+    int for_p = 0, for_m = 0, for_bw = 0, for_nnz = 0;   // what it was planned for
+    double* obs = nullptr;
+    unsigned char* pade = nullptr;
 };
 
 // ---- per-trajectory reduction over row groups ------------------------------
@@ -349,6 +355,25 @@ __global__ void k_tke_pops(int n, int B, const cd* __restrict__ psi, double* __r
     }
 }
 
+// corr[step+1] += sum_b <psi0|psi_b>, ipr[step+1] += sum_b 1 / sum |psi_b|^4 from the trajectories' values
+__global__ void k_tke_totals(int B, const double* __restrict__ obs, cd* corr_pt, double* ipr_pt) {
+    __shared__ double scratch[32];
+    double cr = 0.0, ci = 0.0, ip = 0.0;
+    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+        cr += obs[b];
+        ci += obs[B + b];
+        ip += 1.0 / obs[2 * B + b];
+    }
+    cr = block_sum(cr, scratch);
+    ci = block_sum(ci, scratch);
+    ip = block_sum(ip, scratch);
+    if (threadIdx.x == 0) {
+        corr_pt->x += cr;
+        corr_pt->y += ci;
+        if (ipr_pt) *ipr_pt += ip;
+    }
+}
+
 __global__ void k_tke_set_psi0(int n, int B, const cd* __restrict__ psi0, cd* __restrict__ psi) {
     const size_t total = (size_t)n * B;
     for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < total; x += (size_t)gridDim.x * blockDim.x)
@@ -386,6 +411,7 @@ void tk_ensemble_free(dq_ctx* c) {
     TkEnsemble* t = c->tke;
     if (!t) return;
     cudaFree(t->eps); cudaFree(t->deps); cudaFree(t->diag); cudaFree(t->psi); cudaFree(t->Q); cudaFree(t->x2);
+    cudaFree(t->obs); cudaFree(t->pade);
     cudaFree(t->acc); cudaFree(t->w); cudaFree(t->scal_mem); cudaFree(t->s.ticket); cudaFree(t->s.status);
     delete t;
     c->tke = nullptr;
@@ -430,6 +456,27 @@ static dq_status tk_ensemble_alloc(dq_ctx* c) {
     return DQ_OK;
 }
 
+// The one-launch form's shape for the matrices that are set, with its scratch.
+static dq_status tk_plan(dq_ctx* c) {
+    TkEnsemble* t = c->tke;
+    const int bw = std::max(c->bw, c->tk_bw), nnz = std::max(c->nnz_off, c->tk_nnz);
+    if (t->for_p == c->tk_p && t->for_m == c->tk_m && t->for_bw == bw && t->for_nnz == nnz) return DQ_OK;
+    t->cluster = TaylorCluster();
+    cudaFree(t->pade);
+    t->pade = nullptr;
+    TaylorCluster P = taylor_cluster_plan(c->n, t->B, c->tk_m, bw, (double)nnz / c->n);
+    if (P.ctas) {
+        if (!t->obs) DQ_CU(cudaMalloc(&t->obs, sizeof(double) * 3 * (size_t)t->B));
+        DQ_CU(cudaMalloc(&t->pade, (size_t)P.chunks * pade_smem_bytes(c->tk_m + c->tk_p)));
+    }
+    t->cluster = P;
+    t->for_p = c->tk_p;
+    t->for_m = c->tk_m;
+    t->for_bw = bw;
+    t->for_nnz = nnz;
+    return DQ_OK;
+}
+
 // Draws every trajectory's static energies, OU offsets and ZZ phases, sets
 // every state to psi0 and adds the initial observable records (allocates the
 // workspace on first use).
@@ -438,6 +485,7 @@ dq_status tk_ensemble_reset(dq_ctx* c) {
     if (c->tke && (c->tke->B != c->cfg.n_traj || c->tke->mb_alloc < c->tk_m)) tk_ensemble_free(c);
     if (!c->tke && (st = tk_ensemble_alloc(c))) return st;
     TkEnsemble* t = c->tke;
+    if ((st = tk_plan(c))) return st;
     const int n = c->n, B = t->B;
     const int blocks = std::min(n, 148 * 8);
     const int thr = std::min(256, ((B + 31) / 32) * 32);
@@ -470,9 +518,57 @@ dq_status tk_ensemble_run(dq_ctx* c, int n_steps) {
     const bool bil = c->cfg.dot_mode == DQ_DOT_BILINEAR;
     for (int k = 0; k < n_steps; ++k) {
         const int step = c->steps_done + k;
-        k_tke_noise<<<grid, kTkThreads, 0, st>>>(n, B, c->traj0, step, c->cfg.noise_model, ns, subdt, sqrt_subdt,
-                                                 c->cfg.seed, c->d_sigma, c->d_invtau, c->d_coeff, zz, t->eps,
-                                                 t->deps, t->diag);
+        const bool one = t->cluster.ctas > 0;
+        if (!one || c->cfg.noise_model == DQ_NOISE_ZZ)
+            k_tke_noise<<<grid, kTkThreads, 0, st>>>(n, B, c->traj0, step, c->cfg.noise_model, ns, subdt, sqrt_subdt,
+                                                     c->cfg.seed, c->d_sigma, c->d_invtau, c->d_coeff, zz, t->eps,
+                                                     t->deps, t->diag);
+        if (one) {
+            TaylorStep q;
+            q.n = n;
+            q.B = B;
+            q.mb = mb;
+            q.p = p;
+            q.bw = std::max(c->bw, c->tk_bw);
+            q.dot_mode = c->cfg.dot_mode;
+            q.norm_mode = c->cfg.norm_mode;
+            q.rowptr = c->d_rowptr;
+            q.col = c->d_col;
+            q.val = c->d_val;
+            q.b_rowptr = c->d_tk_rowptr;
+            q.b_col = c->d_tk_col;
+            q.b_val = c->d_tk_val;
+            q.b_diag = c->d_tk_diag;
+            q.coef = c->tk_coef.data();
+            q.diag = t->diag;
+            q.psi = t->psi;
+            q.Q = t->Q;
+            q.yt = reinterpret_cast<double*>(t->s.yt);
+            q.status = t->s.status;
+            q.obs = t->obs;
+            q.tau_im = c->tau_im;
+            q.noise = c->cfg.noise_model;
+            q.ns = ns;
+            q.traj0 = c->traj0;
+            q.step = step;
+            q.subdt = subdt;
+            q.seed = c->cfg.seed;
+            q.sigma = c->d_sigma;
+            q.invtau = c->d_invtau;
+            q.coeff = c->d_coeff;
+            q.eps = t->eps;
+            q.deps = t->deps;
+            q.erracc = c->d_erracc;
+            q.bra = corr_bra(c);
+            q.scratch = t->pade;
+            DQ_CU(taylor_cluster_launch(t->cluster, q, st));
+            k_tke_totals<<<1, 256, 0, st>>>(B, t->obs, c->d_corr + step + 1, c->ipr_on ? c->d_ipr + step + 1 : nullptr);
+            if ((step + 1) % pe == 0)
+                k_tke_pops<<<std::max(1, std::min(148 * 4, (n + 7) / 8)), 256, 0, st>>>(
+                    n, B, t->psi, c->d_pops + (size_t)((step + 1) / pe) * n);
+            DQ_CU(cudaGetLastError());
+            continue;
+        }
         const cd* x = t->psi;
         for (int kk = 1; kk <= p; ++kk) {
             cd* y = (kk == p) ? t->Q + se : t->x2 + (size_t)(kk & 1) * se;

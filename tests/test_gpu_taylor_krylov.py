@@ -166,3 +166,33 @@ def test_taylor_krylov_with_zz_noise(oracle):
     prop.run_plain(T)
     assert np.abs(prop.populations() - ref["pops"]).max() <= TOL_FP64
     prop.close()
+
+
+# sizes around the one-launch form's shapes (one CTA, several, ragged chunks) and past it, against the
+# per-trajectory path on the same draws
+@pytest.mark.parametrize("around,along,B,p_tk,m_b,dot", [(3, 4, 1, 2, 1, 1), (10, 6, 3, 4, 10, 0), (12, 11, 7, 3, 8, 1),
+                                                         (23, 31, 33, 5, 12, 1), (40, 60, 20, 2, 6, 1)])
+@pytest.mark.parametrize("noise", [0, 2])
+def test_ensemble_sizes_match_per_trajectory_path(around, along, B, p_tk, m_b, dot, noise):
+    import dynaquant_b200 as dq
+    from dynaquant_b200 import systems
+    s = systems.tube(around, along)
+    rng = np.random.default_rng(around)
+    val = s.val.copy()
+    rows = np.repeat(np.arange(s.n), np.diff(s.rowptr))
+    val[rows == s.col] = rng.normal(0.0, 60.0, s.n)
+    got = []
+    for run in ("run", "run_plain"):
+        prop = dq.Propagator(s.n, m=min(12, s.n), n_traj=B, dt=1.0, noise=noise, seed=13, dot=dot, pop_every=2,
+                             max_steps=5, sigma_static=70.0, precision=dq.PREC_FP64)
+        prop.set_system(s)
+        prop.set_noise_params(np.full(s.n, 120.0), np.full(s.n, 60.0))
+        prop.set_initial_state(s.bright_state())
+        prop.set_taylor_krylov(p_tk, m_b, s.rowptr, s.col, val)
+        prop.set_ipr(True)
+        getattr(prop, run)(5)
+        got.append((prop.populations(), prop.correlation(), prop.ipr(), prop.error_accum()))
+        prop.close()
+    for a, b in zip(got[0][:3], got[1][:3]):
+        assert np.abs(a - b).max() < TOL_FP64 * max(1.0, np.abs(b).max())
+    assert np.allclose(got[0][3], got[1][3], rtol=1e-6, atol=1e-14)
