@@ -3903,7 +3903,19 @@ dq_status batched_default_tiling(dq_ctx* c) {
     int tc = 16;
     while (tc > tpt && B % tc) tc >>= 1;
     if (B % tc) tc = tpt;
-    dq_status st = batched_set_tiling(c, tc, tpt, 2, 4, 0, 1);
+    // Grid-wide, by what the gathers share.  Step times on a B200, m = 16, the former choice (form 0, four
+    // rows a block) and this one: rows of few couplings (chain of 20,000 x 128) stay with four rows, 0.62
+    // ms; complex64, 30,000 sites with 28 couplings: x 256 4.05 -> 2.42 ms (form 12, whole chunks of 16 and
+    // work for its one 1024-thread CTA per SM), x 24 0.67 -> 0.51, x 100 2.26 -> 1.87 (three rows, packed
+    // records); 12,000 x 64, 0.64 -> 0.50; FP64 30,000 x 64, 2.74 -> 1.90 (two rows, 512-thread CTAs)
+    const bool few = c->nnz_off < 6 * (size_t)c->n;
+    dq_status st;
+    if (few) st = batched_set_tiling(c, tc, tpt, 2, 4, 0, 1);
+    else if (!bs->mixed) st = batched_set_tiling(c, tc, tpt, tc == 16 ? 1 : 2, 2, 5, 1);
+    else if (tc == 16 && (double)c->n * B > 2e6 && c->nnz_off >= 16 * (size_t)c->n)
+        st = batched_set_tiling(c, tc, tpt, 1, 3, 12, 1);
+    else st = batched_set_tiling(c, tc, tpt, 2, 3, 0, 1);
+    if (st) st = batched_set_tiling(c, tc, tpt, 2, 4, 0, 1);
     if (st) {
         c->err = "batched: no valid tiling for n_traj";
         return st;
