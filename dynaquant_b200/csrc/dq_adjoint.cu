@@ -58,6 +58,9 @@ struct BasisLane {
     __device__ __forceinline__ size_t at(int row) const { return base + (size_t)row * stride; }
 };
 
+// complex coefficients per trajectory that k_adj_small leaves for k_adj_sweep
+__host__ __device__ inline int sweep_coefs(int m) { return m * m + 3 * m + 1; }
+
 template <typename Real> struct R2;
 template <> struct R2<float> { using T = float2; };
 template <> struct R2<double> { using T = double2; };
@@ -172,13 +175,11 @@ __global__ void k_lambda_init_norm(int n, int B, const cd* __restrict__ psi0, co
     }
 }
 
-// One CTA per trajectory: the block-triangular exponential and the
-// coefficient sets of the gradient kernel,
-//   M[a][b]  = tau |lam| scW_a N_ab scV_b                  (a, b = 1..m)
-//   P[a][c]  = sum_b M'_ab K_bc, H q^V_b = sum_c K_bc r^V_c (c = 1..m+1)
+// One CTA per trajectory: the block-triangular exponential and what the sweep
+// kernel needs of it,
+//   M[a][b]  = tau |lam| scW_a N_ab                        (a, b = 1..m)
 //   yw[a]    = |lam| conj(E_a0) scW_a
-// with M'_ab = tau |lam| scW_a N_ab and K from beta_b q_{b+1} = H q_b -
-// alpha_b q_b - beta_{b-1} q_{b-1} (complex alpha), q_c = sc_c r_c.
+//   (scV_c, beta_c), c = 1..m+1, and alpha_c, c = 1..m, of the kept step.
 //
 // N and E e_0 come from the two Krylov sequences of e_1 alone: with w_k =
 // (tau T_W)^k e_1 / k! and v_l likewise (one warp each, the neighbour products
@@ -291,61 +292,54 @@ __global__ void __launch_bounds__(256) k_adj_small(int m, int B, double tau_im, 
         }
     }
     const double ln = sqrt(SW.norm2[b]);
-    const int CS = m * (2 * m + 2);
-    T2* out = coef + (size_t)b * CS;
-    // M'(a, bb), 1-based
-    auto mp = [&](int a, int bb) -> cd {
-        const cd nab = E[(a - 1) * L + m + (bb - 1)];
-        return cmul(cmk(0.0, tau_im * ln * scW[a]), nab);
+    T2* out = coef + (size_t)b * sweep_coefs(m);
+    auto put = [&](int e, double x, double y) {
+        T2 o;
+        o.x = (Real)x;
+        o.y = (Real)y;
+        out[e] = o;
     };
     for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int a = e / m + 1, bb = e % m + 1;
-        const cd v = cscale(mp(a, bb), scV[bb]);
-        T2 o;
-        o.x = (Real)v.x;
-        o.y = (Real)v.y;
-        out[e] = o;
-    }
-    for (int e = threadIdx.x; e < m * (m + 1); e += blockDim.x) {
-        const int a = e / (m + 1) + 1, cc = e % (m + 1) + 1;
-        cd p = cmk(0.0, 0.0);
-        // H q_{c-1} holds r_c with weight beta_{c-1} sc_c (1 when the slab keeps
-        // the unnormalised residual, beta_{c-1} when it keeps q_c itself)
-        if (cc - 1 >= 1) p = cadd(p, cscale(mp(a, cc - 1), beV[cc - 1] * scV[cc]));
-        if (cc <= m) p = cadd(p, cmul(mp(a, cc), cmk(alV[cc] * scV[cc], aiV[cc] * scV[cc])));
-        if (cc + 1 <= m) p = cadd(p, cscale(mp(a, cc + 1), beV[cc] * scV[cc]));
-        T2 o;
-        o.x = (Real)p.x;
-        o.y = (Real)p.y;
-        out[m * m + e] = o;
+        const int a = e / m, bb = e % m;
+        const cd v = cmul(cmk(0.0, tau_im * ln * scW[a + 1]), E[a * L + m + bb]);
+        put(e, v.x, v.y);
     }
     for (int a = threadIdx.x; a < m; a += blockDim.x) {
-        const cd z = cconj(E[a * L]);
-        const cd v = cscale(z, ln * scW[a + 1]);
-        T2 o;
-        o.x = (Real)v.x;
-        o.y = (Real)v.y;
-        out[m * m + m * (m + 1) + a] = o;
+        const cd v = cscale(cconj(E[a * L]), ln * scW[a + 1]);
+        put(m * m + a, v.x, v.y);
     }
+    for (int c = threadIdx.x; c <= m; c += blockDim.x) put(m * m + m + c, scV[c + 1], c < m ? beV[c + 1] : 0.0);
+    for (int c = threadIdx.x; c < m; c += blockDim.x) put(m * m + 2 * m + 1 + c, alV[c + 1], aiV[c + 1]);
 }
 
-// Per (site, trajectory): the site and coupling forms of this step and the
-// new lambda (written over the lambda workspace's slab 1, which holds the
-// old one: each element is read by its own thread before it is replaced).
-// Sums over the CTA's trajectories go to gsite/gcpl[row][traj group] (one
+// One step of the backward sweep.  Per (site, trajectory), with
+//   t_b(i) = sum_a M_ab conj(rW_a(i))                        (b = 1..m)
+// the site form is Re sum_b t_b q_b(i) (q_b = scV_b rV_b), the whole coupling
+// form Re sum_c (beta_{c-1} t_{c-1} + alpha_c t_c + beta_c t_{c+1}) q_c(i),
+// c = 1..m+1, by the Lanczos relation H q_b = beta_b q_{b+1} + alpha_b q_b +
+// beta_{b-1} q_{b-1} (no extra SpMM), and with several coupling classes (C > 0)
+//   dL/dscale_c += sum_{p in c} vbase_p Re sum_b t_b(i) q_b(col_p)
+// gathers V at the neighbours of those classes (skip0: class 0 follows on the
+// host from the whole form).  The new lambda goes over the old one (slab 1 of
+// the lambda workspace: each element is read by its own thread first).
+// One pass over W and V: t is formed once, m^2 complex products a site, and a
+// thread takes NR rows so that a coefficient read from shared memory serves
+// them all (one coefficient per eight products kept the shared-memory pipe
+// busy).  64 x 64 lattice, 128 trajectories, m = 16, two classes: 333 us for
+// the two former kernels (m^2 products in one, 2 m^2 + m in the other), 216 us.
+// Sums over the CTA's trajectories go to gsite/gcpl/gcls[row][traj group] (one
 // writer each, deterministic); |lambda|^2 partials to lpart[cta][b].
-template <typename Real, int MM>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m, int tcv, int tcw, int rows_per_cta, int G,
-                                                         const Real* __restrict__ sV, Real* sW, size_t slab_reals,
-                                                         const Real* __restrict__ d, const cd* __restrict__ psi0,
-                                                         const cd* __restrict__ Gt, double invB, int write_lam,
-                                                         const typename R2<Real>::T* __restrict__ coef,
-                                                         double* __restrict__ lpart, double* __restrict__ gsite,
-                                                         double* __restrict__ gcpl) {
+template <typename Real, int MM, int NR>
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_sweep(
+    int n, int B, int m, int tcv, int tcw, int rows_per_cta, int G, int C, const Real* __restrict__ sV, Real* sW,
+    size_t slab_reals, const Real* __restrict__ d, const cd* __restrict__ psi0, const cd* __restrict__ Gt, double invB,
+    int write_lam, const int* __restrict__ rowptr, const int* __restrict__ col, const int* __restrict__ cls,
+    const double* __restrict__ vbase, const typename R2<Real>::T* __restrict__ coef, double* __restrict__ lpart,
+    double* __restrict__ gsite, double* __restrict__ gcpl, double* __restrict__ gcls, int skip0) {
     using T2 = typename R2<Real>::T;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T2* cs = reinterpret_cast<T2*>(sm_raw);
-    const int CS = m * (2 * m + 2);
+    const int CS = sweep_coefs(m);
     const int tl = threadIdx.x % kAdjTraj, rl = threadIdx.x / kAdjTraj;
     constexpr int kRowLanes = kAdjThreads / kAdjTraj;
     const int b = blockIdx.y * kAdjTraj + tl;
@@ -354,97 +348,208 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m
         cs[e] = coef[(size_t)(blockIdx.y * kAdjTraj + t) * CS + idx];
     }
     __syncthreads();
-    const T2* Mc = cs;
-    const T2* Pc = cs + (size_t)m * m * kAdjTraj;
-    const T2* Yc = Pc + (size_t)m * (m + 1) * kAdjTraj;
+    const T2* Mc = cs + tl;
+    const T2* Yc = Mc + (size_t)m * m * kAdjTraj;
+    const T2* Zc = Yc + (size_t)m * kAdjTraj;          // (scV, beta), m + 1
+    const T2* Ac = Zc + (size_t)(m + 1) * kAdjTraj;    // alpha, m
     const cd g = Gt[0];
     const double sr = g.x * invB, si = -g.y * invB;
     const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
     const BasisLane bv(n, B, tcv, b), bw(n, B, tcw, b);
     double lnn = 0.0;
-    // uniform trip count across the warp: the trajectory-lane shuffles below
-    // need every lane
-    for (int base = r0; base < r1; base += kRowLanes) {
-        const int row = base + rl;
-        const bool valid = row < r1;
-        const size_t x = (size_t)(valid ? row : r0) * B + b, xv = bv.at(valid ? row : r0),
-                     xw = bw.at(valid ? row : r0);
-        Real vr[MM + 1], vi[MM + 1];
+    // uniform trip count across the warp: the trajectory-lane shuffles below need every lane
+    for (int base = r0; base < r1; base += NR * kRowLanes) {
+        int row[NR];
+        bool valid[NR];
+        size_t x[NR], xw[NR], xv[NR];
+        Real tr[NR][MM], ti[NR][MM], lr[NR], li[NR];
 #pragma unroll
-        for (int c = 0; c <= MM; ++c) {
-            if (c <= m) {
-                const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * (c ? xv : x));
-                vr[c] = v.x;
-                vi[c] = v.y;
-            } else {
-                vr[c] = 0;
-                vi[c] = 0;
-            }
+        for (int q = 0; q < NR; ++q) {
+            const int r = base + q * kRowLanes + rl;
+            valid[q] = r < r1;
+            row[q] = valid[q] ? r : r0;
+            x[q] = (size_t)row[q] * B + b;
+            xw[q] = bw.at(row[q]);
+            xv[q] = bv.at(row[q]);
+            const cd p0 = psi0[row[q]];
+            lr[q] = (Real)(sr * p0.x - si * p0.y);
+            li[q] = (Real)(sr * p0.y + si * p0.x);
+#pragma unroll
+            for (int c = 0; c < MM; ++c) tr[q][c] = ti[q][c] = 0;
         }
-        Real site = 0, cpl = 0;
-        const cd p0 = psi0[valid ? row : r0];
-        Real lr = (Real)(sr * p0.x - si * p0.y), li = (Real)(sr * p0.y + si * p0.x);
-        // W column streamed four entries ahead (a register pipeline), so its
-        // loads overlap the products
-        auto ldw = [&](int a) {
+        auto ldw = [&](int a, int q) {
             T2 v;
-            if (a < m) v = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * (a ? xw : x));
+            if (a < m) v = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * (a ? xw[q] : x[q]));
             else { v.x = 0; v.y = 0; }
             return v;
         };
-        auto body = [&](int a, const T2& w) {
-            Real Xr = 0, Xi = 0, Yr = 0, Yi = 0;
+        // W streamed two entries ahead, so its loads overlap the products
+        T2 w0[NR], w1[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            w0[q] = ldw(0, q);
+            w1[q] = ldw(1, q);
+        }
+        for (int a = 0; a < m; ++a) {
+            T2 w2[NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) w2[q] = ldw(a + 2, q);
+            const T2 y = Yc[a * kAdjTraj];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                lr[q] = fma(y.x, w0[q].x, fma(-y.y, w0[q].y, lr[q]));
+                li[q] = fma(y.x, w0[q].y, fma(y.y, w0[q].x, li[q]));
+            }
 #pragma unroll
             for (int c = 0; c < MM; ++c) {
                 if (c < m) {
-                    const T2 M = Mc[(a * m + c) * kAdjTraj + tl];
-                    Xr = fma(M.x, vr[c], fma(-M.y, vi[c], Xr));
-                    Xi = fma(M.x, vi[c], fma(M.y, vr[c], Xi));
+                    const T2 M = Mc[(a * m + c) * kAdjTraj];
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) {
+                        tr[q][c] = fma(M.x, w0[q].x, fma(M.y, w0[q].y, tr[q][c]));    // M conj(w)
+                        ti[q][c] = fma(M.y, w0[q].x, fma(-M.x, w0[q].y, ti[q][c]));
+                    }
                 }
             }
 #pragma unroll
-            for (int c = 0; c <= MM; ++c) {
-                if (c <= m) {
-                    const T2 P = Pc[(a * (m + 1) + c) * kAdjTraj + tl];
-                    Yr = fma(P.x, vr[c], fma(-P.y, vi[c], Yr));
-                    Yi = fma(P.x, vi[c], fma(P.y, vr[c], Yi));
+            for (int q = 0; q < NR; ++q) {
+                w0[q] = w1[q];
+                w1[q] = w2[q];
+            }
+        }
+        // the forms: V at the own sites
+        Real site[NR], cpl[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) site[q] = cpl[q] = 0;
+#pragma unroll
+        for (int c = 0; c <= MM; ++c) {
+            if (c <= m) {
+                const T2 z = Zc[c * kAdjTraj];
+                const Real bm = c > 0 ? Zc[(c > 0 ? c - 1 : 0) * kAdjTraj].y : Real(0);
+                T2 al;
+                al.x = al.y = 0;
+                if (c < m) al = Ac[c * kAdjTraj];
+#pragma unroll
+                for (int q = 0; q < NR; ++q) {
+                    T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * (c ? xv[q] : x[q]));
+                    v.x *= z.x;
+                    v.y *= z.x;
+                    Real pr = 0, pi = 0;
+                    if (c > 0) {
+                        pr = bm * tr[q][c > 0 ? c - 1 : 0];
+                        pi = bm * ti[q][c > 0 ? c - 1 : 0];
+                    }
+                    if constexpr (MM > 0) {
+                        if (c < MM && c < m) {
+                            const Real ur = tr[q][c < MM ? c : 0], ui = ti[q][c < MM ? c : 0];
+                            site[q] = fma(ur, v.x, fma(-ui, v.y, site[q]));    // Re(t q)
+                            pr = fma(al.x, ur, fma(-al.y, ui, pr));
+                            pi = fma(al.x, ui, fma(al.y, ur, pi));
+                        }
+                        if (c + 1 < MM && c + 1 < m) {
+                            pr = fma(z.y, tr[q][c + 1 < MM ? c + 1 : 0], pr);
+                            pi = fma(z.y, ti[q][c + 1 < MM ? c + 1 : 0], pi);
+                        }
+                    }
+                    cpl[q] = fma(pr, v.x, fma(-pi, v.y, cpl[q]));
                 }
             }
-            site = fma(w.x, Xr, fma(w.y, Xi, site));
-            cpl = fma(w.x, Yr, fma(w.y, Yi, cpl));
-            const T2 y = Yc[a * kAdjTraj + tl];
-            lr = fma(y.x, w.x, fma(-y.y, w.y, lr));
-            li = fma(y.x, w.y, fma(y.y, w.x, li));
-        };
-        T2 w0 = ldw(0), w1 = ldw(1), w2 = ldw(2), w3 = ldw(3);
-        for (int a = 0; a < m; a += 4) {
-            const T2 n0 = ldw(a + 4), n1 = ldw(a + 5), n2 = ldw(a + 6), n3 = ldw(a + 7);
-            body(a, w0);
-            if (a + 1 < m) body(a + 1, w1);
-            if (a + 2 < m) body(a + 2, w2);
-            if (a + 3 < m) body(a + 3, w3);
-            w0 = n0;
-            w1 = n1;
-            w2 = n2;
-            w3 = n3;
-        }
-        double s_d = valid ? (double)site : 0.0;
-        double c_d = valid ? (double)cpl - (double)d[x] * (double)site : 0.0;
-        if (valid && write_lam) {
-            T2 o;
-            o.x = lr;
-            o.y = li;
-            *reinterpret_cast<T2*>(sW + slab_reals + 2 * x) = o;
-            lnn += (double)lr * lr + (double)li * li;
         }
 #pragma unroll
-        for (int o = 1; o < kAdjTraj; o <<= 1) {
-            s_d += __shfl_xor_sync(0xffffffffu, s_d, o);
-            c_d += __shfl_xor_sync(0xffffffffu, c_d, o);
+        for (int q = 0; q < NR; ++q) {
+            double s_d = valid[q] ? (double)site[q] : 0.0;
+            double c_d = valid[q] ? (double)cpl[q] - (double)d[x[q]] * (double)site[q] : 0.0;
+            if (valid[q] && write_lam) {
+                T2 o;
+                o.x = lr[q];
+                o.y = li[q];
+                *reinterpret_cast<T2*>(sW + slab_reals + 2 * x[q]) = o;
+                lnn += (double)lr[q] * lr[q] + (double)li[q] * li[q];
+            }
+#pragma unroll
+            for (int o = 1; o < kAdjTraj; o <<= 1) {
+                s_d += __shfl_xor_sync(0xffffffffu, s_d, o);
+                c_d += __shfl_xor_sync(0xffffffffu, c_d, o);
+            }
+            if (valid[q] && tl == 0) {
+                gsite[(size_t)row[q] * G + blockIdx.y] += s_d;
+                gcpl[(size_t)row[q] * G + blockIdx.y] += c_d;
+            }
         }
-        if (valid && tl == 0) {
-            gsite[(size_t)row * G + blockIdx.y] += s_d;
-            gcpl[(size_t)row * G + blockIdx.y] += c_d;
+        if (C > 0) {
+            // t_b scV_b, then the rows' couplings of the gathered classes in batches of KP: for each
+            // Krylov index the batch's gathers are independent loads
+#pragma unroll
+            for (int c = 0; c < MM; ++c) {
+                if (c < m) {
+                    const Real z = Zc[c * kAdjTraj].x;
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) {
+                        tr[q][c] *= z;
+                        ti[q][c] *= z;
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                double acc[kAdjMaxClasses];
+#pragma unroll
+                for (int k = 0; k < kAdjMaxClasses; ++k) acc[k] = 0.0;
+                if (valid[q]) {
+                    constexpr int KP = 4;
+                    const int pe = rowptr[row[q] + 1];
+                    int p = rowptr[row[q]];
+                    while (p < pe) {
+                        int xk[KP], qk[KP];
+                        double vk[KP];
+#pragma unroll
+                        for (int k = 0; k < KP; ++k) { xk[k] = row[q]; qk[k] = 0; vk[k] = 0.0; }
+                        int nk = 0;
+                        for (; p < pe && nk < KP; ++p) {
+                            const int cl = cls[p];
+                            if (skip0 && cl == 0) continue;
+                            const int xc = col[p];
+                            const double vv = vbase[p];
+#pragma unroll
+                            for (int k = 0; k < KP; ++k)   // register slots, no indexed local array
+                                if (k == nk) { xk[k] = xc; qk[k] = cl; vk[k] = vv; }
+                            ++nk;
+                        }
+                        if (nk == 0) break;   // the rest of the row is class 0
+                        Real rr[KP];
+                        size_t xg[KP];
+#pragma unroll
+                        for (int k = 0; k < KP; ++k) {
+                            rr[k] = 0;
+                            xg[k] = bv.at(xk[k]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < MM; ++c) {
+                            if (c < m) {
+#pragma unroll
+                                for (int k = 0; k < KP; ++k) {   // unused slots read the own row, weight 0
+                                    const size_t xs = c ? xg[k] : (size_t)xk[k] * B + b;
+                                    const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * xs);
+                                    rr[k] = fma(tr[q][c], v.x, fma(-ti[q][c], v.y, rr[k]));   // Re(t v)
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int k = 0; k < KP; ++k) {
+                            const double contrib = vk[k] * (double)rr[k];
+#pragma unroll
+                            for (int u = 0; u < kAdjMaxClasses; ++u) acc[u] += (u == qk[k]) ? contrib : 0.0;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kAdjMaxClasses; ++u) {
+                    if (u >= C) break;   // uniform
+#pragma unroll
+                    for (int o = 1; o < kAdjTraj; o <<= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+                    if (valid[q] && tl == 0) gcls[((size_t)row[q] * G + blockIdx.y) * C + u] += acc[u];
+                }
+            }
         }
     }
     __shared__ double red[kAdjThreads];
@@ -454,115 +559,6 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_grad(int n, int B, int m
         double s = 0.0;
         for (int r = 0; r < kRowLanes; ++r) s += red[r * kAdjTraj + tl];
         lpart[(size_t)blockIdx.x * B + b] = s;
-    }
-}
-
-// Coupling-class gradients when there are several classes:
-//   dL/dscale_c += sum_{p in c} vbase_p Re sum_b t_b(i) rV_b(col_p),
-//   t_b(i) = sum_a M_ab conj(rW_a(i)),
-// gathering the V basis at every neighbour column (m loads per entry).  With
-// skip0, class-0 entries are left out: their sum follows on the host from the
-// total off-diagonal form (free from the Lanczos relation in k_adj_grad).
-template <typename Real, int MM>
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_cls(int n, int B, int m, int tcv, int tcw, int rows_per_cta, int G, int C,
-                                                        const Real* __restrict__ sV, const Real* __restrict__ sW,
-                                                        size_t slab_reals, const int* __restrict__ rowptr,
-                                                        const int* __restrict__ col, const int* __restrict__ cls,
-                                                        const double* __restrict__ vbase,
-                                                        const typename R2<Real>::T* __restrict__ coef,
-                                                        double* __restrict__ gcls, int skip0) {
-    using T2 = typename R2<Real>::T;
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    T2* Mc = reinterpret_cast<T2*>(sm_raw);
-    const int CS = m * (2 * m + 2);
-    const int tl = threadIdx.x % kAdjTraj, rl = threadIdx.x / kAdjTraj;
-    constexpr int kRowLanes = kAdjThreads / kAdjTraj;
-    const int b = blockIdx.y * kAdjTraj + tl;
-    for (int e = threadIdx.x; e < m * m * kAdjTraj; e += blockDim.x) {
-        const int t = e % kAdjTraj, idx = e / kAdjTraj;
-        Mc[e] = coef[(size_t)(blockIdx.y * kAdjTraj + t) * CS + idx];
-    }
-    __syncthreads();
-    const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
-    const BasisLane bv(n, B, tcv, b), bw(n, B, tcw, b);
-    for (int base = r0; base < r1; base += kRowLanes) {
-        const int row = base + rl;
-        const bool valid = row < r1;
-        const int own = valid ? row : r0;
-        const size_t x = (size_t)own * B + b, xw = bw.at(own);
-        Real tr[MM], ti[MM];
-#pragma unroll
-        for (int c = 0; c < MM; ++c) { tr[c] = 0; ti[c] = 0; }
-        for (int a = 0; a < m; ++a) {
-            const T2 w = *reinterpret_cast<const T2*>(sW + (size_t)(a + 1) * slab_reals + 2 * (a ? xw : x));
-#pragma unroll
-            for (int c = 0; c < MM; ++c) {
-                if (c < m) {
-                    const T2 M = Mc[(a * m + c) * kAdjTraj + tl];
-                    tr[c] = fma(M.x, w.x, fma(M.y, w.y, tr[c]));    // M conj(w)
-                    ti[c] = fma(M.y, w.x, fma(-M.x, w.y, ti[c]));
-                }
-            }
-        }
-        double acc[kAdjMaxClasses];
-#pragma unroll
-        for (int q = 0; q < kAdjMaxClasses; ++q) acc[q] = 0.0;
-        if (valid) {
-            // the row's couplings (of the gathered classes) in batches of KP:
-            // for each Krylov index the batch's gathers are independent loads,
-            // so a batch keeps up to KP x m loads in flight instead of a chain
-            // per entry (KP = 8 against 4 and 2: 179 vs 203 and 204 us per
-            // launch on the 64 x 64 lattice, 232 us one entry at a time)
-            constexpr int KP = 8;
-            const int pe = rowptr[row + 1];
-            int p = rowptr[row];
-            while (p < pe) {
-                int xk[KP];
-                int qk[KP];
-                double vk[KP];
-#pragma unroll
-                for (int k = 0; k < KP; ++k) { xk[k] = own; qk[k] = 0; vk[k] = 0.0; }
-                int nk = 0;
-                for (; p < pe && nk < KP; ++p) {
-                    const int q = cls[p];
-                    if (skip0 && q == 0) continue;
-                    const int xv = col[p];
-                    const double vv = vbase[p];
-#pragma unroll
-                    for (int k = 0; k < KP; ++k)   // register slots, no indexed local array
-                        if (k == nk) { xk[k] = xv; qk[k] = q; vk[k] = vv; }
-                    ++nk;
-                }
-                if (nk == 0) break;   // the rest of the row is class 0
-                Real rr[KP];
-#pragma unroll
-                for (int k = 0; k < KP; ++k) rr[k] = 0;
-#pragma unroll
-                for (int c = 0; c < MM; ++c) {
-                    if (c < m) {
-#pragma unroll
-                        for (int k = 0; k < KP; ++k) {   // unused slots read the own row, weight 0
-                            const size_t xv = c ? bv.at(xk[k]) : (size_t)xk[k] * B + b;
-                            const T2 v = *reinterpret_cast<const T2*>(sV + (size_t)c * slab_reals + 2 * xv);
-                            rr[k] = fma(tr[c], v.x, fma(-ti[c], v.y, rr[k]));   // Re(t v)
-                        }
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < KP; ++k) {
-                    const double contrib = vk[k] * (double)rr[k];
-#pragma unroll
-                    for (int q = 0; q < kAdjMaxClasses; ++q) acc[q] += (q == qk[k]) ? contrib : 0.0;
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < kAdjMaxClasses; ++q) {
-#pragma unroll
-            for (int o = 1; o < kAdjTraj; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-        }
-        if (valid && tl == 0)
-            for (int q = 0; q < C; ++q) gcls[((size_t)row * G + blockIdx.y) * C + q] += acc[q];
     }
 }
 
@@ -642,11 +638,13 @@ static size_t adj_small_smem(int m) {
 
 static int mm_bucket(int m) { return m <= 8 ? 8 : m <= 16 ? 16 : 24; }
 
+// rows per thread of the sweep: two while their Krylov coefficients fit the registers
+template <typename Real, int MM>
+constexpr int sweep_rows() { return sizeof(Real) == 4 && MM <= 16 ? 2 : 1; }
+
 template <typename Real, int MM>
 static cudaError_t grad_attr(int bytes) {
-    cudaError_t e = raise_smem_limit(k_adj_grad<Real, MM>, bytes);
-    if (e != cudaSuccess) return e;
-    return raise_smem_limit(k_adj_cls<Real, MM>, bytes);
+    return raise_smem_limit(k_adj_sweep<Real, MM, sweep_rows<Real, MM>()>, bytes);
 }
 
 // Makes set k (segment s uses set s % 2) the one seg_V / seg_sc / seg_diag
@@ -665,54 +663,31 @@ static unsigned char* slot_V(AdjointState* a, int m, int slot) {
 }
 
 template <typename Real>
-static void launch_grad(dq_ctx* c, AdjointState* a, int t, int slot, int write_lam) {
+static void launch_sweep(dq_ctx* c, AdjointState* a, int t, int slot, int write_lam) {
     BatchedState* bs = c->bat;
     const int n = c->n, B = bs->B, m = c->cfg.m, G = B / kAdjTraj;
     const size_t slab_reals = (size_t)n * B * 2;
-    const int CS = m * (2 * m + 2);
-    const size_t smem = (size_t)CS * kAdjTraj * sizeof(typename R2<Real>::T);
-    const dim3 grid(a->row_ctas, G);
     using T2 = typename R2<Real>::T;
-#define DQ_GRAD(MMV)                                                                                               \
-    k_adj_grad<Real, MMV><<<grid, kAdjThreads, smem, c->stream>>>(                                                  \
-        n, B, m, a->seg_tc, batched_basis_chunk(a->ws2), a->rows_per_cta, G, (const Real*)slot_V(a, m, slot), (Real*)a->ws2->slabs, slab_reals,          \
-        (const Real*)(a->seg_diag + (size_t)slot * a->diag_bytes),                                                 \
-        c->d_psi0, a->d_G + t, a->inv_norm, write_lam, (const T2*)a->d_coef, a->d_lpart, a->d_gsite, a->d_gcpl)
-    switch (mm_bucket(m)) {
-        case 8: DQ_GRAD(8); break;
-        case 16: DQ_GRAD(16); break;
-        default: DQ_GRAD(24); break;
-    }
-#undef DQ_GRAD
-}
-
-template <typename Real>
-static void launch_cls(dq_ctx* c, AdjointState* a, int slot) {
-    BatchedState* bs = c->bat;
-    const int n = c->n, B = bs->B, m = c->cfg.m, G = B / kAdjTraj;
-    const size_t slab_reals = (size_t)n * B * 2;
-    const size_t smem = (size_t)m * m * kAdjTraj * sizeof(typename R2<Real>::T);
+    const size_t smem = (size_t)sweep_coefs(m) * kAdjTraj * sizeof(T2);
     const dim3 grid(a->row_ctas, G);
-    using T2 = typename R2<Real>::T;
-#define DQ_CLS(MMV)                                                                                                  \
-    k_adj_cls<Real, MMV><<<grid, kAdjThreads, smem, c->stream>>>(n, B, m, a->seg_tc, batched_basis_chunk(a->ws2), a->rows_per_cta, G, a->n_cls,                \
-                                                               (const Real*)slot_V(a, m, slot),                      \
-                                                               (const Real*)a->ws2->slabs,                           \
-                                                               slab_reals, c->d_rowptr, c->d_col, a->d_cls,           \
-                                                               a->d_vbase, (const T2*)a->d_coef, a->d_gcls,    \
-                                                               c->scales[0] != 0.0)
+#define DQ_SWEEP(MMV)                                                                                              \
+    k_adj_sweep<Real, MMV, sweep_rows<Real, MMV>()><<<grid, kAdjThreads, smem, c->stream>>>(                        \
+        n, B, m, a->seg_tc, batched_basis_chunk(a->ws2), a->rows_per_cta, G, a->n_cls,                              \
+        (const Real*)slot_V(a, m, slot), (Real*)a->ws2->slabs, slab_reals,                                         \
+        (const Real*)(a->seg_diag + (size_t)slot * a->diag_bytes), c->d_psi0, a->d_G + t, a->inv_norm, write_lam,   \
+        c->d_rowptr, c->d_col, a->d_cls, a->d_vbase, (const T2*)a->d_coef, a->d_lpart, a->d_gsite, a->d_gcpl,       \
+        a->d_gcls, a->n_cls && c->scales[0] != 0.0)
     switch (mm_bucket(m)) {
-        case 8: DQ_CLS(8); break;
-        case 16: DQ_CLS(16); break;
-        default: DQ_CLS(24); break;
+        case 8: DQ_SWEEP(8); break;
+        case 16: DQ_SWEEP(16); break;
+        default: DQ_SWEEP(24); break;
     }
-#undef DQ_CLS
+#undef DQ_SWEEP
 }
 
 template <typename Real>
 static cudaError_t set_attrs(int m) {
-    const int CS = m * (2 * m + 2);
-    const int smem = CS * kAdjTraj * (int)sizeof(typename R2<Real>::T);
+    const int smem = sweep_coefs(m) * kAdjTraj * (int)sizeof(typename R2<Real>::T);
     cudaError_t e = raise_smem_limit(k_adj_small<Real>, (int)adj_small_smem(m));
     if (e != cudaSuccess) return e;
     switch (mm_bucket(m)) {
@@ -877,7 +852,7 @@ dq_status dq_adjoint_setup(dq_ctx* c, int n_steps, int fft_len, double scale, co
             if ((st = check_cuda(c, cudaMalloc(&a->ck_deps, sizeof(double) * (size_t)n * B * (n_seg - 1)),
                                  "adjoint checkpoints"))) break;
         }
-        const int CS = m * (2 * m + 2);
+        const int CS = sweep_coefs(m);
         if ((st = check_cuda(c, cudaMalloc(&a->d_coef, 2 * rsz * (size_t)B * CS), "adjoint alloc"))) break;
         const int G = B / kAdjTraj;
         a->row_ctas = std::max(1, std::min((bs->sms * 4 + G - 1) / G, (n + 31) / 32));
@@ -1078,13 +1053,11 @@ dq_status dq_backward(dq_ctx* c, double* grad_sites, double* grad_classes) {
             SV.sc = SV.beta + (size_t)kMaxL * B;
             if (bs->mixed) {
                 k_adj_small<float><<<B, 256, small_smem, c->stream>>>(m, B, c->tau_im, SV, w2->s, (float2*)a->d_coef);
-                if (a->n_cls) launch_cls<float>(c, a, slot);   // reads lambda(t+1) before k_adj_grad replaces it
-                launch_grad<float>(c, a, t, slot, t > 0);
+                launch_sweep<float>(c, a, t, slot, t > 0);
             } else {
                 k_adj_small<double><<<B, 256, small_smem, c->stream>>>(m, B, c->tau_im, SV, w2->s,
                                                                        (double2*)a->d_coef);
-                if (a->n_cls) launch_cls<double>(c, a, slot);
-                launch_grad<double>(c, a, t, slot, t > 0);
+                launch_sweep<double>(c, a, t, slot, t > 0);
             }
             if (t > 0) k_lam_norm<<<sc_blocks, 256, 0, c->stream>>>(B, a->row_ctas, a->d_lpart, w2->s);
             DQ_CU(cudaGetLastError());
