@@ -27,6 +27,7 @@
 
 #include "dq_batched.cuh"
 #include "dq_rng.cuh"
+#include "dq_tma.cuh"
 
 namespace dq {
 
@@ -72,6 +73,7 @@ struct ClusterArgs {
     double* pops_row;
     cd* corr_pt;
     PlainScalars* ps;
+    PlainGrid* grid;          // kDropInGrid: the partial sums and the barrier
     // Taylor-Krylov step (kTaylor): psi_in and psi_out are the ensemble's states, the matrix above is the
     // step's Hamiltonian, the Lanczos iterations run on B; per trajectory <bra|psi> and sum |psi|^4
     int tk_p;
@@ -257,6 +259,101 @@ struct ClSum {
     }
 };
 
+// The same over the whole grid (one trajectory, a cooperative launch).  A CTA
+// writes its part, fences it with its slab rows and counts itself in; one
+// thread of each CTA waits for the count, then all CTAs add the parts in rank
+// order.  The parts are double-buffered by the barrier's parity: a CTA writes
+// a buffer again only after a barrier that all readers of its old contents
+// have passed.  (Parts as tagged words polled by a thread per rank, without a
+// count, took 3700 to 12,500 cycles with 63 CTAs: the polls crowd the words.)
+// The wait is bounded: a CTA that gives up records DQ_ERR_TIMEOUT and stops
+// waiting for the rest of the launch (its results are void, its accesses stay
+// in bounds), so every CTA ends.
+struct ClGridSum {
+    double2* ex;    // [2]: the totals
+    double2* red;   // [2][warps]
+    PlainGrid* g;
+    int* status;
+    int* dead;      // shared: this CTA gave up
+    int G;
+    unsigned rank;
+    unsigned seq;   // barriers passed
+    int pending;
+
+    template <bool kPair>
+    __device__ __forceinline__ void part(int buf, const double (&x)[1], const double (&y)[1]) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const double a = warp_sum(x[0]), b = kPair ? warp_sum(y[0]) : 0.0;
+        if (lane == 0) red[buf * kClWarps + warp] = make_double2(a, b);
+        pending |= 1 << buf;
+    }
+    __device__ __forceinline__ void sync() {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const unsigned par = seq & 1;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            // a warp: lane w + 16 buf holds a warp's part of sum buf
+            static_assert(kClWarps == 16, "a half warp per sum");
+            double2 v = red[lane];
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) {
+                v.x += __shfl_down_sync(0xffffffffu, v.x, o, 16);
+                v.y += __shfl_down_sync(0xffffffffu, v.y, o, 16);
+            }
+            if ((lane & 15) == 0 && ((pending >> (lane >> 4)) & 1)) __stcg(&g->part[par][lane >> 4][rank], v);
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence();   // the CTA's stores (ordered by the barriers before this) before the count
+                atomicAdd(&g->count, 1u);
+                const unsigned want = (seq + 1) * (unsigned)G;
+                const long long t0 = clock64();
+                while (*dead == 0) {
+                    unsigned c;
+                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&g->count) : "memory");
+                    if (c >= want) break;
+                    if (clock64() - t0 > kWaitCycles) {
+                        *dead = 1;
+                        atomicCAS(status, 0, DQ_ERR_TIMEOUT);
+                    }
+                }
+                __threadfence();
+            }
+        }
+        __syncthreads();
+        for (int buf = 0; buf < 2; ++buf) {
+            if (!((pending >> buf) & 1)) continue;
+            double2 s = make_double2(0.0, 0.0);
+            if ((int)threadIdx.x < G) s = __ldcg(&g->part[par][buf][threadIdx.x]);
+            s.x = warp_sum(s.x);
+            s.y = warp_sum(s.y);
+            if (lane == 0) red[buf * kClWarps + warp] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2 && ((pending >> threadIdx.x) & 1)) {
+            double2 s = red[threadIdx.x * kClWarps];
+            for (int w = 1; w < kPlainGridMax / 32; ++w) {
+                const double2 v = red[threadIdx.x * kClWarps + w];
+                s.x += v.x;
+                s.y += v.y;
+            }
+            ex[threadIdx.x] = s;
+        }
+        __syncthreads();
+        pending = 0;
+        ++seq;
+    }
+    __device__ __forceinline__ double2 get(int buf, int) const { return ex[buf]; }
+    // the last CTA to leave clears the count for the next launch
+    __device__ __forceinline__ void leave() {
+        if (threadIdx.x == 0 && atomicAdd(&g->left, 1u) == (unsigned)G - 1) {
+            g->count = 0;
+            g->left = 0;
+            __threadfence();
+        }
+    }
+};
+static_assert(kPlainGridMax <= kClThreads && kPlainGridMax / 32 <= kClWarps, "a thread per rank");
+
 __device__ __forceinline__ unsigned sm_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ float4 lds_f4(unsigned a) {
     float4 v;
@@ -397,20 +494,21 @@ __device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double 
 }
 
 // What a launch carries through its step.
-enum { kEnsemble = 0, kDropIn = 1, kTaylor = 2 };
+enum { kEnsemble = 0, kDropIn = 1, kTaylor = 2, kDropInGrid = 3 };
 
 template <typename Real, int TPT, int R, bool kLocal, int kMode = kEnsemble>
 __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArgs A) {
-    constexpr bool kPlain = kMode == kDropIn, kTk = kMode == kTaylor;
+    constexpr bool kGrid = kMode == kDropInGrid, kPlain = kMode == kDropIn || kGrid, kTk = kMode == kTaylor;
     using T = typename VL<Real, TPT>::T;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int mtr[kMaxTC];
     __shared__ int flag;   // some trajectory's exponential needs the dense form
     const int TC = A.TC, TL = TC / TPT, B = A.B, n = A.n;
-    const int CS = kLocal ? 1 : (int)cl_size();
-    const unsigned rank = kLocal ? 0u : cl_rank();
+    __shared__ int dead;
+    const int CS = kLocal ? 1 : kGrid ? (int)gridDim.x : (int)cl_size();
+    const unsigned rank = kLocal ? 0u : kGrid ? blockIdx.x : cl_rank();
     const int bw = kLocal ? 0 : A.bw;
-    const ClLayout Y = cl_layout(n, CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem, kTk);
+    const ClLayout Y = cl_layout(n, kGrid ? 2 : CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem, kTk);
     double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
     double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
     // [0][t] the update's coefficients, [1][t] (sc_j, the factor of r_{j-1}), [2][t] complex64: Im alpha's low part
@@ -421,11 +519,16 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     Real* win = reinterpret_cast<Real*>(smem + Y.win);
     Real* prev = reinterpret_cast<Real*>(smem + Y.prev);
     Real* dsm = reinterpret_cast<Real*>(smem + Y.d);
-    const ClSum<TPT, kLocal> sum{reinterpret_cast<double2*>(smem + Y.ex), reinterpret_cast<double2*>(smem + Y.red),
-                                 TC, CS, rank, (int)threadIdx.x % TC, (int)threadIdx.x / TC};
+    auto make_sum = [&]() {
+        double2* ex = reinterpret_cast<double2*>(smem + Y.ex);
+        double2* red = reinterpret_cast<double2*>(smem + Y.red);
+        if constexpr (kGrid) return ClGridSum{ex, red, A.grid, A.S.status, &dead, CS, rank, 0u, 0};
+        else return ClSum<TPT, kLocal>{ex, red, TC, CS, rank, (int)threadIdx.x % TC, (int)threadIdx.x / TC};
+    };
+    auto sum = make_sum();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tl = threadIdx.x % TL, rl = threadIdx.x / TL, RL = kClThreads / TL;
-    const int chunk = blockIdx.x / CS, c0 = chunk * TC;
+    const int chunk = kGrid ? 0 : blockIdx.x / CS, c0 = chunk * TC;
     const int b0 = c0 + tl * TPT;
     const bool act = b0 < B;                 // lanes past the last trajectory only keep the barriers
     const int bb = act ? b0 : 0;
@@ -564,7 +667,12 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         par[TC + threadIdx.x] = make_double2(s1, 0.0);
         mtr[threadIdx.x] = 0;
     }
-    sum.sync();   // every CTA of the cluster runs; the window is in place
+    if constexpr (kGrid) {
+        if (threadIdx.x == 0) dead = 0;
+        __syncthreads();
+    } else {
+        sum.sync();   // every CTA of the cluster runs; the window is in place
+    }
 
     const int rowb = rowr * (int)sizeof(Real);
     const unsigned wcol = sm_addr(cur) - (unsigned)(r0 * rowb) + tl * TPT * 2 * (int)sizeof(Real);   // global row 0
@@ -586,7 +694,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     // The window's margins of r_j (j >= 2): the neighbours' rows from their shared memory, or, when
     // the margins are wide, from the slab that the barrier has just published (a window of all 5,278
     // rows in 11 CTAs: a step of 12 iterations took 232 us by DSMEM, 199 us this way)
-    const bool wide = (size_t)(hlo + hhi) * rowr * sizeof(Real) > kClWideMargin;
+    const bool wide = kGrid || (size_t)(hlo + hhi) * rowr * sizeof(Real) > kClWideMargin;
     auto margins = [&](int j) {
         if constexpr (!kLocal) {
             const int nh = act ? hlo + hhi : 0;
@@ -600,8 +708,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                     if (h >= nh) break;
                     const int g = r0 + (h < hlo ? h - hlo : nrow + h - hlo);
                     if (wide) {
-                        v[q] = src[(size_t)g * stride];
-                    } else {
+                        v[q] = __ldcg(src + (size_t)g * stride);
+                    } else if constexpr (!kGrid) {
                         const int own = g / A.rpc;
                         // the owner's own rows start after its lower margin
                         const int at = min(bw, own * A.rpc) + g - own * A.rpc;
@@ -878,7 +986,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     if (!(A.flags & kClFinish)) {
         // the neighbours may still read this CTA's rows of the last window
-        if constexpr (!kLocal) cl_sync();
+        if constexpr (!kLocal && !kGrid) cl_sync();
         return;
     }
     // ---- ||H q_{m+1}|| ---------------------------------------------------------
@@ -1048,7 +1156,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             else stv<Real, TPT>(slab(1), x, o);
         }
     // ex[0] still holds ||H q_{m+1}||, which slower CTAs may be reading
-    sum.sync();
+    if constexpr (kGrid) __syncthreads();
+    else sum.sync();
     sum.template part<true>(0, cr, ci);
     sum.template part<kTk>(1, nn, q4);
     sum.sync();
@@ -1092,6 +1201,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 A.corr_pt->y += c.y * inv;
             }
         }
+        if constexpr (kGrid) sum.leave();
     } else if (rank == 0) {
         double* cs = reinterpret_cast<double*>(sum.red);   // free again: the chunk's correlation terms
         if (threadIdx.x < TC) {
@@ -1367,6 +1477,28 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
             best.rec = room;
         }
     }
+    // Larger systems: a cooperative grid, of as few CTAs as hold the records and give every row a
+    // thread (fewer have a cheaper barrier, and steps of other streams run beside them).  Its two
+    // barriers take about 4500 of an iteration's 14,800 cycles each (30,000 sites with 28 couplings,
+    // m = 20: 184 us a step as 2 m + 5 launches, 91 us this way, three states in turn)
+    int dev = 0, sms = 0;
+    if (z > 0.0 && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
+        for (int G = kClMaxCtas + 1; G <= std::min(sms, kPlainGridMax); ++G) {
+            const int rpc = cl_rows(n, G, 1);
+            if (rpc > kClThreads) continue;
+            const size_t fixed = cl_layout(n, 2, 1, m, rpc, bw, sizeof(double), 0).total;
+            if (fixed + 4096 > kClSmemMax || rpc * (z * 1.15 + 2.0) * 12.0 > (double)(kClSmemMax - fixed - 4096)) continue;
+            const double t = 400.0 + 75.0 * z + 0.25 * rpc * z + 6500.0;
+            if (t < t_best) {
+                best.ctas = (n + rpc - 1) / rpc;
+                best.rpc = rpc;
+                best.rec = (kClSmemMax - fixed) / 16 * 16 - 16;
+                best.smem = fixed + best.rec;
+            }
+            break;
+        }
+    }
     return best;
 }
 
@@ -1376,6 +1508,7 @@ cudaError_t plain_cluster_attributes() {
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_cluster_step<double, 1, 1, false, kDropIn>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = raise_smem_limit(k_cluster_step<double, 1, 1, false, kDropInGrid>, (int)kClSmemMax);
     return e;
 }
 
@@ -1419,9 +1552,16 @@ cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cuda
     a.pops_row = q.pops_row;
     a.corr_pt = q.corr_pt;
     a.ps = q.ps;
+    a.grid = q.grid;
     a.scratch = q.scratch;
     cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = cl_config(1, P.ctas, P.smem, st, &at);
+    cudaLaunchConfig_t cfg = cl_config(1, P.ctas, P.smem, st, &at);
+    if (P.ctas > kClMaxCtas) {
+        // every CTA resident at once: they wait for one another
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        return cudaLaunchKernelEx(&cfg, k_cluster_step<double, 1, 1, false, kDropInGrid>, a);
+    }
     return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, kDropIn>
                                                 : k_cluster_step<double, 1, 1, false, kDropIn>, a);
 }

@@ -36,8 +36,19 @@ constexpr int kMaxPartials = 4096;
 constexpr int kMaxZZOsc = 1024;   // oscillators of one ZZ spectral density
 constexpr int kIprRowGroups = 296; // row groups of the ensemble IPR reduction (2 per SM)
 
-// The one-launch drop-in step (dq_cluster.cu): CTAs of its cluster (0: the
-// system is too large for it), rows per CTA, shared memory.
+// What the CTAs of a step that the whole grid takes tell one another: each
+// rank's sums, by the barrier's parity, and the counts of CTAs that arrived
+// and that left (zero between launches).
+constexpr int kPlainGridMax = 256;
+struct PlainGrid {
+    double2 part[2][2][kPlainGridMax];
+    alignas(128) unsigned int count;
+    alignas(128) unsigned int left;
+};
+
+// The one-launch drop-in step (dq_cluster.cu): its CTAs (at most 16: one
+// cluster; more: the whole grid; 0: the system is too large for it), rows per
+// CTA, shared memory.
 struct PlainCluster {
     int ctas = 0, rpc = 0;
     size_t smem = 0, rec = 0;
@@ -54,6 +65,7 @@ struct PlainStep {
     cd* psi_out;
     cd* Q;                   // m + 2 vectors of n
     PlainScalars* ps;
+    PlainGrid* grid;         // used by the whole-grid form (zero between launches)
     double tau_im;
     // noise of the step (draw): trajectory, step and the parameters of k_noise
     bool draw;
@@ -158,6 +170,7 @@ struct dq_ctx {
     double* d_partial = nullptr;  // kMaxPartials x 2
     dq::PlainScalars* d_ps = nullptr;
     unsigned char* d_pade = nullptr;       // the one-launch step's dense exponential
+    dq::PlainGrid* d_grid = nullptr;       // and its whole-grid form's barrier
     dq::PlainCluster plain;                // its shape for the Hamiltonian that is set
 
     // observables (sums over trajectories; divided by n_traj on read)

@@ -514,6 +514,8 @@ dq_status plain_alloc(dq_ctx* c) {
     DQ_CU(cudaMalloc(&c->d_partial, sizeof(double) * 2 * kMaxPartials));
     DQ_CU(cudaMalloc(&c->d_ps, sizeof(PlainScalars)));
     DQ_CU(cudaMalloc(&c->d_pade, pade_smem_bytes(m + 2)));
+    DQ_CU(cudaMalloc(&c->d_grid, sizeof(PlainGrid)));
+    DQ_CU(cudaMemsetAsync(c->d_grid, 0, sizeof(PlainGrid), c->stream));
     DQ_CU(cudaMemsetAsync(c->d_ps, 0, sizeof(PlainScalars), c->stream));
     DQ_CU(cudaMemsetAsync(c->d_Q, 0, sizeof(cd) * (size_t)n * (m + 2), c->stream));
     // the limit is a per-function attribute shared by every context (and by
@@ -530,7 +532,9 @@ dq_status plain_alloc(dq_ctx* c) {
 void plain_free(dq_ctx* c) {
     cudaFree(c->d_eps_p); cudaFree(c->d_deps_p); cudaFree(c->d_diag); cudaFree(c->d_Q); cudaFree(c->d_w);
     cudaFree(c->d_psi_a); cudaFree(c->d_psi_b); cudaFree(c->d_partial); cudaFree(c->d_ps); cudaFree(c->d_pade);
+    cudaFree(c->d_grid);
     c->d_pade = nullptr;
+    c->d_grid = nullptr;
     c->d_eps_p = c->d_deps_p = c->d_diag = c->d_partial = nullptr;
     c->d_Q = c->d_w = c->d_psi_a = c->d_psi_b = nullptr;
     c->d_ps = nullptr;
@@ -648,6 +652,7 @@ dq_status plain_step(dq_ctx* c, int traj, int step, const cd* psi_in, cd* psi_ou
         q.psi_out = psi_out;
         q.Q = c->d_Q;
         q.ps = c->d_ps;
+        q.grid = c->d_grid;
         q.tau_im = c->tau_im;
         q.draw = c->cfg.noise_model != DQ_NOISE_ZZ;
         q.noise = c->cfg.noise_model;

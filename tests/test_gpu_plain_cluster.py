@@ -21,7 +21,7 @@ def _oracle_step(oracle, s, m, dt, dot, norm, noise, traj, steps, psi):
 
 
 @pytest.mark.parametrize("shape", [(2,), (33,), (511,), (512,), (513,), (1024,), (1025,), (4000,), (8191,), (20000,),
-                                   (10, 7), (23, 30), (58, 91)])
+                                   (10, 7), (23, 30), (58, 91), (60, 150), (60, 500)])
 @pytest.mark.parametrize("dot,norm", [(0, 0), (1, 1)])
 def test_step_sizes_match_oracle(oracle, shape, dot, norm):
     import torch
@@ -48,6 +48,33 @@ def test_step_sizes_match_oracle(oracle, shape, dot, norm):
         ref, err_o = _oracle_step(oracle, s, m, 0.7, dot, norm, 2, 1 + shift, 1, psi)
         assert np.abs(out.cpu().numpy() - ref).max() < PSI_TOL, shift
         assert err == pytest.approx(err_o, rel=1e-3, abs=1e-14)
+    p.close()
+
+
+@pytest.mark.parametrize("shape", [(58, 91), (60, 150)])
+def test_consecutive_steps_match_oracle(oracle, shape):
+    """Steps issued one after another without a synchronisation (cluster and whole-grid form)."""
+    import torch
+    import dynaquant_b200 as dq
+    from dynaquant_b200 import systems
+    s = systems.tube(*shape)
+    p = dq.Propagator(s.n, m=9, n_traj=2, dt=0.7, noise=dq.NOISE_OU, sigma_static=80.0, seed=21, dot=1, norm=1,
+                      precision=dq.PREC_FP64, max_steps=2)
+    p.set_system(s)
+    p.set_noise_params(np.full(s.n, 150.0), np.full(s.n, 70.0))
+    psi = s.bright_state()
+    p.set_initial_state(psi)
+    p.reset()
+    a = torch.from_numpy(psi).cuda()
+    b = torch.empty_like(a)
+    torch.cuda.synchronize()
+    for k in range(5):
+        p.prop_step(1, k, a.data_ptr(), b.data_ptr())
+        a, b = b, a
+    err = p.prop_step(1, 5, a.data_ptr(), b.data_ptr(), want_error=True)
+    ref, err_o = _oracle_step(oracle, s, 9, 0.7, 1, 1, 2, 1, 6, psi)
+    assert np.abs(b.cpu().numpy() - ref).max() < PSI_TOL
+    assert err == pytest.approx(err_o, rel=1e-3, abs=1e-14)
     p.close()
 
 
