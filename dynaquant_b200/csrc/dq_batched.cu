@@ -2808,8 +2808,11 @@ __global__ void __launch_bounds__(32 * kPadeWarps) k_pade_b(int mmax, int B, dou
 // psi = sum_j yt_j r_j written over slab 1; ||psi||^2 and <psi0|psi> per
 // trajectory; correlation point step+1 per chunk (propStep.cu:31-44,
 // systemClass.cu:1771-1829, spectraClass.cu:510-571)
+// The streaming grid is one wave of kStreamCtasPerSm CTAs per SM, so the
+// registers must allow as many: three took 438 us instead of 282 (30,000 sites
+// x 256, m = 20).
 template <typename Real, int TPT>
-__global__ void __launch_bounds__(kBThreads) k_combine_b(int n, int B, int TC, int rpc, int m,
+__global__ void __launch_bounds__(kBThreads, kStreamCtasPerSm) k_combine_b(int n, int B, int TC, int rpc, int m,
                                                         Real* __restrict__ slabs, size_t slab_stride,
                                                         const cd* __restrict__ psi0, BatchedScalars S) {
     const Tile<TPT> T(TC, rpc, n);
@@ -3542,7 +3545,11 @@ dq_status batched_set_tiling(dq_ctx* c, int tc, int tpt, int ctas_per_sm, int R,
     const int nb = (n + R - 1) / R;
     int gxs = std::max(1, (bs->sms * ctas_per_sm) / cpg);
     int bpc = (nb + gxs - 1) / gxs;
-    bpc = ((bpc + RPC_spmm - 1) / RPC_spmm) * RPC_spmm;
+    // whole passes of the CTA, or for form 12, whose one large CTA per SM takes few passes, whole warps:
+    // 9 CTAs a chunk with 8.7 passes each instead of 8 with 9 and one with 6 (30,000 sites x 256: 95.4 ->
+    // 92.9 us a launch; 78 couplings a row x 256: 181 -> 176)
+    const int unit = staged == 12 ? std::max(1, 32 / TPR) : RPC_spmm;
+    bpc = ((bpc + unit - 1) / unit) * unit;
     gxs = (nb + bpc - 1) / bpc;
     if (gx > kMaxCtasPerChunk || (size_t)gx * B * 2 > bs->partial_cap) return DQ_ERR_ARG;
     if (gxs > kMaxCtasPerChunk || (size_t)gxs * B * 2 > bs->partial_cap) return DQ_ERR_ARG;
