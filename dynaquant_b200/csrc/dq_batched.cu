@@ -26,6 +26,7 @@
 // One time step (propagate.cu:199-259 for all trajectories at once):
 //   k_noise_b, m x {k_spmm, k_axpy_beta}, k_spmm (norm), k_pade_b,
 //   k_combine_b, k_pop_b
+// or, for ensembles that fit on the chip (form 13), k_cluster_step, k_pop_b;
 // captured once into a CUDA graph and replayed per step; the step index lives
 // in device memory.
 #include <climits>

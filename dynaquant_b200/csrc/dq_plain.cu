@@ -1,7 +1,10 @@
 // dq_plain.cu — the plain FP64 per-trajectory form: the drop-in for one
 // reference time step (propagate.cu:211-254).
 //
-// Per step, all on the context's stream, no host synchronisation:
+// Per step, all on the context's stream, no host synchronisation: one launch of
+// dq_cluster.cu where its plan takes the system and the state is 16-byte
+// aligned (one cluster up to about 16 CTAs' worth of rows, a cooperative grid
+// above), else, and for full reorthogonalisation and Taylor-Krylov steps:
 //   k_noise          OU / Gaussian update of this trajectory's diagonal
 //                    (gpuSysHelper.cu:32-128, Philox instead of cuRAND)
 //   m x { k_spmv_alpha, k_axpy_norm }

@@ -2,6 +2,9 @@
 // in Taylor-Krylov mode; taylorKrylovClass.cu:223-434 per trajectory in the
 // reference).
 //
+// Ensembles that fit on the chip take one launch a step (dq_cluster.cu); what
+// follows is the form for the others.
+//
 // FP64 throughout, on [site][traj] slabs of complex128 (coalesced over the
 // trajectories of one site).  Every kernel runs on a grid of row groups x
 // trajectory blocks: thread (g, b) handles trajectory b on rows g, g + G, ...
