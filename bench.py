@@ -189,8 +189,8 @@ def plain_roofline(s, value):
     peak, kind = _peaks()
     gbs = value * per / 1e9
     return {"bytes_per_traj_step": per, "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
-            "peak_kind": kind, "note": "about 45 launches per trajectory-step, one trajectory at a time: "
-                                       "launch-latency bound, not HBM bound"}
+            "peak_kind": kind, "note": "one launch per trajectory-step, one trajectory at a time: "
+                                       "bound by its barriers, not HBM bound"}
 
 
 def dominant_kernel(s, B, m, staged, prof):
