@@ -166,6 +166,13 @@ class Propagator:
         the ring form's CTAs first wait that many cycles on a barrier nothing completes, so they time out)."""
         self._check(self.L.dq_debug_set_wait_cycles(self.h, int(cycles)))
 
+    def debug_step_shape(self):
+        """Test hook: CTAs of the drop-in step, CTAs, trajectories and record bytes of the Taylor-Krylov
+        ensemble's cluster (0 CTAs: a step of several launches)."""
+        v = [C.c_int() for _ in range(4)]
+        self._check(self.L.dq_debug_step_shape(self.h, *[C.byref(x) for x in v]))
+        return tuple(x.value for x in v)
+
     def autotune_raw(self, reps=5):
         ms = C.c_double()
         self._check(self.L.dq_autotune(self.h, reps, C.byref(ms)))

@@ -784,3 +784,27 @@ extern "C" dq_status dq_debug_set_wait_cycles(dq_ctx* c, int cycles) {
     if (!c) return DQ_ERR_ARG;
     return batched_set_wait_cycles(c, cycles);
 }
+
+extern "C" dq_status dq_debug_taylor_shape(int n, int ctas, int traj_chunk, int m_b, int bandwidth, int* smem, int* rec,
+                                           int* head) {
+    if (n < 2 || ctas < 1 || ctas > 16 || traj_chunk < 1 || traj_chunk > 32 || (traj_chunk & (traj_chunk - 1)) ||
+        m_b < 1 || m_b > kMaxM || bandwidth < 0 || !smem || !rec || !head)
+        return DQ_ERR_ARG;
+    TaylorCluster P;
+    if (!taylor_cluster_shape(n, ctas, traj_chunk, m_b, bandwidth, &P)) return DQ_ERR_ARG;
+    *smem = (int)P.smem;
+    *rec = (int)P.rec;
+    *head = (int)taylor_cluster_head(P);
+    return DQ_OK;
+}
+
+extern "C" dq_status dq_debug_step_shape(dq_ctx* c, int* plain_ctas, int* taylor_ctas, int* taylor_traj,
+                                         int* taylor_rec) {
+    if (!c || !plain_ctas || !taylor_ctas || !taylor_traj || !taylor_rec) return DQ_ERR_ARG;
+    const TaylorCluster P = tk_ensemble_shape(c);
+    *plain_ctas = c->plain.ctas;
+    *taylor_ctas = P.ctas;
+    *taylor_traj = P.tc;
+    *taylor_rec = (int)P.rec;
+    return DQ_OK;
+}

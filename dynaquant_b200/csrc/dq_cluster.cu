@@ -117,6 +117,11 @@ static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int 
     return L;
 }
 
+// Bytes of the block and group starts in front of the records of nb row blocks, `per` to a group.
+static __host__ __device__ inline size_t cl_rec_head(size_t nb, int per) {
+    return ((nb + (nb + per - 1) / per + 2) * 4 + 15) / 16 * 16;
+}
+
 __device__ __forceinline__ unsigned cl_rank() {
     unsigned r;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -555,9 +560,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     ClRecs Q;
     auto load_records = [&](const int* gptr, const int* gcol, const void* gcoef) {
         Q = ClRecs{gptr + kb0, gcol, gcoef, 0u, 0u, nullptr, -1};
-        if (!A.rec_smem) return;
         // block starts, group starts (a group is as long as its longest block), columns (FP64), coefficients
         const int lg = __ffs(32 / TL) - 1, per = 1 << lg, ng = (nbo + per - 1) >> lg;
+        const size_t head = cl_rec_head(nbo, per);
+        if (head > (size_t)A.rec_smem) return;
         int* sb = reinterpret_cast<int*>(smem + Y.rec);
         int* sg = sb + nbo + 1;
         for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(gptr + kb0 + k);
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             for (int g = 0; g < ng; ++g) sg[g + 1] += sg[g];
         }
         __syncthreads();
-        const size_t slots = (size_t)sg[ng] << lg, head = (((size_t)nbo + ng + 2) * 4 + 15) / 16 * 16;
+        const size_t slots = (size_t)sg[ng] << lg;
         const size_t cols = sizeof(Real) == 8 ? (slots * 4 + 15) / 16 * 16 : 0;
         unsigned char* q = smem + Y.rec + head + cols;
         Q.bptr = sb;
@@ -1286,7 +1292,7 @@ static cudaLaunchConfig_t cl_config(int chunks, int CS, size_t smem, cudaStream_
 // Bytes of the largest CTA's coupling records (block starts, columns, coefficients).
 static size_t cl_rec_bytes(const ::BlockFmt& f, bool mixed, int rpc, int R, int TL) {
     const size_t per = 32 / TL, nb = rpc / R, slots = (nb + per - 1) / per * per * (size_t)f.max_block;
-    const size_t head = ((nb + (nb + per - 1) / per + 2) * 4 + 15) / 16 * 16;
+    const size_t head = cl_rec_head(nb, (int)per);
     if (mixed) return head + slots * 16;
     return head + (slots * 4 + 15) / 16 * 16 + slots * R * sizeof(double);
 }
@@ -1567,6 +1573,26 @@ cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cuda
 }
 
 // ---- Taylor-Krylov steps of an ensemble --------------------------------------
+// The shape of n sites on CS CTAs with tc trajectories (false: it does not fit):
+// rows per CTA, shared memory, the part of it left for the records.  The kernel
+// decides whether a CTA's records fit there; where not even their block starts
+// do, none is asked for and all is read through L1.
+bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P) {
+    const int rpc = cl_rows(n, CS, 1);
+    if (CS > 1 && (size_t)rpc * (CS - 1) >= (size_t)n) return false;
+    const size_t fixed = cl_layout(n, CS, tc, mb, rpc, bw, sizeof(double), 0, true).total;
+    if (fixed + 4096 > kClSmemMax) return false;
+    const size_t room = (kClSmemMax - fixed) / 16 * 16 - 16;
+    P->ctas = CS;
+    P->tc = tc;
+    P->rpc = rpc;
+    P->rec = cl_rec_head(rpc, 32 / tc) <= room ? room : 0;
+    P->smem = fixed + P->rec;
+    return true;
+}
+
+size_t taylor_cluster_head(const TaylorCluster& P) { return cl_rec_head(P.rpc, 32 / P.tc); }
+
 // CTAs and trajectories of a cluster for n sites x B trajectories, z couplings
 // per row of the larger matrix and bandwidth bw, by cluster_plan's estimate;
 // ctas = 0: nothing fits.
@@ -1580,15 +1606,13 @@ TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z) {
         return best;
     }
     for (int CS = 1; CS <= kClMaxCtas; ++CS) {
-        const int rpc = cl_rows(n, CS, 1);
-        if (CS > 1 && (size_t)rpc * (CS - 1) >= (size_t)n) continue;
         int fit = 0;   // one CTA per SM whatever its shared memory: resident clusters depend on CS alone
         for (int tc = 1; tc <= 32 && tc < 2 * B; tc *= 2) {
-            const size_t fixed = cl_layout(n, CS, tc, mb, rpc, bw, sizeof(double), 0, true).total;
-            if (fixed + 4096 > kClSmemMax) continue;
-            const size_t room = (kClSmemMax - fixed) / 16 * 16 - 16;
-            const bool in_smem = rpc * (z * 1.15 + 2.0) * 12.0 <= (double)room;
-            const int chunks = (B + tc - 1) / tc;
+            TaylorCluster P;
+            if (!taylor_cluster_shape(n, CS, tc, mb, bw, &P)) continue;
+            const int rpc = P.rpc;
+            const bool in_smem = rpc * (z * 1.15 + 2.0) * 12.0 <= (double)P.rec;
+            P.chunks = (B + tc - 1) / tc;
             const double cycles = 5500.0 + 60.0 * CS +
                                   1.6 * (rpc * z * tc * 16.0 / 128.0 * 1.3 + rpc * z * (in_smem ? 0.125 : 1.6)) +
                                   0.8 * rpc * tc;
@@ -1602,15 +1626,10 @@ TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z) {
                 }
             }
             if (fit < 1) continue;
-            const double t = cycles * ((chunks + fit - 1) / fit);
+            const double t = cycles * ((P.chunks + fit - 1) / fit);
             if (t < t_best) {
                 t_best = t;
-                best.ctas = CS;
-                best.tc = tc;
-                best.rpc = rpc;
-                best.chunks = chunks;
-                best.smem = fixed + room;
-                best.rec = room;
+                best = P;
             }
         }
     }

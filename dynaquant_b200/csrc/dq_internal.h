@@ -254,6 +254,8 @@ dq_status read_status(dq_ctx* c, int code, const char* what);
 // implemented in dq_cluster.cu
 PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
 cudaError_t plain_cluster_attributes();
+bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P);
+size_t taylor_cluster_head(const TaylorCluster& P);
 TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z);
 cudaError_t taylor_cluster_launch(const TaylorCluster& P, const TaylorStep& q, cudaStream_t st);
 cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cudaStream_t st);
@@ -285,6 +287,7 @@ dq_status tk_ensemble_reset(dq_ctx* c);
 dq_status tk_ensemble_run(dq_ctx* c, int n_steps);
 dq_status tk_ensemble_states(dq_ctx* c, dq_cdouble* out);
 void tk_ensemble_free(dq_ctx* c);
+TaylorCluster tk_ensemble_shape(const dq_ctx* c);
 // implemented in dq_fft.cu
 // M(k) *= exp(-(dt (k + 1) / sigma)^2 / 2) for k < n_dress (spectraClass.cu:583-600)
 dq_status dress_correlation(dq_ctx* c, int n_dress, cd* x);

@@ -480,6 +480,8 @@ static dq_status tk_plan(dq_ctx* c) {
     return DQ_OK;
 }
 
+TaylorCluster tk_ensemble_shape(const dq_ctx* c) { return c->tke ? c->tke->cluster : TaylorCluster(); }
+
 // Draws every trajectory's static energies, OU offsets and ZZ phases, sets
 // every state to psi0 and adds the initial observable records (allocates the
 // workspace on first use).

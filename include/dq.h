@@ -305,6 +305,18 @@ DQ_API dq_status dq_time_gather_floor(dq_ctx *ctx, int reps, double *ms);
  * a generation that never comes, with the same outcome.  It applies to every
  * context on the device until changed again. */
 DQ_API dq_status dq_debug_set_wait_cycles(dq_ctx *ctx, int cycles);
+/* Test hooks, no reference counterparts: how the one-launch steps lay a system
+ * out.  dq_debug_taylor_shape (no device): a Taylor-Krylov ensemble of n sites
+ * with clusters of `ctas` CTAs and traj_chunk trajectories; DQ_ERR_ARG when
+ * the shape does not fit, else the bytes of a CTA's shared memory, of the part
+ * for its coupling records (0: read through L1) and of the row starts that
+ * come before them.  dq_debug_step_shape: CTAs of the drop-in step, CTAs and
+ * trajectories per cluster and record bytes of the Taylor-Krylov ensemble (as
+ * the last dq_reset left it); 0 CTAs stand for the step of several launches. */
+DQ_API dq_status dq_debug_taylor_shape(int n, int ctas, int traj_chunk, int m_b, int bandwidth, int *smem, int *rec,
+                                       int *head);
+DQ_API dq_status dq_debug_step_shape(dq_ctx *ctx, int *plain_ctas, int *taylor_ctas, int *taylor_traj,
+                                     int *taylor_rec);
 
 /* Kernel kinds of one ensemble step, for dq_profile_step. */
 enum {
