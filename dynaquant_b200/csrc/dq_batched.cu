@@ -2671,8 +2671,11 @@ __global__ void __launch_bounds__(kBThreads) k_reorth_apply_b(int n, int B, int 
 }
 
 // ---- adaptive Krylov dimension (cfg.m_min > 0) -------------------------------
-// trajectories (warps) per CTA of the Padé kernels
-constexpr int kPadeWarps = 4;
+// threads per CTA of the exponential's kernels, one CTA per trajectory: its first
+// warp sums the series, the whole CTA takes the dense form where that is needed.
+// With four trajectories to a CTA the series cost the same, but the dense form,
+// 45 us for one trajectory of m = 16, came four times in a row.
+constexpr int kPadeThreads = 128;
 
 __global__ void k_adapt_reset(int B, int chunks, int mmax, BatchedScalars S) {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) {
@@ -2684,39 +2687,38 @@ __global__ void k_adapt_reset(int B, int chunks, int mmax, BatchedScalars S) {
     }
 }
 
-// One warp per undecided trajectory after iteration j: EXPOKIT's first error
+// One CTA per undecided trajectory after iteration j: EXPOKIT's first error
 // term beta_j |E(j-1, j)| of exp(tau Tbar_j); the trajectory keeps dimension
 // j when it meets the tolerance.
-__global__ void __launch_bounds__(32 * kPadeWarps) k_mcheck_b(int j, int B, int TC, double tau_im, int norm_mode,
-                                                             double tol, BatchedScalars S) {
+__global__ void __launch_bounds__(kPadeThreads) k_mcheck_b(int j, int B, int TC, double tau_im, int norm_mode,
+                                                          double tol, BatchedScalars S) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ cd al[kMaxL], be[kMaxL];
-    __shared__ bool dense[kPadeWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bw = blockIdx.x * kPadeWarps + warp;
-    const bool mine = bw < B && S.mtraj[bw] == 0 && !S.cdone[bw / TC];
-    bool ok = true;
-    if (mine) {
-        const size_t k = (size_t)(min(lane, j - 1) + 1) * B + bw;
+    __shared__ bool dense;
+    const int b = blockIdx.x;
+    const bool skip = S.mtraj[b] != 0 || S.cdone[b / TC];
+    __syncthreads();   // all have read the choice before it is made below
+    if (skip) return;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const size_t k = (size_t)(min(lane, j - 1) + 1) * B + b;
         cd y, f1, f2;
         int s;
-        ok = series_exp_tbar(j, cmk(S.alpha[2 * k], S.alpha[2 * k + 1]), S.beta[k], tau_im, norm_mode, y, f1, f2, s);
-        if (ok && s >= 0 && lane == j - 1 && fabs(S.beta[k]) * sqrt(cabs2(f1)) <= tol) S.mtraj[bw] = j;
+        const bool ok = series_exp_tbar(j, cmk(S.alpha[2 * k], S.alpha[2 * k + 1]), S.beta[k], tau_im, norm_mode, y, f1,
+                                        f2, s);
+        if (lane == 0) dense = !ok;
+        if (ok && s >= 0 && lane == j - 1 && fabs(S.beta[k]) * sqrt(cabs2(f1)) <= tol) S.mtraj[b] = j;
     }
-    if (lane == 0) dense[warp] = !ok;
     __syncthreads();
-    for (int q = 0; q < kPadeWarps; ++q) {
-        if (!dense[q]) continue;   // uniform over the CTA
-        const int b = blockIdx.x * kPadeWarps + q;
-        for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) {
-            const size_t k = (size_t)i * B + b;
-            al[i] = (i >= 1 && i <= j) ? cmk(S.alpha[2 * k], S.alpha[2 * k + 1]) : cmk(0, 0);
-            be[i] = (i >= 1 && i <= j) ? cmk(S.beta[k], 0.0) : cmk(0, 0);
-        }
-        __syncthreads();
-        const PadeOut o = pade_exp_tbar(j, al, be, cmk(0.0, tau_im), norm_mode, nullptr, smem);
-        if (threadIdx.x == 0 && o.s >= 0 && fabs(be[j].x) * sqrt(cabs2(o.e_m1_m)) <= tol) S.mtraj[b] = j;
-        __syncthreads();
+    if (!dense) return;
+    for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) {
+        const size_t k = (size_t)i * B + b;
+        al[i] = (i >= 1 && i <= j) ? cmk(S.alpha[2 * k], S.alpha[2 * k + 1]) : cmk(0, 0);
+        be[i] = (i >= 1 && i <= j) ? cmk(S.beta[k], 0.0) : cmk(0, 0);
     }
+    __syncthreads();
+    const PadeOut o = pade_exp_tbar(j, al, be, cmk(0.0, tau_im), norm_mode, nullptr, smem);
+    if (threadIdx.x == 0 && o.s >= 0 && fabs(be[j].x) * sqrt(cabs2(o.e_m1_m)) <= tol) S.mtraj[b] = j;
 }
 
 // Per chunk: all trajectories decided -> its remaining iterations are skipped;
@@ -2745,65 +2747,59 @@ __global__ void k_chunk_flags(int TC, int mmax, int final_pass, BatchedScalars S
     }
 }
 
-// One warp per trajectory: exp(tau Tbar), combine weights, error estimate.
-// The CTA takes the trajectories its warps could not do (dense form) together.
-__global__ void __launch_bounds__(32 * kPadeWarps) k_pade_b(int mmax, int B, double tau_im, int norm_mode,
-                                                           BatchedScalars S, double* erracc) {
+// One CTA per trajectory: exp(tau Tbar), combine weights, error estimate.
+__global__ void __launch_bounds__(kPadeThreads) k_pade_b(int mmax, int B, double tau_im, int norm_mode,
+                                                        BatchedScalars S, double* erracc) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ cd al[kMaxL], be[kMaxL], y[kMaxM];
-    __shared__ bool dense[kPadeWarps];
+    __shared__ bool dense;
+    const int b = blockIdx.x;
+    // adaptive dimension: this trajectory's choice; weights past it are zero
+    const int m = S.mtraj ? S.mtraj[b] : mmax;
     // with the adaptive dimension only err1 (||H q_{m+1}|| belongs to the largest m)
-    auto estimate = [&](double beta_m, int b, cd e1, cd e2) {
+    auto estimate = [&](double beta_m, cd e1, cd e2) {
         return S.mtraj ? fmax(fabs(beta_m) * sqrt(cabs2(e1)), 1.110223e-16) : expokit_error(beta_m, S.nav[b], e1, e2);
     };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bw = blockIdx.x * kPadeWarps + warp;
-    bool ok = true;
-    if (bw < B) {
-        // adaptive dimension: this trajectory's choice; weights past it are zero
-        const int m = S.mtraj ? S.mtraj[bw] : mmax;
-        const size_t k = (size_t)(min(lane, m - 1) + 1) * B + bw;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const size_t k = (size_t)(min(lane, m - 1) + 1) * B + b;
         const double beta = S.beta[k];
         cd yl, f1, f2;
         int s;
-        ok = series_exp_tbar(m, cmk(S.alpha[2 * k], S.alpha[2 * k + 1]), beta, tau_im, norm_mode, yl, f1, f2, s);
+        const bool ok = series_exp_tbar(m, cmk(S.alpha[2 * k], S.alpha[2 * k + 1]), beta, tau_im, norm_mode, yl, f1, f2,
+                                        s);
+        if (lane == 0) dense = !ok;
         if (ok && s < 0) {
             if (lane == 0) atomicCAS(S.status, 0, DQ_ERR_SCALING);
         } else if (ok) {
             if (lane < mmax) {
-                const size_t ky = (size_t)(lane + 1) * B + bw;
+                const size_t ky = (size_t)(lane + 1) * B + b;
                 const cd v = lane < m ? cscale(yl, S.sc[ky]) : cmk(0.0, 0.0);
                 *reinterpret_cast<double2*>(S.yt + 2 * ky) = make_double2(v.x, v.y);
             }
-            if (lane == m - 1) erracc[bw] += estimate(beta, bw, f1, f2);
+            if (lane == m - 1) erracc[b] += estimate(beta, f1, f2);
         }
     }
-    if (lane == 0) dense[warp] = !ok;
     __syncthreads();
-    for (int q = 0; q < kPadeWarps; ++q) {
-        if (!dense[q]) continue;   // uniform over the CTA
-        const int b = blockIdx.x * kPadeWarps + q;
-        const int m = S.mtraj ? S.mtraj[b] : mmax;
-        for (int j = threadIdx.x; j <= m + 1; j += blockDim.x) {
-            const size_t k = (size_t)j * B + b;
-            al[j] = (j >= 1 && j <= m) ? cmk(S.alpha[2 * k], S.alpha[2 * k + 1]) : cmk(0, 0);
-            be[j] = (j >= 1 && j <= m) ? cmk(S.beta[k], 0.0) : cmk(0, 0);
-        }
-        __syncthreads();
-        const PadeOut o = pade_exp_tbar(m, al, be, cmk(0.0, tau_im), norm_mode, y, smem);
-        __syncthreads();
-        if (o.s < 0) {
-            if (threadIdx.x == 0) atomicCAS(S.status, 0, o.s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
-            continue;
-        }
-        for (int j = threadIdx.x; j < mmax; j += blockDim.x) {
-            const size_t k = (size_t)(j + 1) * B + b;
-            const cd v = j < m ? cscale(y[j], S.sc[k]) : cmk(0.0, 0.0);
-            S.yt[2 * k] = v.x;
-            S.yt[2 * k + 1] = v.y;
-        }
-        if (threadIdx.x == 0) erracc[b] += estimate(be[m].x, b, o.e_m1_m, o.e_m1_mp1);
-        __syncthreads();
+    if (!dense) return;
+    for (int j = threadIdx.x; j <= m + 1; j += blockDim.x) {
+        const size_t k = (size_t)j * B + b;
+        al[j] = (j >= 1 && j <= m) ? cmk(S.alpha[2 * k], S.alpha[2 * k + 1]) : cmk(0, 0);
+        be[j] = (j >= 1 && j <= m) ? cmk(S.beta[k], 0.0) : cmk(0, 0);
     }
+    __syncthreads();
+    const PadeOut o = pade_exp_tbar(m, al, be, cmk(0.0, tau_im), norm_mode, y, smem);
+    if (o.s < 0) {
+        if (threadIdx.x == 0) atomicCAS(S.status, 0, o.s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
+        return;
+    }
+    for (int j = threadIdx.x; j < mmax; j += blockDim.x) {
+        const size_t k = (size_t)(j + 1) * B + b;
+        const cd v = j < m ? cscale(y[j], S.sc[k]) : cmk(0.0, 0.0);
+        S.yt[2 * k] = v.x;
+        S.yt[2 * k + 1] = v.y;
+    }
+    if (threadIdx.x == 0) erracc[b] += estimate(be[m].x, o.e_m1_m, o.e_m1_mp1);
 }
 
 // psi = sum_j yt_j r_j written over slab 1; ||psi||^2 and <psi0|psi> per
@@ -4463,7 +4459,8 @@ static dq_status enqueue_step(dq_ctx* c, StepTimer* tm, const std::function<void
             enqueue_iteration<Real, TPT>(c, j, tm, 0, bs->chunks);
             if (j >= m_min && j < m && (j - m_min) % kMCheckStride == 0) {
                 mark(DQ_KIND_PADE);
-                k_mcheck_b<<<(B + kPadeWarps - 1) / kPadeWarps, 32 * kPadeWarps, pade_smem_bytes(j + 2), st>>>(j, B, TC, c->tau_im, c->cfg.norm_mode, tol, bs->s);
+                k_mcheck_b<<<B, kPadeThreads, pade_smem_bytes(j + 2), st>>>(j, B, TC, c->tau_im, c->cfg.norm_mode, tol,
+                                                                            bs->s);
                 k_chunk_flags<<<bs->chunks, 64, 0, st>>>(TC, m, 0, bs->s);
             }
         }
@@ -4482,7 +4479,7 @@ static dq_status enqueue_step(dq_ctx* c, StepTimer* tm, const std::function<void
     }
     if (!cluster) {
     mark(DQ_KIND_PADE);
-    k_pade_b<<<(B + kPadeWarps - 1) / kPadeWarps, 32 * kPadeWarps, pade_smem_bytes(m + 2), st>>>(m, B, c->tau_im, c->cfg.norm_mode, bs->s, c->d_erracc);
+    k_pade_b<<<B, kPadeThreads, pade_smem_bytes(m + 2), st>>>(m, B, c->tau_im, c->cfg.norm_mode, bs->s, c->d_erracc);
     mark(DQ_KIND_COMBINE);
     k_combine_b<Real, TPT><<<grid, kBThreads, 0, st>>>(n, B, TC, rpc, m, slabs, se, corr_bra(c), bs->s);
     }
