@@ -83,13 +83,14 @@ struct ClusterArgs {
     const double* b_diag;
     cd tk_coef[kMaxL];        // tau^k / k!
     double* tk_obs;           // [3][B]
-    unsigned char* scratch;   // per chunk, for the dense exponential
-    size_t scratch_stride;
+    int smem;                 // dynamic shared memory of a CTA
+    unsigned char* scratch;   // the dense exponential's matrices where shared memory is too small for them
+    size_t scratch_stride;    // of one CTA that takes trajectories
 };
 
 // Shared memory of a CTA: reductions, the chunk's scalars, the vectors, the records.
 struct ClLayout {
-    size_t ex, red, al, y, par, be, sc, win, prev, d, acc, rec, total;
+    size_t ex, red, al, y, par, be, sc, acc, win, prev, d, rec, total;
 };
 
 static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int m, int rpc, int bw, size_t rsz,
@@ -105,16 +106,28 @@ static __host__ __device__ inline ClLayout cl_layout(int n, int CS, int TC, int 
     L.sc = p; p += sizeof(double) * (m + 2) * TC;
     p = (p + 127) & ~(size_t)127;
     const size_t row = (size_t)TC * 2 * rsz;
+    L.acc = p; p += taylor ? rpc * row : 0;   // the Taylor sum of the own rows
+    p = (p + 15) & ~(size_t)15;
+    // from here on the dense exponential may take the place of everything
     const size_t wide = rpc + 2 * (size_t)bw;   // never more than the rows there are (bw may be n)
     L.win = p; p += (CS > 1 ? (wide < (size_t)n ? wide : (size_t)(n > rpc ? n : rpc)) : rpc) * row;
     L.prev = p; p += rpc * row;
     L.d = p; p += rpc * row / 2;
     p = (p + 15) & ~(size_t)15;
-    L.acc = p; p += taylor ? rpc * row : 0;   // the Taylor sum of the own rows
-    p = (p + 15) & ~(size_t)15;
     L.rec = p; p += rec;
     L.total = (p + 15) & ~(size_t)15;
     return L;
+}
+
+// What a launch carries through its step.
+// (kAdaptive: an ensemble with the adaptive dimension, whose checks stay out of the other kernels' registers)
+enum { kEnsemble = 0, kDropIn = 1, kTaylor = 2, kDropInGrid = 3, kAdaptive = 4 };
+
+// The layout of one of a launch's CTAs.
+template <typename Real, int kMode>
+__device__ __forceinline__ ClLayout cl_shape(const ClusterArgs& A, int CS) {
+    return cl_layout(A.n, kMode == kDropInGrid ? 2 : CS, A.TC, A.m, A.rpc, A.bw, sizeof(Real), A.rec_smem,
+                     kMode == kTaylor);
 }
 
 // Bytes of the block and group starts in front of the records of nb row blocks, `per` to a group.
@@ -159,41 +172,139 @@ __device__ __forceinline__ T cl_load(const T* p, unsigned rank) {
     return v;
 }
 
-// the dense exponential out of line: its registers stay out of the step's
-__device__ __noinline__ PadeOut cl_dense(int m, const cd* al, const cd* be, double tau_im, int norm_mode, cd* y,
-                                         unsigned char* scratch) {
-    return pade_exp_tbar(m, al, be, cmk(0.0, tau_im), norm_mode, y, scratch);
+// Trajectory b's error estimate of the step.
+template <bool kPlain>
+__device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double est) {
+    if (kPlain) {
+        A.ps->err = est;
+        if (A.erracc) *A.erracc += est;
+    } else {
+        A.erracc[b] += est;
+    }
 }
 
-// the same for Taylor-Krylov's augmented matrix: y is its last column
-__device__ __noinline__ PadeOut cl_dense_tk(int mb, int p, const cd* al, const cd* be, double tau_im, int norm_mode,
-                                            cd* y, unsigned char* scratch) {
-    const int L = mb + p;
-    cd* A = reinterpret_cast<cd*>(scratch);
-    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
-        const int i = e / L, j = e % L;
+// The dense exponential of a cluster's trajectories (absolute site energies or
+// long steps).  CTA `rank` takes trajectories rank, rank + CS, ... and works on
+// up to kMaxTeams of them at once, each by its own part of the CTA with its
+// matrices (6 L^2 complex) in the shared memory of the window, the diagonal and
+// the records.  An LU of this size is a chain of small steps with a barrier
+// each, 30 to 60 us for m = 12 to 20 whatever the threads, so trajectories side
+// by side are what counts: one CTA that took all of them in a row, its matrices
+// in global memory, spent 1.08 ms of a step of 1.43 ms (4,731 sites x 100,
+// eight to a cluster of nine CTAs), and 1.6 ms of 2.0 ms at 132 x 4,096, 32 to
+// a CTA.
+// Teams for nt trajectories with matrices of L rows in `room` bytes (0: not even one fits).
+static __host__ __device__ inline int cl_dense_teams(size_t room, int L, int nt) {
+    if (pade_mats_bytes(L) > room) return 0;
+    int teams = 1;
+    while (teams < kMaxTeams && teams < nt && 2 * (size_t)teams * pade_mats_bytes(L) <= room) teams *= 2;
+    return teams;
+}
+// Shared memory from the window on that holds all teams of a CTA, in all at most `room`.
+static __host__ inline size_t cl_dense_bytes(size_t room, int L, int nt) {
+    return cl_dense_teams(room, L, nt) * pade_mats_bytes(L);
+}
+
+// One team's view of that work: its trajectories t = first, first + step, ...
+// < nt of the chunk.
+struct ClDense {
+    const double2* al;        // [j][t]
+    const double* be;
+    const double* sc;
+    const double2* nav;       // [t].x: ||H q_{m+1}||
+    int TC, c0, nt, first, step;
+    WarpsTeam team;
+    unsigned char* mats;
+};
+
+// matrices of at most L rows
+template <typename Real, int kMode>
+__device__ __forceinline__ ClDense cl_dense(const ClusterArgs& A, unsigned char* smem, int chunk, int rank, int CS,
+                                            int L) {
+    const ClLayout Y = cl_shape<Real, kMode>(A, CS);
+    ClDense D;
+    D.al = reinterpret_cast<const double2*>(smem + Y.al);
+    D.be = reinterpret_cast<const double*>(smem + Y.be);
+    D.sc = reinterpret_cast<const double*>(smem + Y.sc);
+    D.nav = reinterpret_cast<const double2*>(smem + Y.par) + 2 * A.TC;
+    D.TC = A.TC;
+    D.c0 = chunk * A.TC;
+    D.nt = min(A.TC, A.B - D.c0);
+    int teams = cl_dense_teams(A.smem - Y.win, L, (D.nt + CS - 1) / CS);
+    D.mats = smem + Y.win;
+    if (teams == 0) {
+        teams = 1;
+        D.mats = A.scratch + ((size_t)chunk * min(CS, A.TC) + min(rank, A.TC - 1)) * A.scratch_stride;
+    }
+    D.team = WarpsTeam{(int)threadIdx.x / (kClThreads / teams), kClThreads / teams};
+    D.mats += D.team.id() * pade_mats_bytes(L);
+    D.first = rank + D.team.id() * CS;
+    D.step = CS * teams;
+    return D;
+}
+
+// exp(tau Tbar) of trajectory t, dimension m with p rows of augmentation
+__device__ __forceinline__ int cl_dense_one(const ClusterArgs& A, const ClDense& D, int t, int m, int p, cd** E) {
+    const int L = m + p;
+    cd* M = reinterpret_cast<cd*>(D.mats);
+    for (int e = D.team.rank(); e < L * L; e += D.team.size()) {
+        const int i = e / L, j = e - i * L;
         cd v = cmk(0.0, 0.0);
-        if (i < mb && j < mb) {
-            if (i == j) v = al[i + 1];
-            else if (j == i + 1) v = be[i + 1];
-            else if (i == j + 1) v = be[j + 1];
-        } else if ((i == 0 && j == mb) || (i >= mb && j == i + 1)) {
+        if (i < m && j < m) {
+            if (i == j) v = cmk(D.al[(i + 1) * D.TC + t].x, D.al[(i + 1) * D.TC + t].y);
+            else if (j == i + 1) v = cmk(D.be[(i + 1) * D.TC + t], 0.0);
+            else if (i == j + 1) v = cmk(D.be[(j + 1) * D.TC + t], 0.0);
+        } else if ((i == 0 && j == m) || (i >= m && j == i + 1)) {
             v = cmk(1.0, 0.0);
         }
-        A[e] = cmul(cmk(0.0, tau_im), v);
+        M[e] = cmul(cmk(0.0, A.tau_im), v);
     }
-    __syncthreads();
-    cd* E = nullptr;
-    PadeOut o;
-    o.s = pade_exp_sm(L, norm_mode, scratch, &E);
-    o.e_m1_m = o.e_m1_mp1 = cmk(0.0, 0.0);
-    if (o.s >= 0) {
-        for (int j = threadIdx.x; j < mb; j += blockDim.x) y[j] = E[j * L + L - 1];
-        o.e_m1_m = E[(mb - 1) * L + mb];
-        o.e_m1_mp1 = E[(mb - 1) * L + mb + 1];
+    D.team.sync();
+    return pade_exp_team(D.team, L, A.norm_mode, D.mats, E);
+}
+
+// The combine weights of the CTA's marked trajectories (mtr = -m), zero from
+// their dimension to mmax, through global memory, and their error estimates.
+// Taylor-Krylov: the last column's times ||A^p psi|| = 1 / sc_1.
+template <typename Real, int kMode>
+__device__ __noinline__ void cl_dense_weights(const ClusterArgs& A, unsigned char* smem, const int* mtr, int chunk,
+                                              int rank, int CS, int mmax) {
+    constexpr bool kTk = kMode == kTaylor, kPlain = kMode == kDropIn || kMode == kDropInGrid;
+    const int p = kTk ? A.tk_p : 2;
+    const ClDense D = cl_dense<Real, kMode>(A, smem, chunk, rank, CS, mmax + p);
+    double* yt = kPlain ? reinterpret_cast<double*>(A.ps->yt) : A.S.yt;   // [j][trajectory]
+    for (int t = D.first; t < D.nt; t += D.step) {
+        if (mtr[t] >= 0) continue;   // uniform over the team
+        const int m = -mtr[t], L = m + p, b = D.c0 + t;
+        cd* E = nullptr;
+        const int s = cl_dense_one(A, D, t, m, p, &E);
+        for (int j = D.team.rank(); j < mmax; j += D.team.size()) {
+            cd v = cmk(0.0, 0.0);
+            if (j < m && s >= 0) {
+                v = E[j * L + (kTk ? L - 1 : 0)];
+                if (kTk) v = cscale(v, 1.0 / D.sc[D.TC + t]);
+                v = cscale(v, D.sc[(j + 1) * D.TC + t]);
+            }
+            double* y = yt + 2 * ((size_t)(j + 1) * A.B + b);
+            y[0] = v.x;
+            y[1] = v.y;
+        }
+        if (D.team.rank() == 0) {
+            if (s < 0) {
+                atomicCAS(A.S.status, 0, s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
+            } else {
+                const double bm = D.be[m * D.TC + t];
+                const cd e1 = E[(m - 1) * L + m], e2 = E[(m - 1) * L + m + 1];
+                // with the adaptive dimension only err1 (||H q_{m+1}|| belongs to the largest m)
+                const double est = kMode == kAdaptive ? fmax(fabs(bm) * sqrt(cabs2(e1)), 1.110223e-16)
+                                                      : expokit_error(bm, D.nav[t].x, e1, e2);
+                if (kTk) A.tk_obs[b] = est;   // completed with the norm
+                else cl_estimate<kPlain>(A, b, est);
+            }
+            if (kMode == kAdaptive) A.S.mtraj[b] = m;
+        }
+        D.team.sync();
     }
-    __syncthreads();
-    return o;
 }
 
 // One CTA's view of its cluster's sums.
@@ -392,6 +503,68 @@ struct ClRecs {
     int lg;
 };
 
+// The records of a CTA's nbo row blocks from kb0 on, copied to `area` where its
+// `room` bytes hold them; all threads of the CTA, which sync before they use them.
+template <typename Real, int R>
+__device__ __forceinline__ ClRecs cl_load_records(unsigned char* area, size_t room, int kb0, int nbo, int TL,
+                                                  const int* gptr, const int* gcol, const void* gcoef) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            ClRecs Q = ClRecs{gptr + kb0, gcol, gcoef, 0u, 0u, nullptr, -1};
+            // block starts, group starts (a group is as long as its longest block), columns (FP64), coefficients
+            const int lg = __ffs(32 / TL) - 1, per = 1 << lg, ng = (nbo + per - 1) >> lg;
+            const size_t head = cl_rec_head(nbo, per);
+            if (head > room) return Q;
+            int* sb = reinterpret_cast<int*>(area);
+            int* sg = sb + nbo + 1;
+            for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(gptr + kb0 + k);
+            __syncthreads();
+            for (int g = warp; g < ng; g += kClWarps) {
+                const int k = (g << lg) + lane;
+                int len = lane < per && k < nbo ? sb[k + 1] - sb[k] : 0;
+                len = __reduce_max_sync(0xffffffffu, len);
+                if (lane == 0) sg[g + 1] = len;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                sg[0] = 0;
+                for (int g = 0; g < ng; ++g) sg[g + 1] += sg[g];
+            }
+            __syncthreads();
+            const size_t slots = (size_t)sg[ng] << lg;
+            const size_t cols = sizeof(Real) == 8 ? (slots * 4 + 15) / 16 * 16 : 0;
+            unsigned char* q = area + head + cols;
+            Q.bptr = sb;
+            if (head + cols + slots * (sizeof(Real) == 8 ? R * 8 : 16) <= room) {
+                int* scol = reinterpret_cast<int*>(area + head);
+                // a warp per block, a lane per entry
+                for (int k = warp; k < nbo; k += kClWarps) {
+                    const int p0 = sb[k], ne = sb[k + 1] - p0, g = sg[k >> lg], i = k & (per - 1);
+                    for (int e = lane; e < ne; e += 32) {
+                        if constexpr (sizeof(Real) == 4) {
+                            reinterpret_cast<float4*>(q)[(g + e) * per + i] =
+                                __ldg(reinterpret_cast<const float4*>(gcoef) + p0 + e);
+                        } else {
+                            const Real* gr = reinterpret_cast<const Real*>(gcoef) + (size_t)(p0 + e) * R;
+                            scol[(g + e) * per + i] = __ldg(gcol + p0 + e);
+                            if constexpr (R == 1) {
+                                reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
+                            } else {
+    #pragma unroll
+                                for (int h = 0; h < R / 2; ++h)
+                                    reinterpret_cast<double2*>(q)[((g + e) * (R / 2) + h) * per + i] =
+                                        __ldg(reinterpret_cast<const double2*>(gr) + h);
+                            }
+                        }
+                    }
+                }
+                Q.scol = sm_addr(scol);
+                Q.srec = sm_addr(q);
+                Q.goff = sg;
+                Q.lg = lg;
+            }
+    return Q;
+}
+
 // Four coupling entries of one row block: column and R coefficients each.
 template <typename Real, int R>
 struct ClRec {
@@ -487,33 +660,129 @@ __device__ __forceinline__ void cl_gather(const ClRecs& Q, int off, int len, uns
     }
 }
 
-// Trajectory b's error estimate of the step.
-template <bool kPlain>
-__device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double est) {
-    if (kPlain) {
-        A.ps->err = est;
-        if (A.erracc) *A.erracc += est;
-    } else {
-        A.erracc[b] += est;
+// Brings back what the dense exponential overwrote after iteration j: the
+// records, the window of r_{j+1} with its margins, r_j and the diagonal, all of
+// which are in global memory too.
+template <typename Real, int TPT, int R>
+__device__ __forceinline__ void cl_restore(const ClusterArgs& A, unsigned char* smem, int chunk, int rank, int CS, int j) {
+    using T = typename VL<Real, TPT>::T;
+    const ClLayout Y = cl_shape<Real, kAdaptive>(A, CS);
+    const int TC = A.TC, TL = TC / TPT, B = A.B, n = A.n, tl = threadIdx.x % TL, RL = kClThreads / TL;
+    const int c0 = chunk * TC, r0 = min(rank * A.rpc, n), nrow = min(n - r0, A.rpc);
+    const int bw = CS == 1 ? 0 : A.bw, hlo = min(bw, r0), hhi = min(bw, n - (r0 + nrow));
+    cl_load_records<Real, R>(smem + Y.rec, (size_t)A.rec_smem, r0 / R, (nrow + R - 1) / R, TL, A.bptr, A.bcol, A.bcoef);
+    if (c0 + tl * TPT < B) {
+        const int tca = min(TC, B - c0);
+        const Real* slabs = reinterpret_cast<const Real*>(A.slabs);
+        // this thread's trajectories on site g of slab q: [chunk][site][trajectory of the chunk], slab 1 plain
+        auto at = [&](int q, int g) {
+            const size_t x = q == 1 ? (size_t)g * B + c0 : (size_t)c0 * n + (size_t)g * tca;
+            return __ldcg(reinterpret_cast<const T*>(slabs + 2 * (A.slab * q + x)) + tl);
+        };
+        T* win = reinterpret_cast<T*>(smem + Y.win);
+        T* prev = reinterpret_cast<T*>(smem + Y.prev);
+        Real* dsm = reinterpret_cast<Real*>(smem + Y.d);
+        const Real* dg = reinterpret_cast<const Real*>(A.diag);
+        for (int h = threadIdx.x / TL; h < hlo + nrow + hhi; h += RL) {
+            const int row = h - hlo, g = r0 + row;
+            win[(size_t)h * TL + tl] = at(j + 1, g);
+            if (row < 0 || row >= nrow) continue;
+            prev[(size_t)row * TL + tl] = at(j, g);
+#pragma unroll
+            for (int t = 0; t < TPT; ++t) dsm[(size_t)row * TC + tl * TPT + t] = dg[(size_t)g * B + c0 + tl * TPT + t];
+        }
     }
+    __syncthreads();
 }
 
-// What a launch carries through its step.
-enum { kEnsemble = 0, kDropIn = 1, kTaylor = 2, kDropInGrid = 3 };
+// A CTA's words shared by its threads: a chunk's choices of the adaptive
+// dimension (elsewhere marks of the trajectories whose exponential is dense),
+// whether there are any, and whether it gave up waiting.
+struct ClWords {
+    int mtr[kMaxTC];
+    int flag, dead;
+};
 
-template <typename Real, int TPT, int R, bool kLocal, int kMode = kEnsemble>
-__global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArgs A) {
+// The adaptive dimension's check after iteration j: EXPOKIT's first term of the
+// nt trajectories' undecided ones, a warp each.  Returns, to every thread of the
+// CTA, whether some need the dense form (the CTA syncs before the next call).
+__device__ __forceinline__ bool cl_series_check(const ClusterArgs& A, const double2* al, const double* be, ClWords& W,
+                                                int nt, int j) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) W.flag = 0;
+    __syncthreads();
+    bool dense = false;
+    for (int t = warp; t < nt; t += kClWarps) {
+        if (W.mtr[t]) continue;
+        const int q = (min(lane, j - 1) + 1) * A.TC + t;
+        cd y, f1, f2;
+        int s;
+        const bool ok = series_exp_tbar(j, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
+        if (ok && s >= 0 && lane == j - 1 && fabs(be[q]) * sqrt(cabs2(f1)) <= A.tol) W.mtr[t] = j;
+        dense = dense || !ok;
+    }
+    if (dense && lane == 0) atomicOr(&W.flag, 1);
+    __syncthreads();
+    return W.flag != 0;
+}
+
+// The whole check, dense forms included; every CTA of the cluster decides
+// alike.  Returns whether all trajectories of the chunk have chosen.
+template <typename Real, int TPT, int R>
+__device__ __noinline__ bool cl_check(const ClusterArgs& A, unsigned char* smem, ClWords& W, int chunk, int rank,
+                                      int CS, int j) {
+    int* mtr = W.mtr;
+    const ClLayout Y = cl_shape<Real, kAdaptive>(A, CS);
+    const double2* al = reinterpret_cast<const double2*>(smem + Y.al);
+    const double* be = reinterpret_cast<const double*>(smem + Y.be);
+    const int TC = A.TC, c0 = chunk * TC, nt = min(TC, A.B - c0);
+    auto sync = [&]() {
+        if (CS == 1) __syncthreads();
+        else cl_sync();
+    };
+    const bool dense = cl_series_check(A, al, be, W, nt, j);
+    if (dense) {
+        // each CTA its own trajectories, the choices, made before or now, through global memory
+        sync();   // the neighbours have their margins from this CTA's window
+        const ClDense D = cl_dense<Real, kAdaptive>(A, smem, chunk, rank, CS, j + 2);
+        for (int t = D.first; t < D.nt; t += D.step) {
+            int choice = mtr[t];
+            if (choice == 0) {
+                cd* E = nullptr;
+                const int s = cl_dense_one(A, D, t, j, 2, &E);
+                if (s >= 0 && fabs(D.be[j * D.TC + t]) * sqrt(cabs2(E[(j - 1) * (j + 2) + j])) <= A.tol) choice = j;
+                D.team.sync();
+            }
+            if (D.team.rank() == 0) A.S.mtraj[c0 + t] = choice;
+        }
+        sync();
+        if ((int)threadIdx.x < nt) mtr[threadIdx.x] = A.S.mtraj[c0 + threadIdx.x];
+        sync();   // the choices may be written again only after all have read them
+    }
+    bool done = true;
+    for (int t = 0; t < nt; ++t) done = done && mtr[t] != 0;
+    if (dense && !done) cl_restore<Real, TPT, R>(A, smem, chunk, rank, CS, j);
+    return done;
+}
+
+// A launch's whole work.  An ensemble with the adaptive dimension whose check
+// needs the dense exponential leaves at that iteration (its number is
+// returned, else 0) and comes back in here as kResume from it.  The two are
+// copies of the code because the loop has few registers to spare: with the
+// dense check's call in it a step takes 8 to 13 % longer (600 sites x 1024 FP64:
+// 329 us, 301 without), with the second copy out of line 4 %.
+template <typename Real, int TPT, int R, bool kLocal, int kMode, bool kResume>
+__device__ __forceinline__ int cl_step(const ClusterArgs& A, unsigned char* smem, ClWords& W, int resume) {
     constexpr bool kGrid = kMode == kDropInGrid, kPlain = kMode == kDropIn || kGrid, kTk = kMode == kTaylor;
+    constexpr bool adaptive = kMode == kAdaptive, kEns = kMode == kEnsemble || adaptive;
     using T = typename VL<Real, TPT>::T;
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int mtr[kMaxTC];
-    __shared__ int flag;   // some trajectory's exponential needs the dense form
+    int* mtr = W.mtr;
+    int& flag = W.flag;
     const int TC = A.TC, TL = TC / TPT, B = A.B, n = A.n;
-    __shared__ int dead;
     const int CS = kLocal ? 1 : kGrid ? (int)gridDim.x : (int)cl_size();
     const unsigned rank = kLocal ? 0u : kGrid ? blockIdx.x : cl_rank();
     const int bw = kLocal ? 0 : A.bw;
-    const ClLayout Y = cl_layout(n, kGrid ? 2 : CS, TC, A.m, A.rpc, bw, sizeof(Real), A.rec_smem, kTk);
+    const ClLayout Y = cl_shape<Real, kMode>(A, CS);
     double2* al = reinterpret_cast<double2*>(smem + Y.al);     // [j][t]
     double2* yts = reinterpret_cast<double2*>(smem + Y.y);     // [j - 1][t]
     // [0][t] the update's coefficients, [1][t] (sc_j, the factor of r_{j-1}), [2][t] complex64: Im alpha's low part
@@ -527,7 +796,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     auto make_sum = [&]() {
         double2* ex = reinterpret_cast<double2*>(smem + Y.ex);
         double2* red = reinterpret_cast<double2*>(smem + Y.red);
-        if constexpr (kGrid) return ClGridSum{ex, red, A.grid, A.S.status, &dead, CS, rank, 0u, 0};
+        if constexpr (kGrid) return ClGridSum{ex, red, A.grid, A.S.status, &W.dead, CS, rank, 0u, 0};
         else return ClSum<TPT, kLocal>{ex, red, TC, CS, rank, (int)threadIdx.x % TC, (int)threadIdx.x / TC};
     };
     auto sum = make_sum();
@@ -559,65 +828,13 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     const int kb0 = r0 / R, nbo = (nrow + R - 1) / R;
     ClRecs Q;
     auto load_records = [&](const int* gptr, const int* gcol, const void* gcoef) {
-        Q = ClRecs{gptr + kb0, gcol, gcoef, 0u, 0u, nullptr, -1};
-        // block starts, group starts (a group is as long as its longest block), columns (FP64), coefficients
-        const int lg = __ffs(32 / TL) - 1, per = 1 << lg, ng = (nbo + per - 1) >> lg;
-        const size_t head = cl_rec_head(nbo, per);
-        if (head > (size_t)A.rec_smem) return;
-        int* sb = reinterpret_cast<int*>(smem + Y.rec);
-        int* sg = sb + nbo + 1;
-        for (int k = threadIdx.x; k <= nbo; k += kClThreads) sb[k] = __ldg(gptr + kb0 + k);
-        __syncthreads();
-        for (int g = warp; g < ng; g += kClWarps) {
-            const int k = (g << lg) + lane;
-            int len = lane < per && k < nbo ? sb[k + 1] - sb[k] : 0;
-            len = __reduce_max_sync(0xffffffffu, len);
-            if (lane == 0) sg[g + 1] = len;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            sg[0] = 0;
-            for (int g = 0; g < ng; ++g) sg[g + 1] += sg[g];
-        }
-        __syncthreads();
-        const size_t slots = (size_t)sg[ng] << lg;
-        const size_t cols = sizeof(Real) == 8 ? (slots * 4 + 15) / 16 * 16 : 0;
-        unsigned char* q = smem + Y.rec + head + cols;
-        Q.bptr = sb;
-        if (head + cols + slots * (sizeof(Real) == 8 ? R * 8 : 16) <= (size_t)A.rec_smem) {
-            int* scol = reinterpret_cast<int*>(smem + Y.rec + head);
-            // a warp per block, a lane per entry
-            for (int k = warp; k < nbo; k += kClWarps) {
-                const int p0 = sb[k], ne = sb[k + 1] - p0, g = sg[k >> lg], i = k & (per - 1);
-                for (int e = lane; e < ne; e += 32) {
-                    if constexpr (sizeof(Real) == 4) {
-                        reinterpret_cast<float4*>(q)[(g + e) * per + i] =
-                            __ldg(reinterpret_cast<const float4*>(gcoef) + p0 + e);
-                    } else {
-                        const Real* gr = reinterpret_cast<const Real*>(gcoef) + (size_t)(p0 + e) * R;
-                        scol[(g + e) * per + i] = __ldg(gcol + p0 + e);
-                        if constexpr (R == 1) {
-                            reinterpret_cast<Real*>(q)[(g + e) * per + i] = __ldg(gr);
-                        } else {
-#pragma unroll
-                            for (int h = 0; h < R / 2; ++h)
-                                reinterpret_cast<double2*>(q)[((g + e) * (R / 2) + h) * per + i] =
-                                    __ldg(reinterpret_cast<const double2*>(gr) + h);
-                        }
-                    }
-                }
-            }
-            Q.scol = sm_addr(scol);
-            Q.srec = sm_addr(q);
-            Q.goff = sg;
-            Q.lg = lg;
-        }
+        Q = cl_load_records<Real, R>(smem + Y.rec, (size_t)A.rec_smem, kb0, nbo, TL, gptr, gcol, gcoef);
     };
     load_records(A.bptr, A.bcol, A.bcoef);
 
     // ---- r_1 = psi over the window, the diagonal (noise of this step, or as it is)
-    if (act) {
-        const int step = kMode != kEnsemble ? A.step : *A.S.step;
+    if (!kResume && act) {
+        const int step = kEns ? *A.S.step : A.step;
         const double* D = A.noise == DQ_NOISE_ZZ && (A.flags & kClNoise)
                               ? A.zzD + (size_t)(step - *A.zz_start) * n * B : nullptr;
         Real* dg = reinterpret_cast<Real*>(A.diag);
@@ -667,14 +884,14 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             }
         }
     }
-    if (threadIdx.x < TC) {
+    if (!kResume && threadIdx.x < TC) {
         const double s1 = kPlain || kTk ? 1.0 : c0 + (int)threadIdx.x < B ? A.S.sc[(size_t)B + c0 + threadIdx.x] : 0.0;
         scs[TC + threadIdx.x] = s1;
         par[TC + threadIdx.x] = make_double2(s1, 0.0);
         mtr[threadIdx.x] = 0;
     }
     if constexpr (kGrid) {
-        if (threadIdx.x == 0) dead = 0;
+        if (threadIdx.x == 0) W.dead = 0;
         __syncthreads();
     } else {
         sum.sync();   // every CTA of the cluster runs; the window is in place
@@ -733,7 +950,6 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     };
 
-    const bool adaptive = kMode == kEnsemble && A.S.mtraj != nullptr;
     // the last warp's lanes take the sums' scalars: the margins' loads start with the first warps
     const int last = warp == kClWarps - 1 ? lane : kMaxTC;
     if constexpr (kTk) {
@@ -789,7 +1005,16 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         }
     }
     int jl = A.m;   // iterations done
-    for (int j = 1; j <= A.m; ++j) {
+    int j0 = 1;
+    if constexpr (kResume) {
+        // the check that the first pass left at
+        j0 = resume + 1;
+        if (cl_check<Real, TPT, R>(A, smem, W, chunk, (int)rank, CS, resume)) {
+            jl = resume;
+            j0 = A.m + 1;
+        }
+    }
+    for (int j = j0; j <= A.m; ++j) {
         // u = H r_j - (beta_{j-1} sc_{j-1} / sc_j) r_{j-1} over r_{j-1} (w = sc_j u); alpha_j
         double x2[TPT], y2[TPT], sc[TPT];
         Real fm[TPT];
@@ -815,7 +1040,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
                 for (int t = 0; t < TPT; ++t) {
                     const Real dv = dsm[l + t];
                     Real ur = acc[i].v[2 * t], ui = acc[i].v[2 * t + 1];
-                    if constexpr (kMode != kEnsemble) {
+                    if constexpr (!kEns) {
                         // the reference's order: alpha_j from H q_j alone (the unconjugated dot of
                         // complex states does not make q_j orthogonal to q_{j-1})
                         ur = fma(dv, x.v[2 * t], ur);
@@ -931,46 +1156,18 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
         margins(j + 1);
         __syncthreads();
         if (adaptive && j >= A.m_min && j < A.m && (j - A.m_min) % kMCheckStride == 0) {
-            // EXPOKIT's first term per undecided trajectory; every CTA decides alike
-            if (threadIdx.x == 0) flag = 0;
-            __syncthreads();
-            for (int t = warp; t < TC; t += kClWarps) {
-                if (c0 + t >= B || mtr[t]) continue;
-                const int q = (min(lane, j - 1) + 1) * TC + t;
-                cd y, f1, f2;
-                int s;
-                const bool ok = series_exp_tbar(j, cmk(al[q].x, al[q].y), be[q], A.tau_im, A.norm_mode, y, f1, f2, s);
-                if (ok && s >= 0 && lane == j - 1 && fabs(be[q]) * sqrt(cabs2(f1)) <= A.tol) mtr[t] = j;
-                if (!ok && lane == 0) atomicOr(&flag, 1);
-            }
-            __syncthreads();
-            if (flag) {
-                // the dense form on rank 0, the choices through global memory
-                __shared__ cd ald[kMaxL], bed[kMaxL];
-                if (rank == 0) {
-                    for (int t = 0; t < TC && c0 + t < B; ++t) {
-                        int mt = mtr[t];
-                        __syncthreads();
-                        if (mt == 0) {
-                            for (int i = threadIdx.x; i <= j + 1; i += kClThreads) {
-                                ald[i] = i >= 1 && i <= j ? cmk(al[i * TC + t].x, al[i * TC + t].y) : cmk(0, 0);
-                                bed[i] = i >= 1 && i <= j ? cmk(be[i * TC + t], 0.0) : cmk(0, 0);
-                            }
-                            __syncthreads();
-                            const PadeOut o = cl_dense(j, ald, bed, A.tau_im, A.norm_mode, nullptr,
-                                                       A.scratch + chunk * A.scratch_stride);
-                            if (o.s >= 0 && fabs(bed[j].x) * sqrt(cabs2(o.e_m1_m)) <= A.tol) mt = j;
-                            __syncthreads();
-                        }
-                        if (threadIdx.x == 0) A.S.mtraj[c0 + t] = mt;
-                    }
+            bool done;
+            if constexpr (kResume) {
+                done = cl_check<Real, TPT, R>(A, smem, W, chunk, (int)rank, CS, j);
+            } else {
+                const int nt = min(TC, B - c0);
+                if (cl_series_check(A, al, be, W, nt, j)) {
+                    __syncthreads();   // all have read the flag
+                    return j;
                 }
-                sum.sync();
-                if (threadIdx.x < TC && c0 + (int)threadIdx.x < B) mtr[threadIdx.x] = A.S.mtraj[c0 + threadIdx.x];
-                sum.sync();   // rank 0 may write the choices again only after all have read them
+                static_assert(kMaxTC <= 64, "two trajectories a lane");
+                done = __all_sync(0xffffffffu, (lane >= nt || mtr[lane] != 0) && (lane + 32 >= nt || mtr[lane + 32] != 0));
             }
-            bool done = true;
-            for (int t = 0; t < TC && c0 + t < B; ++t) done = done && mtr[t] != 0;
             if (done) {
                 jl = j;
                 break;
@@ -979,7 +1176,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     // ---- the recurrence's scalars (the adjoint and the getters read them) ----
     __syncthreads();
-    if (kMode == kEnsemble && rank == 0) {
+    if (kEns && rank == 0) {
         for (int e = threadIdx.x; e < jl * TC; e += kClThreads) {
             const int j = 1 + e / TC, t = e % TC;
             if (c0 + t >= B) continue;
@@ -993,7 +1190,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     if (!(A.flags & kClFinish)) {
         // the neighbours may still read this CTA's rows of the last window
         if constexpr (!kLocal && !kGrid) cl_sync();
-        return;
+        return 0;
     }
     // ---- ||H q_{m+1}|| ---------------------------------------------------------
     double nav = 0.0;   // set where it is used, per trajectory
@@ -1067,42 +1264,11 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
     }
     __syncthreads();
     if (flag) {
-        __shared__ cd ald[kMaxL], bed[kMaxL], yd[kMaxM];
-        if (rank == 0) {
-            for (int t = 0; t < TC && c0 + t < B; ++t) {
-                if (mtr[t] >= 0) continue;
-                const int m = -mtr[t];
-                for (int i = threadIdx.x; i <= m + 1; i += kClThreads) {
-                    ald[i] = i >= 1 && i <= m ? cmk(al[i * TC + t].x, al[i * TC + t].y) : cmk(0, 0);
-                    bed[i] = i >= 1 && i <= m ? cmk(be[i * TC + t], 0.0) : cmk(0, 0);
-                }
-                __syncthreads();
-                PadeOut o;
-                if constexpr (kTk) {
-                    o = cl_dense_tk(m, A.tk_p, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
-                    for (int j = threadIdx.x; j < m; j += kClThreads) yd[j] = cscale(yd[j], 1.0 / scs[TC + t]);
-                } else {
-                    o = cl_dense(m, ald, bed, A.tau_im, A.norm_mode, yd, A.scratch + chunk * A.scratch_stride);
-                }
-                __syncthreads();
-                if (o.s < 0 && threadIdx.x == 0)
-                    atomicCAS(A.S.status, 0, o.s == -1 ? DQ_ERR_SCALING : DQ_ERR_SINGULAR);
-                for (int j = threadIdx.x; j < mmax; j += kClThreads) {
-                    const cd v = j < m && o.s >= 0 ? cscale(yd[j], scs[(j + 1) * TC + t]) : cmk(0.0, 0.0);
-                    const size_t k = (size_t)(j + 1) * B + c0 + t;
-                    double* yt = kPlain ? reinterpret_cast<double*>(A.ps->yt) : A.S.yt;   // [j][trajectory]
-                    yt[2 * k] = v.x;
-                    yt[2 * k + 1] = v.y;
-                }
-                if (threadIdx.x == 0 && o.s >= 0) {
-                    if (!adaptive) nav = sqrt(sum.get(0, t).x) * scs[(A.m + 1) * TC + t];
-                    if constexpr (kTk) A.tk_obs[c0 + t] = estimate(m, t, o.e_m1_m, o.e_m1_mp1);
-                    else cl_estimate<kPlain>(A, c0 + t, estimate(m, t, o.e_m1_m, o.e_m1_mp1));
-                }
-                if (adaptive && threadIdx.x == 0) A.S.mtraj[c0 + t] = m;
-                __syncthreads();
-            }
-        }
+        if constexpr (adaptive) sum.sync();   // as in the check
+        else if (threadIdx.x < TC)
+            par[2 * TC + threadIdx.x].x = sqrt(sum.get(0, threadIdx.x).x) * scs[(A.m + 1) * TC + threadIdx.x];
+        __syncthreads();
+        cl_dense_weights<Real, kMode>(A, smem, mtr, chunk, (int)rank, CS, mmax);
         sum.sync();
         for (int e = threadIdx.x; e < mmax * TC; e += kClThreads) {
             const int j = e / TC, t = e % TC;
@@ -1238,31 +1404,36 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const ClusterArg
             cp[1] = si;
         }
     }
+    return 0;
+}
+
+template <typename Real, int TPT, int R, bool kLocal, int kMode = kEnsemble>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_step(const __grid_constant__ ClusterArgs A) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ ClWords W;
+    const int left = cl_step<Real, TPT, R, kLocal, kMode, false>(A, smem, W, 0);
+    if constexpr (kMode == kAdaptive)
+        if (left) cl_step<Real, TPT, R, kLocal, kAdaptive, true>(A, smem, W, left);
 }
 
 // ---------------------------------------------------------------------------
 using ClKernel = void (*)(const ClusterArgs);
 
-template <typename Real, int TPT>
-static ClKernel cl_pick(int R, bool local) {
-    switch (R) {
-        case 1: return local ? k_cluster_step<Real, TPT, 1, true> : k_cluster_step<Real, TPT, 1, false>;
-        case 2: return local ? k_cluster_step<Real, TPT, 2, true> : k_cluster_step<Real, TPT, 2, false>;
-        case 3:
-            if constexpr (sizeof(Real) == 4)
-                return local ? k_cluster_step<Real, TPT, 3, true> : k_cluster_step<Real, TPT, 3, false>;
-            return nullptr;
-        case 4:
-            if constexpr (sizeof(Real) == 8)
-                return local ? k_cluster_step<Real, TPT, 4, true> : k_cluster_step<Real, TPT, 4, false>;
-            return nullptr;
-        default: return nullptr;
-    }
+template <typename Real, int TPT, int R>
+static ClKernel cl_pick(bool local, bool adaptive) {
+    if (adaptive) return local ? k_cluster_step<Real, TPT, R, true, kAdaptive> : k_cluster_step<Real, TPT, R, false, kAdaptive>;
+    return local ? k_cluster_step<Real, TPT, R, true> : k_cluster_step<Real, TPT, R, false>;
 }
 
-static ClKernel cl_kernel(bool mixed, int tpt, int R, bool local) {
-    if (!mixed) return cl_pick<double, 1>(R, local);
-    return tpt == 2 ? cl_pick<float, 2>(R, local) : nullptr;
+static ClKernel cl_kernel(bool mixed, int tpt, int R, bool local, bool adaptive) {
+    if (mixed && tpt != 2) return nullptr;
+    switch (R) {
+        case 1: return mixed ? cl_pick<float, 2, 1>(local, adaptive) : cl_pick<double, 1, 1>(local, adaptive);
+        case 2: return mixed ? cl_pick<float, 2, 2>(local, adaptive) : cl_pick<double, 1, 2>(local, adaptive);
+        case 3: return mixed ? cl_pick<float, 2, 3>(local, adaptive) : nullptr;
+        case 4: return mixed ? nullptr : cl_pick<double, 1, 4>(local, adaptive);
+        default: return nullptr;
+    }
 }
 
 static const ::BlockFmt& cl_fmt(const BatchedState* bs, int R) {
@@ -1305,7 +1476,7 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
     const int n = c->n, m = c->cfg.m;
     if (CS < 1 || CS > kClMaxCtas) return 0;
     if (tc < tpt || tc > kMaxTC || tc % tpt || ((tc / tpt) & (tc / tpt - 1)) || tc / tpt > 32) return 0;
-    ClKernel k = cl_kernel(bs->mixed, tpt, R, CS == 1);
+    ClKernel k = cl_kernel(bs->mixed, tpt, R, CS == 1, bs->s.mtraj != nullptr);
     if (!k) return 0;
     const size_t rsz = bs->mixed ? sizeof(float) : sizeof(double);
     const int rpc = cl_rows(n, CS, R);
@@ -1316,6 +1487,9 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
         sm = cl_layout(n, CS, tc, m, rpc, c->bw, rsz, 0).total;
     }
     if (sm > kClSmemMax) return 0;
+    // the dense exponential's matrices, in the place of the window and what follows it
+    const size_t win = cl_layout(n, CS, tc, m, rpc, c->bw, rsz, 0).win;
+    sm = std::max(sm, win + cl_dense_bytes(kClSmemMax - win, m + 2, (std::min(tc, bs->B) + CS - 1) / CS));
     int found = 0;
     if (raise_smem_limit(k, (int)kClSmemMax) == cudaSuccess &&
         (CS <= 8 || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
@@ -1417,10 +1591,11 @@ cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
     a.erracc = c->d_erracc;
     a.bra = corr_bra(c);
     a.scratch = static_cast<unsigned char*>(bs->cl_scratch);
-    a.scratch_stride = pade_smem_bytes(c->cfg.m + 2);
+    a.scratch_stride = pade_mats_bytes(c->cfg.m + 2);
+    a.smem = (int)bs->win_smem;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cl_config(bs->chunks, bs->ctas_per_sm, bs->win_smem, c->stream, &at);
-    return cudaLaunchKernelEx(&cfg, cl_kernel(bs->mixed, bs->TPT, bs->R, bs->ctas_per_sm == 1), a);
+    return cudaLaunchKernelEx(&cfg, cl_kernel(bs->mixed, bs->TPT, bs->R, bs->ctas_per_sm == 1, bs->s.mtraj != nullptr), a);
 }
 
 // Shapes `bs` for the cluster form (its coupling blocks of R rows exist).
@@ -1429,7 +1604,9 @@ dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R) {
     size_t smem = 0, rec = 0;
     if (cluster_resident(c, tc, tpt, CS, R, cl_fmt(bs, R), &smem, &rec) < 1) return DQ_ERR_ARG;
     const int chunks = (bs->B + tc - 1) / tc;
-    const size_t need = (size_t)chunks * pade_smem_bytes(c->cfg.m + 2);
+    const size_t win = cl_layout(c->n, CS, tc, c->cfg.m, cl_rows(c->n, CS, R), c->bw,
+                                 bs->mixed ? sizeof(float) : sizeof(double), 0).win;
+    const size_t mats = pade_mats_bytes(c->cfg.m + 2), need = win + mats <= smem ? 0 : mats * chunks * std::min(CS, tc);
     if (need > bs->cl_scratch_bytes) {
         cudaFree(bs->cl_scratch);
         bs->cl_scratch = nullptr;
@@ -1559,7 +1736,7 @@ cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cuda
     a.corr_pt = q.corr_pt;
     a.ps = q.ps;
     a.grid = q.grid;
-    a.scratch = q.scratch;
+    a.smem = (int)P.smem;   // always room for the dense exponential: one trajectory's scalars take 3 KB
     cudaLaunchAttribute at;
     cudaLaunchConfig_t cfg = cl_config(1, P.ctas, P.smem, st, &at);
     if (P.ctas > kClMaxCtas) {
@@ -1596,7 +1773,7 @@ size_t taylor_cluster_head(const TaylorCluster& P) { return cl_rec_head(P.rpc, 3
 // CTAs and trajectories of a cluster for n sites x B trajectories, z couplings
 // per row of the larger matrix and bandwidth bw, by cluster_plan's estimate;
 // ctas = 0: nothing fits.
-TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z) {
+TaylorCluster taylor_cluster_plan(int n, int B, int mb, int p, int bw, double z) {
     TaylorCluster best;
     double t_best = 1e30;
     ClKernel local = k_cluster_step<double, 1, 1, true, kTaylor>, wide = k_cluster_step<double, 1, 1, false, kTaylor>;
@@ -1632,6 +1809,13 @@ TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z) {
                 best = P;
             }
         }
+    }
+    if (best.ctas) {
+        // the dense exponential's matrices: in the place of the window and what follows it, or in global memory
+        const size_t win = cl_layout(n, best.ctas, best.tc, mb, best.rpc, bw, sizeof(double), 0, true).win;
+        const size_t mats = pade_mats_bytes(mb + p);
+        if (win + mats <= kClSmemMax) best.smem = std::max(best.smem, win + mats);
+        else best.scratch = mats * best.chunks * std::min(best.ctas, best.tc);
     }
     return best;
 }
@@ -1682,8 +1866,9 @@ cudaError_t taylor_cluster_launch(const TaylorCluster& P, const TaylorStep& q, c
     a.b_diag = q.b_diag;
     for (int k = 0; k < q.p; ++k) a.tk_coef[k] = q.coef[k];
     a.tk_obs = q.obs;
+    a.smem = (int)P.smem;
     a.scratch = q.scratch;
-    a.scratch_stride = pade_smem_bytes(q.mb + q.p);
+    a.scratch_stride = pade_mats_bytes(q.mb + q.p);
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cl_config(P.chunks, P.ctas, P.smem, st, &at);
     return cudaLaunchKernelEx(&cfg, P.ctas == 1 ? k_cluster_step<double, 1, 1, true, kTaylor>

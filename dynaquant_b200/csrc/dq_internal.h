@@ -79,7 +79,6 @@ struct PlainStep {
     double* pops_row;
     cd* corr_pt;
     const cd* bra;
-    unsigned char* scratch;  // pade_smem_bytes(m + 2)
 };
 
 // A Taylor-Krylov step of an ensemble as one cluster launch: CTAs (0: nothing
@@ -87,6 +86,7 @@ struct PlainStep {
 struct TaylorCluster {
     int ctas = 0, tc = 0, rpc = 0, chunks = 0;
     size_t smem = 0, rec = 0;
+    size_t scratch = 0;      // bytes in global memory for the dense exponential (0: shared memory holds it)
 };
 
 struct TaylorStep {
@@ -110,7 +110,7 @@ struct TaylorStep {
     double* deps;
     double* erracc;
     const cd* bra;
-    unsigned char* scratch;          // chunks x pade_smem_bytes(mb + p)
+    unsigned char* scratch;          // TaylorCluster::scratch bytes
 };
 
 struct BatchedState;   // dq_batched.cu
@@ -169,8 +169,7 @@ struct dq_ctx {
     dq::cd* d_psi_b = nullptr;
     double* d_partial = nullptr;  // kMaxPartials x 2
     dq::PlainScalars* d_ps = nullptr;
-    unsigned char* d_pade = nullptr;       // the one-launch step's dense exponential
-    dq::PlainGrid* d_grid = nullptr;       // and its whole-grid form's barrier
+    dq::PlainGrid* d_grid = nullptr;       // the one-launch step: its whole-grid form's barrier
     dq::PlainCluster plain;                // its shape for the Hamiltonian that is set
 
     // observables (sums over trajectories; divided by n_traj on read)
@@ -256,7 +255,7 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
 cudaError_t plain_cluster_attributes();
 bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P);
 size_t taylor_cluster_head(const TaylorCluster& P);
-TaylorCluster taylor_cluster_plan(int n, int B, int mb, int bw, double z);
+TaylorCluster taylor_cluster_plan(int n, int B, int mb, int p, int bw, double z);
 cudaError_t taylor_cluster_launch(const TaylorCluster& P, const TaylorStep& q, cudaStream_t st);
 cudaError_t plain_cluster_launch(const PlainCluster& P, const PlainStep& q, cudaStream_t st);
 // implemented in dq_batched.cu

@@ -33,17 +33,39 @@ __host__ __device__ inline PadeCoeffs pade_coeffs() {
     return P;
 }
 
-__host__ __device__ inline size_t pade_smem_bytes(int L) { return sizeof(cd) * 6 * (size_t)L * L + 64 * sizeof(double); }
+// The threads that work on one matrix: a CTA, or one of up to kMaxTeams parts
+// of a CTA (whole warps, `size` threads each) with a named barrier of its own,
+// so that a CTA can take several matrices at once.
+constexpr int kMaxTeams = 8;
+struct CtaTeam {
+    __device__ __forceinline__ int id() const { return 0; }
+    __device__ __forceinline__ int rank() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct WarpsTeam {
+    int id_, size_;
+    __device__ __forceinline__ int id() const { return id_; }
+    __device__ __forceinline__ int rank() const { return threadIdx.x - id_ * size_; }
+    __device__ __forceinline__ int size() const { return size_; }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("barrier.sync %0, %1;" ::"r"(id_ + 1), "r"(size_) : "memory");
+    }
+};
 
-// C = A * B (L x L row-major, shared memory), all threads of the CTA.
-__device__ __forceinline__ void sm_matmul(int L, const cd* A, const cd* B, cd* C) {
-    for (int e = threadIdx.x; e < L * L; e += blockDim.x) {
+__host__ __device__ inline size_t pade_mats_bytes(int L) { return sizeof(cd) * 6 * (size_t)L * L; }
+__host__ __device__ inline size_t pade_smem_bytes(int L) { return pade_mats_bytes(L) + 64 * sizeof(double); }
+
+// C = A * B (L x L row-major, shared memory), all threads of the team.
+template <class Team>
+__device__ __forceinline__ void sm_matmul(const Team& T, int L, const cd* A, const cd* B, cd* C) {
+    for (int e = T.rank(); e < L * L; e += T.size()) {
         int i = e / L, j = e - i * L;
         cd s = cmk(0, 0);
         for (int k = 0; k < L; ++k) s = cadd(s, cmul(A[i * L + k], B[k * L + j]));
         C[e] = s;
     }
-    __syncthreads();
+    T.sync();
 }
 
 struct PadeOut {
@@ -53,13 +75,14 @@ struct PadeOut {
 };
 
 // E = exp(A) for the L x L complex matrix A held in the first L*L entries of
-// smem_raw (6 L^2 complex + 64 doubles of shared memory): Padé(6,6) in the
-// odd/even form with scaling by the row-sum infinity norm (norm_mode 0:
-// |Re|-only sums as padeClass.cu:585-706; 1: complex modulus) and repeated
-// squaring.  Returns the number of squarings s (or -1 when s would reach 50,
+// smem_raw (6 L^2 complex values): Padé(6,6) in the odd/even form with scaling
+// by the row-sum infinity norm (norm_mode 0: |Re|-only sums as
+// padeClass.cu:585-706; 1: complex modulus) and repeated squaring.  Returns the number of squarings s (or -1 when s would reach 50,
 // -2 for a singular quotient) and sets *E_out to the result (A itself or the
-// second buffer).  All threads of the CTA call it and all return s.
-__device__ inline int pade_exp_sm(int L, int norm_mode, unsigned char* smem_raw, cd** E_out) {
+// second buffer).  All threads of the team call it and all return s; the team
+// syncs before its next call.
+template <class Team>
+__device__ __forceinline__ int pade_exp_team(const Team& T, int L, int norm_mode, unsigned char* smem_raw, cd** E_out) {
     const int LL = L * L;
     cd* A = reinterpret_cast<cd*>(smem_raw);
     cd* A2 = A + LL;
@@ -67,18 +90,20 @@ __device__ inline int pade_exp_sm(int L, int norm_mode, unsigned char* smem_raw,
     cd* A6 = A4 + LL;
     cd* U = A6 + LL;
     cd* D = U + LL;
-    __shared__ int s_sh;
-    __shared__ int piv_sh;
-    __shared__ int fail_sh;
+    __shared__ int sh[kMaxTeams][3];
+    int& s_sh = sh[T.id()][0];
+    int& piv_sh = sh[T.id()][1];
+    int& fail_sh = sh[T.id()][2];
+    const int rank = T.rank(), size = T.size();
 
     const PadeCoeffs P = pade_coeffs();
-    if (threadIdx.x == 0) fail_sh = 0;
-    __syncthreads();
+    if (rank == 0) fail_sh = 0;
+    T.sync();
 
     // scaling: s = number of halvings until the row-sum norm is <= 0.5
-    if (threadIdx.x < 32) {
+    if (rank < 32) {
         double mx = 0.0;
-        for (int i = threadIdx.x; i < L; i += 32) {
+        for (int i = rank; i < L; i += 32) {
             double rs = 0.0;
             for (int j = 0; j < L; ++j) {
                 cd a = A[i * L + j];
@@ -88,50 +113,50 @@ __device__ inline int pade_exp_sm(int L, int norm_mode, unsigned char* smem_raw,
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (threadIdx.x == 0) {
+        if (rank == 0) {
             int s = 0;
             double nrm = mx;
             while (nrm > 0.5 && s < 60) { nrm *= 0.5; s++; }
             s_sh = s;
         }
     }
-    __syncthreads();
+    T.sync();
     const int s = s_sh;
     *E_out = A;
     if (s >= 50) return -1;
     if (s > 0) {
         double sc = ldexp(1.0, -s);
-        for (int e = threadIdx.x; e < LL; e += blockDim.x) A[e] = cscale(A[e], sc);
-        __syncthreads();
+        for (int e = rank; e < LL; e += size) A[e] = cscale(A[e], sc);
+        T.sync();
     }
-    sm_matmul(L, A, A, A2);
-    sm_matmul(L, A2, A2, A4);
-    sm_matmul(L, A2, A4, A6);
+    sm_matmul(T, L, A, A, A2);
+    sm_matmul(T, L, A2, A2, A4);
+    sm_matmul(T, L, A2, A4, A6);
     // odd part U = A (c1 I + c3 A^2 + c5 A^4); the bracket goes to D first
-    for (int e = threadIdx.x; e < LL; e += blockDim.x) {
+    for (int e = rank; e < LL; e += size) {
         int i = e / L, j = e - i * L;
         cd t = cadd(cscale(A2[e], P.c[3]), cscale(A4[e], P.c[5]));
         if (i == j) t.x += P.c[1];
         D[e] = t;
     }
-    __syncthreads();
-    sm_matmul(L, A, D, U);
+    T.sync();
+    sm_matmul(T, L, A, D, U);
     // even part V = c0 I + c2 A^2 + c4 A^4 + c6 A^6; D = V - U
-    for (int e = threadIdx.x; e < LL; e += blockDim.x) {
+    for (int e = rank; e < LL; e += size) {
         int i = e / L, j = e - i * L;
         cd t = cadd(cadd(cscale(A2[e], P.c[2]), cscale(A4[e], P.c[4])), cscale(A6[e], P.c[6]));
         if (i == j) t.x += P.c[0];
         D[e] = csub(t, U[e]);
     }
-    __syncthreads();
+    T.sync();
 
     // LU with partial pivoting: D X = U, X overwrites U (stands in for
     // culaDeviceZgesv, padeClass.cu:715-745)
     for (int k = 0; k < L; ++k) {
-        if (threadIdx.x < 32) {
+        if (rank < 32) {
             double best = -1.0;
             int bi = k;
-            for (int i = k + threadIdx.x; i < L; i += 32) {
+            for (int i = k + rank; i < L; i += 32) {
                 double v = cabs2(D[i * L + k]);
                 if (v > best) { best = v; bi = i; }
             }
@@ -141,60 +166,64 @@ __device__ inline int pade_exp_sm(int L, int norm_mode, unsigned char* smem_raw,
                 int oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
             }
-            if (threadIdx.x == 0) {
+            if (rank == 0) {
                 piv_sh = bi;
                 if (best == 0.0) fail_sh = 1;
             }
         }
-        __syncthreads();
+        T.sync();
         if (fail_sh) break;
         const int p = piv_sh;
         if (p != k) {
-            for (int j = threadIdx.x; j < L; j += blockDim.x) {
+            for (int j = rank; j < L; j += size) {
                 cd t = D[k * L + j]; D[k * L + j] = D[p * L + j]; D[p * L + j] = t;
                 t = U[k * L + j]; U[k * L + j] = U[p * L + j]; U[p * L + j] = t;
             }
-            __syncthreads();
+            T.sync();
         }
         const cd inv = cdiv(cmk(1.0, 0.0), D[k * L + k]);
         // multipliers into column k below the pivot
-        for (int i = k + 1 + threadIdx.x; i < L; i += blockDim.x) D[i * L + k] = cmul(D[i * L + k], inv);
-        __syncthreads();
+        for (int i = k + 1 + rank; i < L; i += size) D[i * L + k] = cmul(D[i * L + k], inv);
+        T.sync();
         const int rows = L - k - 1;
-        for (int e = threadIdx.x; e < rows * L; e += blockDim.x) {
+        for (int e = rank; e < rows * L; e += size) {
             int i = k + 1 + e / L, j = e % L;
             cd f = D[i * L + k];
             if (j > k) D[i * L + j] = csub(D[i * L + j], cmul(f, D[k * L + j]));
             U[i * L + j] = csub(U[i * L + j], cmul(f, U[k * L + j]));
         }
-        __syncthreads();
+        T.sync();
     }
     if (fail_sh) return -2;
     for (int k = L - 1; k >= 0; --k) {
         const cd inv = cdiv(cmk(1.0, 0.0), D[k * L + k]);
-        for (int j = threadIdx.x; j < L; j += blockDim.x) {
+        for (int j = rank; j < L; j += size) {
             cd acc = U[k * L + j];
             for (int c = k + 1; c < L; ++c) acc = csub(acc, cmul(D[k * L + c], U[c * L + j]));
             U[k * L + j] = cmul(acc, inv);
         }
-        __syncthreads();
+        T.sync();
     }
     // E = I + 2X
     cd* E = A;
-    for (int e = threadIdx.x; e < LL; e += blockDim.x) {
+    for (int e = rank; e < LL; e += size) {
         int i = e / L, j = e - i * L;
         cd t = cscale(U[e], 2.0);
         if (i == j) t.x += 1.0;
         E[e] = t;
     }
-    __syncthreads();
+    T.sync();
     cd* Tmp = A2;
     for (int k = 0; k < s; ++k) {
-        sm_matmul(L, E, E, Tmp);
+        sm_matmul(T, L, E, E, Tmp);
         cd* sw = E; E = Tmp; Tmp = sw;
     }
     *E_out = E;
     return s;
+}
+
+__device__ inline int pade_exp_sm(int L, int norm_mode, unsigned char* smem_raw, cd** E_out) {
+    return pade_exp_team(CtaTeam{}, L, norm_mode, smem_raw, E_out);
 }
 
 // Computes E = exp(tau * Tbar) for Tbar built from alpha[1..m], beta[1..m]

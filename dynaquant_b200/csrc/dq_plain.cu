@@ -516,7 +516,6 @@ dq_status plain_alloc(dq_ctx* c) {
     DQ_CU(cudaMalloc(&c->d_psi_b, sizeof(cd) * n));
     DQ_CU(cudaMalloc(&c->d_partial, sizeof(double) * 2 * kMaxPartials));
     DQ_CU(cudaMalloc(&c->d_ps, sizeof(PlainScalars)));
-    DQ_CU(cudaMalloc(&c->d_pade, pade_smem_bytes(m + 2)));
     DQ_CU(cudaMalloc(&c->d_grid, sizeof(PlainGrid)));
     DQ_CU(cudaMemsetAsync(c->d_grid, 0, sizeof(PlainGrid), c->stream));
     DQ_CU(cudaMemsetAsync(c->d_ps, 0, sizeof(PlainScalars), c->stream));
@@ -534,9 +533,8 @@ dq_status plain_alloc(dq_ctx* c) {
 
 void plain_free(dq_ctx* c) {
     cudaFree(c->d_eps_p); cudaFree(c->d_deps_p); cudaFree(c->d_diag); cudaFree(c->d_Q); cudaFree(c->d_w);
-    cudaFree(c->d_psi_a); cudaFree(c->d_psi_b); cudaFree(c->d_partial); cudaFree(c->d_ps); cudaFree(c->d_pade);
+    cudaFree(c->d_psi_a); cudaFree(c->d_psi_b); cudaFree(c->d_partial); cudaFree(c->d_ps);
     cudaFree(c->d_grid);
-    c->d_pade = nullptr;
     c->d_grid = nullptr;
     c->d_eps_p = c->d_deps_p = c->d_diag = c->d_partial = nullptr;
     c->d_Q = c->d_w = c->d_psi_a = c->d_psi_b = nullptr;
@@ -673,7 +671,6 @@ dq_status plain_step(dq_ctx* c, int traj, int step, const cd* psi_in, cd* psi_ou
         q.pops_row = (observe && rec >= 0) ? c->d_pops + (size_t)rec * n : nullptr;
         q.corr_pt = observe ? c->d_corr + (step + 1) : nullptr;
         q.bra = corr_bra(c);
-        q.scratch = c->d_pade;
         DQ_CU(plain_cluster_launch(c->plain, q, st));
         if (observe && c->ipr_on) k_ipr_plain<<<G, T, 0, st>>>(n, psi_out, c->d_ipr + step + 1, c->d_partial, c->d_ps);
         DQ_CU(cudaGetLastError());
@@ -812,11 +809,9 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
     const size_t off_w = off_partial + align256(sizeof(double) * 2 * kMaxPartials);
     const size_t off_q = off_w + align256(sizeof(cd) * (size_t)n);
     const size_t need = off_q + sizeof(cd) * (size_t)n * (size_t)(m + 2);
-    // one launch where the whole vector fits every CTA's window (the columns are known on the device
-    // only) and the dense exponential's matrices the rest of the array
-    const size_t off_pade = align256(need);
+    // one launch where the whole vector fits every CTA's window (the columns are known on the device only)
     PlainCluster shape;
-    if (off_pade + pade_smem_bytes(m + 2) <= kStaticScratchBytes && ((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0);
+    if (((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0);
     if (G > kMaxPartials || need > kStaticScratchBytes) {
         char msg[200];
         snprintf(msg, sizeof msg,
@@ -883,7 +878,6 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
         q.Q = Q;
         q.ps = ps;
         q.tau_im = tau_im;
-        q.scratch = base + off_pade;
         e = plain_cluster_launch(shape, q, st);
     } else {
         k_static_begin<<<1, 32, 0, st>>>(ps);

@@ -52,7 +52,7 @@ struct TkEnsemble {
     TkScal s{};
     int mb_alloc = 0;
     // the one-launch form (ctas = 0: the launches below), its trajectories' observables, the
-    // dense exponential's matrices
+    // dense exponential's matrices where shared memory does not hold them
     TaylorCluster cluster;
     int for_p = 0, for_m = 0, for_bw = 0, for_nnz = 0;   // what it was planned for
     double* obs = nullptr;
@@ -467,10 +467,10 @@ static dq_status tk_plan(dq_ctx* c) {
     t->cluster = TaylorCluster();
     cudaFree(t->pade);
     t->pade = nullptr;
-    TaylorCluster P = taylor_cluster_plan(c->n, t->B, c->tk_m, bw, (double)nnz / c->n);
+    TaylorCluster P = taylor_cluster_plan(c->n, t->B, c->tk_m, c->tk_p, bw, (double)nnz / c->n);
     if (P.ctas) {
         if (!t->obs) DQ_CU(cudaMalloc(&t->obs, sizeof(double) * 3 * (size_t)t->B));
-        DQ_CU(cudaMalloc(&t->pade, (size_t)P.chunks * pade_smem_bytes(c->tk_m + c->tk_p)));
+        if (P.scratch) DQ_CU(cudaMalloc(&t->pade, P.scratch));
     }
     t->cluster = P;
     t->for_p = c->tk_p;
