@@ -4754,9 +4754,11 @@ dq_status batched_collect_corr(dq_ctx* c) {
 }
 
 // dq_debug_set_wait_cycles: the budget every bounded wait of this device reads
-// (negative: the forced-timeout test mode of the ring SpMM)
+// (negative: the forced-timeout test mode)
 dq_status batched_set_wait_cycles(dq_ctx* c, int cycles) {
     const long long v = cycles != 0 ? (long long)cycles : kWaitCycles;
+    dq_status st = check_cuda(c, cluster_set_wait_cycles(v), "wait budget");
+    if (st) return st;
     return check_cuda(c, cudaMemcpyToSymbol(g_dq_wait_cycles, &v, sizeof(v)), "wait budget");
 }
 

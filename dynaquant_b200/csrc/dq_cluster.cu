@@ -375,6 +375,11 @@ struct ClSum {
     }
 };
 
+// Budget of the grid barrier's wait in SM cycles, as dq_debug_set_wait_cycles
+// sets it for the device: negative values make a CTA wait that many cycles for
+// a count that never comes.
+__device__ long long g_cl_wait_cycles = kWaitCycles;
+
 // The same over the whole grid (one trajectory, a cooperative launch).  A CTA
 // writes its part, fences it with its slab rows and counts itself in; one
 // thread of each CTA waits for the count, then all CTAs add the parts in rank
@@ -384,7 +389,8 @@ struct ClSum {
 // count, took 3700 to 12,500 cycles with 63 CTAs: the polls crowd the words.)
 // The wait is bounded: a CTA that gives up records DQ_ERR_TIMEOUT and stops
 // waiting for the rest of the launch (its results are void, its accesses stay
-// in bounds), so every CTA ends.
+// in bounds), so every CTA ends; it still counts itself in at every barrier
+// and out at the end, where the last one clears the counts.
 struct ClGridSum {
     double2* ex;    // [2]: the totals
     double2* red;   // [2][warps]
@@ -395,6 +401,7 @@ struct ClGridSum {
     unsigned rank;
     unsigned seq;   // barriers passed
     int pending;
+    long long budget;
 
     template <bool kPair>
     __device__ __forceinline__ void part(int buf, const double (&x)[1], const double (&y)[1]) {
@@ -426,8 +433,8 @@ struct ClGridSum {
                 while (*dead == 0) {
                     unsigned c;
                     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&g->count) : "memory");
-                    if (c >= want) break;
-                    if (clock64() - t0 > kWaitCycles) {
+                    if (c >= want && budget > 0) break;
+                    if (clock64() - t0 > llabs(budget)) {
                         *dead = 1;
                         atomicCAS(status, 0, DQ_ERR_TIMEOUT);
                     }
@@ -796,7 +803,7 @@ __device__ __forceinline__ int cl_step(const ClusterArgs& A, unsigned char* smem
     auto make_sum = [&]() {
         double2* ex = reinterpret_cast<double2*>(smem + Y.ex);
         double2* red = reinterpret_cast<double2*>(smem + Y.red);
-        if constexpr (kGrid) return ClGridSum{ex, red, A.grid, A.S.status, &W.dead, CS, rank, 0u, 0};
+        if constexpr (kGrid) return ClGridSum{ex, red, A.grid, A.S.status, &W.dead, CS, rank, 0u, 0, g_cl_wait_cycles};
         else return ClSum<TPT, kLocal>{ex, red, TC, CS, rank, (int)threadIdx.x % TC, (int)threadIdx.x / TC};
     };
     auto sum = make_sum();
@@ -1683,6 +1690,10 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
         }
     }
     return best;
+}
+
+cudaError_t cluster_set_wait_cycles(long long cycles) {
+    return cudaMemcpyToSymbol(g_cl_wait_cycles, &cycles, sizeof(cycles));
 }
 
 cudaError_t plain_cluster_attributes() {

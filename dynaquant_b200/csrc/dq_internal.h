@@ -253,6 +253,7 @@ dq_status read_status(dq_ctx* c, int code, const char* what);
 // implemented in dq_cluster.cu
 PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
 cudaError_t plain_cluster_attributes();
+cudaError_t cluster_set_wait_cycles(long long cycles);
 bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P);
 size_t taylor_cluster_head(const TaylorCluster& P);
 TaylorCluster taylor_cluster_plan(int n, int B, int mb, int p, int bw, double z);

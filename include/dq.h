@@ -301,9 +301,11 @@ DQ_API dq_status dq_time_gather_floor(dq_ctx *ctx, int reps, double *ms);
  * records DQ_ERR_TIMEOUT, lets its own copies in flight land (with the
  * default budget) and returns, and dq_run reports the status.  The same
  * budget bounds the per-chunk wait for alpha of the cooperative iteration
- * form (staged 11); a negative value makes that wait look -cycles cycles for
- * a generation that never comes, with the same outcome.  It applies to every
- * context on the device until changed again. */
+ * form (staged 11) and the grid barrier of the drop-in step of large systems;
+ * a negative value makes these waits look -cycles cycles for a generation or a
+ * count that never comes, with the same outcome (dq_prop_step reports it with
+ * err_est, dq_run_plain always).  It applies to every context on the device
+ * until changed again. */
 DQ_API dq_status dq_debug_set_wait_cycles(dq_ctx *ctx, int cycles);
 /* Test hooks, no reference counterparts: how the one-launch steps lay a system
  * out.  dq_debug_taylor_shape (no device): a Taylor-Krylov ensemble of n sites
