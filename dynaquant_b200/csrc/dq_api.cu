@@ -186,7 +186,7 @@ dq_status dq_set_hamiltonian_csr(dq_ctx* c, int n, const int* rowptr, const int*
     }
     c->rows_sorted = sorted;
     c->bw = bw;
-    c->plain = plain_cluster_plan(n, c->cfg.m, bw, (double)cl.size() / n);
+    c->plain = plain_cluster_plan(n, c->cfg.m, bw, (double)cl.size() / n, c->plain_fit);
     c->nnz_off = (int)cl.size();
     c->rowptr = std::move(rp);
     c->col = std::move(cl);
@@ -795,6 +795,19 @@ extern "C" dq_status dq_debug_taylor_shape(int n, int ctas, int traj_chunk, int 
     *smem = (int)P.smem;
     *rec = (int)P.rec;
     *head = (int)taylor_cluster_head(P);
+    return DQ_OK;
+}
+
+extern "C" dq_status dq_debug_plain_shape(int n, int m, int bandwidth, double couplings, int fit_cluster, int fit_grid,
+                                          int* ctas, int* rows, int* smem) {
+    if (n < 2 || m < 2 || m > kMaxM || bandwidth < 0 || !(couplings >= 0.0) || !ctas || !rows || !smem) return DQ_ERR_ARG;
+    PlainFit fit;
+    fit.cluster = fit_cluster;
+    fit.grid = fit_grid;
+    const PlainCluster P = plain_cluster_plan(n, m, bandwidth, couplings, fit);
+    *ctas = P.ctas;
+    *rows = P.rpc;
+    *smem = (int)P.smem;
     return DQ_OK;
 }
 

@@ -1641,13 +1641,15 @@ dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R) {
 // thread each, the records in shared memory where a CTA's turn out to fit (the
 // kernel looks).  `bw` is the matrix bandwidth, or n where only the device
 // knows the columns (then every CTA's window is the whole vector); `z` the
-// couplings of a row, 0 when unknown.  ctas = 0: too large for 16 CTAs.
+// couplings of a row, 0 when unknown; `fit` what the device can hold of it at
+// once (a launch beyond that would be refused, or wait for itself).  ctas = 0:
+// no shape fits, the step takes several launches.
 // Estimated cycles of an iteration: rounds of rows by the CTA's threads, the
 // wavefronts of the records and gathers (7 per 32 entries), the barriers.
-PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
+PlainCluster plain_cluster_plan(int n, int m, int bw, double z, const PlainFit& fit) {
     PlainCluster best;
     double t_best = 1e30;
-    for (int CS = 1; CS <= kClMaxCtas; ++CS) {
+    for (int CS = 1; CS <= std::min(kClMaxCtas, fit.cluster); ++CS) {
         const int rpc = cl_rows(n, CS, 1);
         if (CS > 1 && ((size_t)rpc * (CS - 1) >= (size_t)n || rpc < 32)) continue;
         const size_t fixed = cl_layout(n, CS, 1, m, rpc, bw, sizeof(double), 0).total;
@@ -1671,10 +1673,8 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
     // thread (fewer have a cheaper barrier, and steps of other streams run beside them).  Its two
     // barriers take about 4500 of an iteration's 14,800 cycles each (30,000 sites with 28 couplings,
     // m = 20: 184 us a step as 2 m + 5 launches, 91 us this way, three states in turn)
-    int dev = 0, sms = 0;
-    if (z > 0.0 && cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
-        for (int G = kClMaxCtas + 1; G <= std::min(sms, kPlainGridMax); ++G) {
+    if (z > 0.0) {
+        for (int G = kClMaxCtas + 1; G <= std::min(fit.grid, kPlainGridMax); ++G) {
             const int rpc = cl_rows(n, G, 1);
             if (rpc > kClThreads) continue;
             const size_t fixed = cl_layout(n, 2, 1, m, rpc, bw, sizeof(double), 0).total;
@@ -1690,6 +1690,27 @@ PlainCluster plain_cluster_plan(int n, int m, int bw, double z) {
         }
     }
     return best;
+}
+
+// After plain_cluster_attributes, for the current device.
+PlainFit plain_cluster_fit() {
+    PlainFit f;
+    int dev = 0, sms = 0, per = 0;
+    for (int CS = kClMaxCtas; CS >= 1 && f.cluster == 0; --CS) {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = cl_config(1, CS, kClSmemMax, nullptr, &at);
+        int found = 0;
+        const void* k = CS == 1 ? (const void*)k_cluster_step<double, 1, 1, true, kDropIn>
+                                : (const void*)k_cluster_step<double, 1, 1, false, kDropIn>;
+        if (cudaOccupancyMaxActiveClusters(&found, k, &cfg) == cudaSuccess && found > 0) f.cluster = CS;
+    }
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cluster_step<double, 1, 1, false, kDropInGrid>, kClThreads,
+                                                      kClSmemMax) == cudaSuccess)
+        f.grid = sms * per;
+    cudaGetLastError();   // a query that was refused leaves its part at 0
+    return f;
 }
 
 cudaError_t cluster_set_wait_cycles(long long cycles) {

@@ -54,6 +54,12 @@ struct PlainCluster {
     size_t smem = 0, rec = 0;
 };
 
+// What the current device holds of its CTAs at once: the largest cluster it
+// places, and CTAs of a cooperative grid.
+struct PlainFit {
+    int cluster = 0, grid = 0;
+};
+
 // What one such step reads and writes (device pointers).
 struct PlainStep {
     int n, m, bw, dot_mode, norm_mode;
@@ -170,6 +176,7 @@ struct dq_ctx {
     double* d_partial = nullptr;  // kMaxPartials x 2
     dq::PlainScalars* d_ps = nullptr;
     dq::PlainGrid* d_grid = nullptr;       // the one-launch step: its whole-grid form's barrier
+    dq::PlainFit plain_fit;                // what the device holds of it
     dq::PlainCluster plain;                // its shape for the Hamiltonian that is set
 
     // observables (sums over trajectories; divided by n_traj on read)
@@ -251,7 +258,8 @@ dq_status plain_observe_initial(dq_ctx* c);
 dq_status check_cuda(dq_ctx* c, cudaError_t e, const char* what);
 dq_status read_status(dq_ctx* c, int code, const char* what);
 // implemented in dq_cluster.cu
-PlainCluster plain_cluster_plan(int n, int m, int bw, double z);
+PlainCluster plain_cluster_plan(int n, int m, int bw, double z, const PlainFit& fit);
+PlainFit plain_cluster_fit();
 cudaError_t plain_cluster_attributes();
 cudaError_t cluster_set_wait_cycles(long long cycles);
 bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P);

@@ -528,6 +528,7 @@ dq_status plain_alloc(dq_ctx* c) {
     DQ_CU(raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL)));
     DQ_CU(raise_smem_limit(k_pade_tk, (int)pade_smem_bytes(kMaxL)));
     DQ_CU(plain_cluster_attributes());
+    c->plain_fit = plain_cluster_fit();
     return DQ_OK;
 }
 
@@ -738,6 +739,7 @@ struct StaticScratch {
     bool init = false;
     unsigned char* ptr = nullptr;
     CUcontext ctx = nullptr;   // the context the address belongs to
+    dq::PlainFit fit;              // what the device holds of the one-launch step at once
 };
 constexpr int kMaxDevices = 64;
 StaticScratch g_static_scratch[kMaxDevices];
@@ -809,9 +811,6 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
     const size_t off_w = off_partial + align256(sizeof(double) * 2 * kMaxPartials);
     const size_t off_q = off_w + align256(sizeof(cd) * (size_t)n);
     const size_t need = off_q + sizeof(cd) * (size_t)n * (size_t)(m + 2);
-    // one launch where the whole vector fits every CTA's window (the columns are known on the device only)
-    PlainCluster shape;
-    if (((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0);
     if (G > kMaxPartials || need > kStaticScratchBytes) {
         char msg[200];
         snprintf(msg, sizeof msg,
@@ -827,6 +826,7 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
         return DQ_ERR_CUDA;
     }
     unsigned char* base = nullptr;
+    PlainCluster shape;
     {
         std::lock_guard<std::mutex> lock(g_static_mu);
         StaticScratch& sc = g_static_scratch[dev];
@@ -839,6 +839,7 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
             if (e == cudaSuccess)
                 e = raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL));
             if (e == cudaSuccess) e = plain_cluster_attributes();
+            if (e == cudaSuccess) sc.fit = plain_cluster_fit();
             if (e != cudaSuccess) {
                 write_err(errbuf, errbuf_len, cudaGetErrorString(e));
                 return DQ_ERR_CUDA;
@@ -848,6 +849,8 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
             sc.init = true;
         }
         base = sc.ptr;
+        // one launch where the whole vector fits every CTA's window (the columns are known on the device only)
+        if (((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0, sc.fit);
     }
     PlainScalars* ps = reinterpret_cast<PlainScalars*>(base);
     double* partial = reinterpret_cast<double*>(base + off_partial);

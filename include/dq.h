@@ -312,11 +312,16 @@ DQ_API dq_status dq_debug_set_wait_cycles(dq_ctx *ctx, int cycles);
  * with clusters of `ctas` CTAs and traj_chunk trajectories; DQ_ERR_ARG when
  * the shape does not fit, else the bytes of a CTA's shared memory, of the part
  * for its coupling records (0: read through L1) and of the row starts that
- * come before them.  dq_debug_step_shape: CTAs of the drop-in step, CTAs and
+ * come before them.  dq_debug_plain_shape (no device): CTAs, rows per CTA and
+ * shared memory of the drop-in step of n sites with `couplings` per row, on a
+ * device that places clusters of fit_cluster CTAs and cooperative grids of
+ * fit_grid; 0 CTAs as below.  dq_debug_step_shape: CTAs of the drop-in step, CTAs and
  * trajectories per cluster and record bytes of the Taylor-Krylov ensemble (as
  * the last dq_reset left it); 0 CTAs stand for the step of several launches. */
 DQ_API dq_status dq_debug_taylor_shape(int n, int ctas, int traj_chunk, int m_b, int bandwidth, int *smem, int *rec,
                                        int *head);
+DQ_API dq_status dq_debug_plain_shape(int n, int m, int bandwidth, double couplings, int fit_cluster, int fit_grid,
+                                      int *ctas, int *rows, int *smem);
 DQ_API dq_status dq_debug_step_shape(dq_ctx *ctx, int *plain_ctas, int *taylor_ctas, int *taylor_traj,
                                      int *taylor_rec);
 
