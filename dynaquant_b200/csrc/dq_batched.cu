@@ -4614,6 +4614,8 @@ dq_status batched_time_iteration(dq_ctx* c, int reps, double* ms) {
         else if (pform) pf(jt);
         else enqueue_iteration_any(c, js);
     };
+    // a chunk that chose its dimension in an earlier step would skip the iteration
+    if (c->bat->s.cdone) DQ_CU(cudaMemsetAsync(c->bat->s.cdone, 0, sizeof(int) * c->bat->B, c->stream));
     if (!fused && !pform && !cluster && js == 2) enqueue_iteration_any(c, 1);
     if (fused) {
         enqueue_iteration_any(c, 1);

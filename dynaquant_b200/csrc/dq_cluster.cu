@@ -1498,8 +1498,12 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
     const size_t win = cl_layout(n, CS, tc, m, rpc, c->bw, rsz, 0).win;
     sm = std::max(sm, win + cl_dense_bytes(kClSmemMax - win, m + 2, (std::min(tc, bs->B) + CS - 1) / CS));
     int found = 0;
-    if (raise_smem_limit(k, (int)kClSmemMax) == cudaSuccess &&
-        (CS <= 8 || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)) {
+    auto prepare = [&](ClKernel f) {
+        return raise_smem_limit(f, (int)kClSmemMax) == cudaSuccess &&
+               (CS <= 8 || cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+    };
+    // the iterations alone never check: they run the other kernel
+    if (prepare(k) && prepare(cl_kernel(bs->mixed, tpt, R, CS == 1, false))) {
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t cfg = cl_config(1, CS, sm, nullptr, &at);
         if (cudaOccupancyMaxActiveClusters(&found, k, &cfg) != cudaSuccess) found = 0;
@@ -1556,7 +1560,8 @@ double cluster_plan(dq_ctx* c, int R, int* tc_out, int* cs_out) {
 }
 
 // One cluster launch: the whole step (flags kClNoise | kClFinish), or the
-// Lanczos iterations of a given slab 1 and diagonal alone (flags 0).
+// Lanczos iterations of a given slab 1 and diagonal alone (flags 0), all m of
+// them whether or not the ensemble chooses its dimension.
 cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
     BatchedState* bs = c->bat;
     const ::BlockFmt& f = cl_fmt(bs, bs->R);
@@ -1602,7 +1607,8 @@ cudaError_t cluster_launch(dq_ctx* c, bool whole_step, const ZZBlockRef& zz) {
     a.smem = (int)bs->win_smem;
     cudaLaunchAttribute at;
     const cudaLaunchConfig_t cfg = cl_config(bs->chunks, bs->ctas_per_sm, bs->win_smem, c->stream, &at);
-    return cudaLaunchKernelEx(&cfg, cl_kernel(bs->mixed, bs->TPT, bs->R, bs->ctas_per_sm == 1, bs->s.mtraj != nullptr), a);
+    const bool adaptive = whole_step && bs->s.mtraj != nullptr;
+    return cudaLaunchKernelEx(&cfg, cl_kernel(bs->mixed, bs->TPT, bs->R, bs->ctas_per_sm == 1, adaptive), a);
 }
 
 // Shapes `bs` for the cluster form (its coupling blocks of R rows exist).
