@@ -1625,7 +1625,10 @@ dq_status cluster_set(dq_ctx* c, int tc, int tpt, int CS, int R) {
         bs->cl_scratch = nullptr;
         bs->cl_scratch_bytes = 0;
         dq_status st = check_cuda(c, cudaMalloc(&bs->cl_scratch, need), "cluster scratch");
-        if (st) return st;
+        if (st) {
+            cudaGetLastError();   // the caller may go on with another form
+            return st;
+        }
         bs->cl_scratch_bytes = need;
     }
     bs->TC = tc;

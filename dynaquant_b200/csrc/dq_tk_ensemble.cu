@@ -468,9 +468,10 @@ static dq_status tk_plan(dq_ctx* c) {
     cudaFree(t->pade);
     t->pade = nullptr;
     TaylorCluster P = taylor_cluster_plan(c->n, t->B, c->tk_m, c->tk_p, bw, (double)nnz / c->n);
-    if (P.ctas) {
-        if (!t->obs) DQ_CU(cudaMalloc(&t->obs, sizeof(double) * 3 * (size_t)t->B));
-        if (P.scratch) DQ_CU(cudaMalloc(&t->pade, P.scratch));
+    if (P.ctas && ((!t->obs && cudaMalloc(&t->obs, sizeof(double) * 3 * (size_t)t->B) != cudaSuccess) ||
+                   (P.scratch && cudaMalloc(&t->pade, P.scratch) != cudaSuccess))) {
+        cudaGetLastError();   // no memory left for it: the step of several launches needs none
+        P = TaylorCluster();
     }
     t->cluster = P;
     t->for_p = c->tk_p;
