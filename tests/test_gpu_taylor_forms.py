@@ -48,3 +48,19 @@ def test_forms_match_per_trajectory_path(shape, B, m_b, ctas, records):
     for a, b in zip(got[:3], ref[:3]):
         assert np.abs(a - b).max() < TOL * max(1.0, np.abs(b).max())
     assert np.allclose(got[3], ref[3], rtol=1e-6, atol=1e-14)
+
+
+# steps that need the dense exponential: the |Re|-only norm and, in Taylor-Krylov, any halving; one launch
+# (few and many trajectories to a CTA) and several
+@pytest.mark.parametrize("shape,B,m_b,one_launch", [((12, 12), 7, 10, True), ((8, 8), 70, 20, True),
+                                                    ((30, 30), 33, 12, True), ((70000,), 2, 6, False)])
+@pytest.mark.parametrize("norm", [0, 1])
+def test_dense_exponential_matches_per_trajectory_path(shape, B, m_b, one_launch, norm):
+    from dynaquant_b200 import systems
+    s = systems.chain(*shape) if len(shape) == 1 else systems.lattice2d(*shape)
+    got, form = _run(s, "run", B, 3, 3, m_b, dt=9.0, norm=norm)
+    ref, _ = _run(s, "run_plain", B, 3, 3, m_b, dt=9.0, norm=norm)
+    assert (form[1] > 0) == one_launch
+    for a, b in zip(got[:3], ref[:3]):
+        assert np.abs(a - b).max() < TOL * max(1.0, np.abs(b).max())
+    assert np.allclose(got[3], ref[3], rtol=1e-6, atol=1e-14)
