@@ -260,6 +260,8 @@ dq_status read_status(dq_ctx* c, int code, const char* what);
 // implemented in dq_cluster.cu
 PlainCluster plain_cluster_plan(int n, int m, int bw, double z, const PlainFit& fit);
 PlainFit plain_cluster_fit();
+// the same, queried once per device context (0.4 ms); implemented in dq_plain.cu
+PlainFit plain_device_fit();
 cudaError_t plain_cluster_attributes();
 cudaError_t cluster_set_wait_cycles(long long cycles);
 bool taylor_cluster_shape(int n, int CS, int tc, int mb, int bw, TaylorCluster* P);

@@ -528,7 +528,7 @@ dq_status plain_alloc(dq_ctx* c) {
     DQ_CU(raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL)));
     DQ_CU(raise_smem_limit(k_pade_tk, (int)pade_smem_bytes(kMaxL)));
     DQ_CU(plain_cluster_attributes());
-    c->plain_fit = plain_cluster_fit();
+    c->plain_fit = plain_device_fit();
     return DQ_OK;
 }
 
@@ -739,7 +739,6 @@ struct StaticScratch {
     bool init = false;
     unsigned char* ptr = nullptr;
     CUcontext ctx = nullptr;   // the context the address belongs to
-    dq::PlainFit fit;              // what the device holds of the one-launch step at once
 };
 constexpr int kMaxDevices = 64;
 StaticScratch g_static_scratch[kMaxDevices];
@@ -773,6 +772,28 @@ void write_err(char* buf, int len, const char* msg) {
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
+
+namespace dq {
+
+PlainFit plain_device_fit() {
+    struct Known {
+        CUcontext ctx = nullptr;
+        PlainFit fit;
+    };
+    static Known known[kMaxDevices];
+    static std::mutex mu;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return PlainFit();
+    std::lock_guard<std::mutex> lock(mu);
+    const CUcontext ctx = current_context();   // as for the static call's scratch
+    if (!ctx || ctx != known[dev].ctx) {
+        known[dev].fit = plain_cluster_fit();
+        known[dev].ctx = current_context();
+    }
+    return known[dev].fit;
+}
+
+}  // namespace dq
 
 namespace dq {
 
@@ -839,7 +860,6 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
             if (e == cudaSuccess)
                 e = raise_smem_limit(k_pade_plain, (int)pade_smem_bytes(kMaxL));
             if (e == cudaSuccess) e = plain_cluster_attributes();
-            if (e == cudaSuccess) sc.fit = plain_cluster_fit();
             if (e != cudaSuccess) {
                 write_err(errbuf, errbuf_len, cudaGetErrorString(e));
                 return DQ_ERR_CUDA;
@@ -850,7 +870,7 @@ extern "C" dq_status dq_krylov_step_static(int n, const int* rowptr, const int* 
         }
         base = sc.ptr;
         // one launch where the whole vector fits every CTA's window (the columns are known on the device only)
-        if (((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0, sc.fit);
+        if (((uintptr_t)psi_in & 15) == 0) shape = plain_cluster_plan(n, m, n, 0.0, plain_device_fit());
     }
     PlainScalars* ps = reinterpret_cast<PlainScalars*>(base);
     double* partial = reinterpret_cast<double*>(base + off_partial);
