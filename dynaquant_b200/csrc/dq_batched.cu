@@ -3877,7 +3877,8 @@ static dq_status alloc_ws_into(dq_ctx* c, BatchedState* bs, int B, bool mixed, b
 // its estimated iteration beats the grid-wide form's estimate.  On a B200, a
 // step: 1,024 sites x 64 FP64 224 us grid-wide, 81 us as clusters; 4,731 x 100
 // with 28 couplings a row 739 and 331; 4,096 x 128 with 8, 375 and 169; 30,000 x
-// 256 does not fit the chip and stays grid-wide.
+// 256 does not fit the chip and stays grid-wide; 15,000 x 100 FP64 with 2 would fit,
+// 1111 us in four waves of clusters against 802 grid-wide, and stays too.
 dq_status batched_default_tiling(dq_ctx* c) {
     BatchedState* bs = c->bat;
     const int B = bs->B;
@@ -3887,13 +3888,20 @@ dq_status batched_default_tiling(dq_ctx* c) {
         const bool wide = c->nnz_off >= 6 * (size_t)c->n;
         const int R = !wide ? 1 : bs->mixed ? 3 : 2;
         const double elems = (double)c->n * B, z = (double)c->nnz_off / c->n;
-        // grid-wide forms, cycles per iteration: two launches with their reductions, then the data
-        // (with an adaptive dimension also the checks, and the launches past the chosen one)
-        const double grid = (28000.0 + elems * (bs->mixed ? 0.0075 + 0.00075 * z : 0.02 + 0.0015 * z)) *
-                            (c->cfg.m_min > 0 ? 1.6 : 1.0);
+        // Grid-wide forms, cycles per iteration: two launches with their reductions, then the data.
+        // complex128: fitted to 80 ensembles, mostly within 20 %, as the cluster form's estimate is: of 80
+        // choices four are wrong, by 12 % at most (with the former 28000 + elems (0.02 + 0.0015 z) ten
+        // were, a chain of 15,000 sites x 100 by 39 %).  complex64, as it was: no choice of the cluster
+        // form was wrong, a few of the grid-wide ones by up to a third.
+        // With an adaptive dimension also the checks and the launches past the chosen one: over 48 pairs
+        // of runs the cluster form gains 1.0 to 1.2 times in complex128 and up to 1.6 in complex64.
+        const bool adaptive = c->cfg.m_min > 0;
+        const double grid = bs->mixed ? (28000.0 + elems * (0.0075 + 0.00075 * z)) * (adaptive ? 1.6 : 1.0)
+                                      : (30500.0 + elems * (0.0358 + 0.0026 * z)) * (adaptive ? 1.1 : 1.0);
         // what the cluster form takes at least (the union of R rows' columns has z entries or more),
         // before any block is built
-        const double least = 5500.0 + elems / bs->sms * (bs->mixed ? 1.2 + 0.13 * z / R : 0.8 + 0.26 * z / R);
+        const double least = bs->mixed ? 5500.0 + elems / bs->sms * (1.2 + 0.13 * z / R)
+                                       : 4400.0 + elems / bs->sms * (3.8 + 0.26 * z / R);
         if (least < grid) {
             BlockFmt& f = bs->fmt[r_index(R)];
             dq_status st = DQ_OK;

@@ -1514,23 +1514,31 @@ static int cluster_resident(dq_ctx* c, int tc, int tpt, int CS, int R, const ::B
     return found;
 }
 
-// Estimated SM cycles of one Lanczos iteration of this shape, and the shape
-// with the least over CTAs per cluster and trajectories per chunk (R rows per
-// block, its blocks built).  An iteration is a fixed part (two reductions with
-// their barriers, the margins' round trip), the shared-memory wavefronts of
-// the gathers and records (records read through L1: a wavefront each) and the
-// elementwise part, bound by FP64 arithmetic and, in complex64, by
-// conversions; times the waves of clusters that the device needs.  Measured
-// against it on a B200 (us per iteration): 4096 sites x 128, 8 couplings per
-// row, 4 CTAs x 4 trajectories 8.0 (model 8.1); 4731 x 100, 28 couplings, 9 x 8
-// 13.8 (13.0); 8100 x 64, 6 x 4 in an adaptive run.  The order of shapes is what it
-// is used for; those within 10 % change places with the matrix.
+// The shape with the least estimated SM cycles of one Lanczos iteration over
+// CTAs per cluster and trajectories per chunk (R rows per block, its blocks
+// built), and the estimate for the choice between this form and the grid-wide
+// ones.  An iteration is a fixed part (two reductions with their barriers, the
+// margins' round trip), the shared-memory wavefronts of the gathers and records
+// (records read through L1: a wavefront each) and the elementwise part; times
+// the waves of clusters that the device needs.  Measured against it on a B200
+// (us per iteration): 4096 sites x 128, 8 couplings per row, 4 CTAs x 4
+// trajectories 8.0 (model 8.1); 4731 x 100, 28 couplings, 9 x 8 13.8 (13.0).
+// It orders shapes; those within 10 % change places with the matrix.
+//
+// complex64: 1.1 to 1.7 times the model over 80 ensembles (700 to 15,000 sites,
+// 2 to 78 couplings, 16 to 320 trajectories), much like the grid-wide estimate
+// (0.6 to 1.2), so the two are compared as they are.  complex128: 1.3 to 3
+// times, most where a thread has many rows of few couplings (a row's chain of
+// FP64 operations is not hidden), so the choice takes an estimate fitted to 80
+// such ensembles (within 27 %, standard deviation 10 %): a base, 3.8 cycles a
+// row of a thread (4.8 with one trajectory a chunk), 0.26 a gathered value,
+// 1.6 a record.
 double cluster_plan(dq_ctx* c, int R, int* tc_out, int* cs_out) {
     const BatchedState* bs = c->bat;
     const ::BlockFmt& f = cl_fmt(bs, R);
     const int n = c->n, B = bs->B, tpt = bs->mixed ? 2 : 1;
     const double len = (double)f.nunion / std::max(1, f.nb), csz = bs->mixed ? 8.0 : 16.0;
-    double best = 1e30;
+    double best = 1e30, est = 1e30;
     for (int CS = 1; CS <= kClMaxCtas; ++CS) {
         const int rpc = cl_rows(n, CS, R);
         if (CS > 1 && (size_t)rpc * (CS - 1) >= (size_t)n) continue;   // a CTA without rows
@@ -1548,15 +1556,19 @@ double cluster_plan(dq_ctx* c, int R, int* tc_out, int* cs_out) {
             size_t smem = 0, rec = 0;
             const int fit = cluster_resident(c, tc, tpt, CS, R, f, &smem, &rec);
             if (fit < 1) continue;
-            const double t = (double)((chunks + fit - 1) / fit) * cycles(rec > 0);
+            const int waves = (chunks + fit - 1) / fit;
+            const double t = waves * cycles(rec > 0);
             if (t < best) {
                 best = t;
+                est = bs->mixed ? t
+                                : waves * (4400.0 + (tc == 1 ? 4.84 : 3.83) * R * kClThreads * std::ceil(nbk * TL / kClThreads) +
+                                           0.262 * nbk * len * tc + 1.58 * nbk * len);
                 *tc_out = tc;
                 *cs_out = CS;
             }
         }
     }
-    return best;
+    return est;
 }
 
 // One cluster launch: the whole step (flags kClNoise | kClFinish), or the
