@@ -162,8 +162,9 @@ class Propagator:
         return ms.value
 
     def debug_set_wait_cycles(self, cycles):
-        """Test hook: budget of the TMA-fed SpMM forms' barrier waits on this device (0: default; negative:
-        the ring form's CTAs first wait that many cycles on a barrier nothing completes, so they time out)."""
+        """Test hook: budget of the bounded waits on this device (TMA-fed SpMM forms, cooperative iteration,
+        grid barrier of the drop-in step; 0: default; negative: they wait that many cycles for something that
+        never comes, so they time out)."""
         self._check(self.L.dq_debug_set_wait_cycles(self.h, int(cycles)))
 
     def debug_step_shape(self):
