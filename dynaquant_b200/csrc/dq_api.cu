@@ -1,6 +1,7 @@
 // dq_api.cu — the C ABI (include/dq.h): context life cycle, system set-up,
 // the plain drop-in step, the ensemble drivers and the observable getters.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <new>
@@ -730,8 +731,11 @@ extern "C" dq_status dq_autotune(dq_ctx* c, int reps, double* best_ms) {
     dq_status st;
     if ((st = ensure_batched(c))) return st;
     if ((st = dq_reset(c))) return st;
-    int b_tc = 0, b_vec = 0, b_cps = 0, b_r = 0, b_st = 0, b_g = 1;
-    double best = 1e30;
+    // the fastest iteration of the grid-wide forms [0] and of the cluster form [1]
+    struct Found {
+        int tc = 0, vec = 0, cps = 0, R = 0, staged = 0, groups = 1;
+        double ms = 1e30;
+    } found[2];
     const int vecs[2] = {2, 1};
     for (int groups = 1; groups <= 8; groups <<= 1)
         for (int staged = 0; staged <= 13; ++staged)
@@ -743,13 +747,27 @@ extern "C" dq_status dq_autotune(dq_ctx* c, int reps, double* best_ms) {
                             if (batched_set_tiling(c, tc, vecs[vi], cps, R, staged, groups) != DQ_OK) continue;
                             double ms = 0.0;
                             if ((st = batched_time_iteration(c, reps, &ms))) return st;
-                            if (ms < best) {
-                                best = ms; b_tc = tc; b_vec = vecs[vi]; b_cps = cps; b_r = R; b_st = staged;
-                                b_g = groups;
-                            }
+                            Found& f = found[staged == 13];
+                            if (ms < f.ms) f = Found{tc, vecs[vi], cps, R, staged, groups, ms};
                         }
-    if (!b_tc) return fail(c, DQ_ERR_ARG, "autotune: no valid tiling");
-    if ((st = batched_set_tiling(c, b_tc, b_vec, b_cps, b_r, b_st, b_g))) return st;
+    auto apply = [&](const Found& f) { return batched_set_tiling(c, f.tc, f.vec, f.cps, f.R, f.staged, f.groups); };
+    int pick = found[1].ms < found[0].ms;
+    if (!found[pick].tc) return fail(c, DQ_ERR_ARG, "autotune: no valid tiling");
+    if (c->cfg.m_min > 0 && found[0].tc && found[1].tc && c->cfg.max_steps > 1) {
+        // an adaptive step is not m iterations, and what stopping early saves differs between the two
+        // (grid-wide: checks and launches that return at once): whole steps decide
+        const int k = std::min(4, c->cfg.max_steps - 1);
+        double step_ms[2];
+        for (int i = 0; i < 2; ++i) {
+            if ((st = apply(found[i])) || (st = dq_reset(c)) || (st = batched_run(c, 1))) return st;   // captures the step
+            const auto t0 = std::chrono::steady_clock::now();
+            if ((st = batched_run(c, k))) return st;   // ends in a synchronisation
+            step_ms[i] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        }
+        pick = step_ms[1] < step_ms[0];
+    }
+    if ((st = apply(found[pick]))) return st;
+    const double best = found[pick].ms;
     if (best_ms) *best_ms = best;
     c->ready = false;
     return dq_reset(c);

@@ -25,3 +25,26 @@ def test_adaptive_contexts_time_whole_iterations(tiling):
         p.close()
     # the same work: far from the 4 / 28 of a run that stops early, or from none at all
     assert 0.6 < ms[4] / ms[0] < 1.6, ms
+
+
+@pytest.mark.parametrize("m_min", [0, 4])
+def test_autotuned_context_reproduces_an_untuned_one(m_min):
+    """Autotuning, which with an adaptive dimension compares whole steps, leaves a context that starts over."""
+    import dynaquant_b200 as dq
+    from dynaquant_b200 import systems
+    s = systems.tube(20, 30)
+    out = []
+    for tune in (False, True):
+        p = dq.Propagator(s.n, m=16, n_traj=16, dt=0.5, noise=dq.NOISE_OU, seed=5, precision=dq.PREC_FP64, max_steps=3,
+                          m_min=m_min, m_tol=1e-9)
+        p.set_system(s)
+        p.set_noise_params(np.full(s.n, 250.0), np.full(s.n, 50.0))
+        p.set_initial_state(s.bright_state())
+        if tune:
+            assert p.autotune_raw(1) > 0.0
+            assert p.steps_done == 0
+        p.run(3)
+        out.append((p.populations(), p.correlation(), p.error_accum()))
+        p.close()
+    assert np.abs(out[0][0] - out[1][0]).max() < 1e-10 and np.abs(out[0][1] - out[1][1]).max() < 1e-9
+    assert np.allclose(out[0][2], out[1][2], rtol=1e-3, atol=1e-13)
