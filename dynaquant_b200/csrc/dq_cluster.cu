@@ -193,6 +193,7 @@ __device__ __forceinline__ void cl_estimate(const ClusterArgs& A, int b, double 
 // in global memory, spent 1.08 ms of a step of 1.43 ms (4,731 sites x 100,
 // eight to a cluster of nine CTAs), and 1.6 ms of 2.0 ms at 132 x 4,096, 32 to
 // a CTA.
+
 // Teams for nt trajectories with matrices of L rows in `room` bytes (0: not even one fits).
 static __host__ __device__ inline int cl_dense_teams(size_t room, int L, int nt) {
     if (pade_mats_bytes(L) > room) return 0;

@@ -281,7 +281,7 @@ __device__ inline PadeOut pade_exp_tbar(int m, const cd* alpha, const cd* beta, 
 // kSeriesMaxS halvings, and the |Re|-only norm on a matrix of complex norm
 // above 1/2, whose quotient the reference takes unscaled.
 // Measured on a B200 (kernel time): one trajectory, m = 16, 41 us dense and
-// 4.4 us this way; 256 trajectories, m = 20, 61 and 6.6 us.
+// 4.4 us this way; 256 trajectories, m = 20, 61 and 8.4 us (a CTA each).
 // ---------------------------------------------------------------------------
 constexpr int kSeriesMaxS = 4;
 constexpr int kSeriesTerms = 24;   // never reached at a norm <= 1/2 (16 terms); bounds the loops
